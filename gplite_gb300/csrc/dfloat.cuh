@@ -241,6 +241,30 @@ __device__ __forceinline__ double df2d_scaled(float hi, float lo, int sh) {
   return __longlong_as_double((long long)(mag | ((unsigned long long)(bh >> 31) << 63)));
 }
 
+// df2d_scaled without a branch: the same value where it takes its fast path, and
+// slow set (the result void) where it does not.
+__device__ __forceinline__ double df2d_try(float hi, float lo, int sh, bool &slow) {
+  const float s = __fadd_rn(hi, lo);
+  const float bp = __fsub_rn(s, hi);
+  lo = __fadd_rn(__fsub_rn(hi, __fsub_rn(s, bp)), __fsub_rn(lo, bp));
+  hi = s;
+  const uint32_t bh = __float_as_uint(hi), bl = __float_as_uint(lo);
+  const uint32_t eh = (bh >> 23) & 0xFFu, el = (bl >> 23) & 0xFFu;
+  const int ed = (int)eh - 127 + 1023 + sh;
+  const int shift = (int)el - (int)eh + 29;
+  const bool zero = (bh << 1) == 0u;
+  slow |= !zero && (eh == 0u || eh == 0xFFu || el == 0xFFu || ed <= 1 || ed >= 2047 || shift > 5);
+  const uint32_t mh = bh & 0x7FFFFFu;
+  const uint32_t ml = el != 0u ? (bl & 0x7FFFFFu) | 0x800000u : 0u;
+  // ml << shift, or >> -shift: as one right shift of ml << 5 (shift <= 5 here)
+  uint32_t k = (ml << 5) >> min(max(5 - shift, 0), 31);
+  const bool opposite = ((bh ^ bl) >> 31) != 0u;
+  if (opposite && mh == 0u) k <<= 1;
+  unsigned long long mag = ((unsigned long long)(uint32_t)ed << 52) | ((unsigned long long)mh << 29);
+  mag = opposite ? mag - k : mag + k;
+  mag |= (unsigned long long)(bh >> 31) << 63;
+  return __longlong_as_double(zero ? 0ll : (long long)mag);
+}
 __device__ __forceinline__ double f2_to_double(f2 a) { return df2d_scaled(a.h, a.l, 0); }
 
 }  // namespace gpgp

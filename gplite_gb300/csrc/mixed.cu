@@ -16,12 +16,17 @@
 //   (A B^T)_ij = 2^(e_i + f_j - 16) (P_0 + P_1 + P_2 + P_3+).
 // The truncation error is ~2^-(8S+1) of the row maxima.
 //
-// A tcgen05.mma costs about the same whatever its N (measured: N = 32..128 and
-// M = 64 or 128 all take ~88 cycles per instruction here), so the products are
-// issued as few, wide instructions: the B slices are adjacent in shared memory,
-// and A_t times B slices 0..3-t is one MMA of N = 64 (4 - t) whose column blocks
-// are the accumulators of levels t..3. S = 4 takes 7 instructions per K step
-// instead of 13, S = 5 takes 13 instead of 19.
+// The products are issued as few, wide instructions: the B slices are adjacent in
+// shared memory, and A_t times B slices 0..3-t is one MMA of N = 64 (4 - t) whose
+// column blocks are the accumulators of levels t..3. S = 4 takes 7 instructions per K
+// step instead of 13, S = 5 takes 13 instead of 19. The tensor pipe runs N >= 128 at
+// its full rate (4080 multiply-adds per clock; N = 64 takes 48 cycles, N = 128 64,
+// N = 256 128), so a K step of S = 4 is 476 cycles at least. What bounds the kernel:
+// at long K the MMAs (1.37 to 1.5 PFLOP/s at 4096^2 x 4096, S = 4; 1.15 with the issue
+// loop inside one lane's branch), at K <= 384 the epilogue's integer work and C
+// traffic (8192^2, lower-only off: K = 384 0.55 ms, K = 256 0.43, K = 64 0.41; 0.70,
+// 0.60 and 0.63 with 64-bit tile arithmetic in every warp and a branch per converted
+// output).
 //
 // Data path: slices are stored pre-tiled in the canonical no-swizzle K-major
 // UMMA layout (8-row x 16-byte core matrices, 64-row x 32-K tiles), so one
@@ -408,6 +413,13 @@ __device__ __forceinline__ void umma_bf16(uint32_t dtmem, uint64_t adesc, uint64
       "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accum));
 }
 
+// one lane of a converged warp (the predicate stays uniform for the compiler)
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(p));
+  return p != 0;
+}
+
 __device__ __forceinline__ void umma_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
                : "memory");
@@ -466,13 +478,13 @@ __device__ __forceinline__ void df_add(float &hi, float &lo, float v) {
 struct OzGemmArgs {
   const uint16_t *a_sl;
   const int *a_ex;
-  int64_t a_nrb, a_nkc, a_rb0;  // slice-tile geometry (32-wide K chunks); first 64-row tile
+  int a_nrb, a_nkc, a_rb0;  // slice-tile geometry (32-wide K chunks); first 64-row tile
   const uint16_t *b_sl;
   const int *b_ex;
-  int64_t b_nrb, b_nkc, b_rb0;
-  int64_t M, N;
-  int64_t kc0, kc1;  // 32-wide K chunks [kc0, kc1) of both operands
-  int kmode;         // 0 all; 1 start at max(row,col); 2 start at col; 3 end after row
+  int b_nrb, b_nkc, b_rb0;
+  int M, N;
+  int kc0, kc1;  // 32-wide K chunks [kc0, kc1) of both operands
+  int kmode;     // 0 all; 1 start at max(row,col); 2 start at col; 3 end after row
   double alpha, beta;
   double *C;
   int64_t ldc;
@@ -481,38 +493,80 @@ struct OzGemmArgs {
   const int *status;  // optional: skip a problem whose factorisation already failed
   int64_t a_bs_sl, a_bs_ex, b_bs_sl, b_bs_ex, c_bs;  // per-problem strides
   int64_t status_bs;
-  int64_t gx, gy, batch;  // tile grid; tile L = (z gy + by) gx + bx
+  int gx, gy;       // tiles per problem along M and N
+  int order;        // OzOrder
+  int per, ntiles;  // tiles per problem and in the launch
 };
+
+// The order in which a problem's tiles are dealt to the CTAs, longest K range first
+// where the ranges differ (kmode 1 and 3), so that the last round of the persistent
+// grid holds the short ones:
+//  OZ_COLS        columns of tiles, left to right
+//  OZ_ROWS_UP     rows of tiles, last row first (kmode 3: the range ends after the row)
+//  OZ_LOWER       the tiles that meet the lower triangle only, row by row (kmode 1: the
+//                 range starts at the row). Tiles above the diagonal are not dealt: in a
+//                 square product they are half of the list, and skipping them in turn
+//                 left the CTAs with unequal counts.
+enum OzOrder { OZ_COLS = 0, OZ_ROWS_UP = 1, OZ_LOWER = 2 };
 
 struct OzTile {
-  int64_t z, row0, col0, c0, nch;
+  int z, row0, col0, c0, nch;
 };
 
-// The work of tile L (identical in every role): false when the tile is skipped
-// (above the diagonal of a lower-only product, or its problem has failed)
-__device__ __forceinline__ bool oz_tile_at(const OzGemmArgs &g, int64_t L, OzTile &t) {
-  const int64_t per = g.gx * g.gy;
-  t.z = L / per;
-  const int64_t r = L - t.z * per;
-  const int64_t by = r / g.gx, bx = r - by * g.gx;
+// Tiles of the lower triangle: row bx has min(2 bx + 2, gy) of them.
+__host__ __device__ __forceinline__ int oz_lower_tiles(int gx, int gy) {
+  const int q = gy / 2;  // rows below q have 2 bx + 2 <= gy tiles
+  return gx <= q ? gx * (gx + 1) : q * (q + 1) + (gx - q) * gy;
+}
+
+// Position r of a problem's tile list -> tile coordinates (bx, by)
+__host__ __device__ __forceinline__ void oz_tile_xy(int order, int gx, int gy, int r, int *bx, int *by) {
+  if (order == OZ_LOWER) {
+    const int q = gy / 2, cq = q * (q + 1);
+    if (r < cq) {
+      int b = (int)((sqrtf(4.0f * (float)r + 1.0f) - 1.0f) * 0.5f);
+      while (b * (b + 1) > r) --b;
+      while ((b + 1) * (b + 2) <= r) ++b;
+      *bx = b;
+      *by = r - b * (b + 1);
+    } else {
+      const int o = (r - cq) / gy;
+      *bx = q + o;
+      *by = (r - cq) - o * gy;
+    }
+  } else if (order == OZ_ROWS_UP) {
+    const int o = r / gy;
+    *bx = gx - 1 - o;
+    *by = r - o * gy;
+  } else {
+    const int o = r / gx;
+    *by = o;
+    *bx = r - o * gx;
+  }
+}
+
+// The K chunks [k0, k1) of the tile at (row0, col0)
+__host__ __device__ __forceinline__ void oz_krange(int kmode, int grow0, int gcol0, int kc0, int kc1, int *k0,
+                                                   int *k1) {
+  if (kmode == 1) kc0 = max(kc0, max(grow0, gcol0) / OZ_TK);
+  if (kmode == 2) kc0 = max(kc0, gcol0 / OZ_TK);
+  if (kmode == 3) kc1 = min(kc1, (grow0 + OZ_BM + OZ_TK - 1) / OZ_TK);
+  *k0 = kc0;
+  *k1 = kc1;
+}
+
+// The work of position L (identical in every role): false when its problem has failed.
+// All 32-bit: 64-bit divisions here cost every epilogue warp more than the tile's
+// TMEM reads.
+__device__ __forceinline__ bool oz_tile_at(const OzGemmArgs &g, int L, OzTile &t) {
+  t.z = g.per == g.ntiles ? 0 : L / g.per;
+  int bx, by;
+  oz_tile_xy(g.order, g.gx, g.gy, L - t.z * g.per, &bx, &by);
   t.row0 = bx * OZ_BM;
   t.col0 = by * OZ_BN;
-  if (g.lower_only && t.col0 > t.row0 + OZ_BM - 1) return false;
   if (g.status && *(volatile const int *)(g.status + t.z * g.status_bs) != 0) return false;
-  const int64_t grow0 = g.a_rb0 * OZ_TR + t.row0, gcol0 = g.b_rb0 * OZ_TR + t.col0;
-  int64_t k0 = g.kc0, k1 = g.kc1;
-  if (g.kmode == 1) {
-    const int64_t s0 = (grow0 > gcol0 ? grow0 : gcol0) / OZ_TK;
-    k0 = k0 > s0 ? k0 : s0;
-  }
-  if (g.kmode == 2) {
-    const int64_t s0 = gcol0 / OZ_TK;
-    k0 = k0 > s0 ? k0 : s0;
-  }
-  if (g.kmode == 3) {
-    const int64_t e0 = (grow0 + OZ_BM + OZ_TK - 1) / OZ_TK;
-    k1 = k1 < e0 ? k1 : e0;
-  }
+  int k0, k1;
+  oz_krange(g.kmode, g.a_rb0 * OZ_TR + t.row0, g.b_rb0 * OZ_TR + t.col0, g.kc0, g.kc1, &k0, &k1);
   t.c0 = k0;
   t.nch = k1 > k0 ? k1 - k0 : 0;
   return true;
@@ -570,7 +624,7 @@ __global__ void __maxnreg__(96) oz_gemm_kernel(const OzGemmArgs g) {
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = tmem_base_sh;
-  const int64_t ntiles = g.gx * g.gy * g.batch;
+  const int ntiles = g.ntiles;
   int last_full_parity[NST];
 #pragma unroll
   for (int i = 0; i < NST; ++i) last_full_parity[i] = -1;
@@ -581,13 +635,15 @@ __global__ void __maxnreg__(96) oz_gemm_kernel(const OzGemmArgs g) {
     if (lane == 0) {
       int st = 0;
       uint32_t ph = 0;
-      for (int64_t L = blockIdx.x; L < ntiles; L += gridDim.x) {
+      for (int L = blockIdx.x; L < ntiles; L += gridDim.x) {
         OzTile t;
         if (!oz_tile_at(g, L, t) || t.nch == 0) continue;
-        const uint16_t *a_sl = g.a_sl + t.z * g.a_bs_sl;
-        const uint16_t *b_sl = g.b_sl + t.z * g.b_bs_sl;
-        const int64_t arb = g.a_rb0 + t.row0 / OZ_TR, brb = g.b_rb0 + t.col0 / OZ_TR;
-        for (int64_t c = 0; c < t.nch; ++c) {
+        const uint16_t *ap = g.a_sl + t.z * g.a_bs_sl +
+                             ((int64_t)t.c0 * g.a_nrb + g.a_rb0 + t.row0 / OZ_TR) * OZ_TILE;
+        const uint16_t *bp = g.b_sl + t.z * g.b_bs_sl +
+                             ((int64_t)t.c0 * g.b_nrb + g.b_rb0 + t.col0 / OZ_TR) * OZ_TILE;
+        const int64_t asl = (int64_t)g.a_nkc * g.a_nrb * OZ_TILE, bsl = (int64_t)g.b_nkc * g.b_nrb * OZ_TILE;
+        for (int c = 0; c < t.nch; ++c) {
           if (!oz_wait(bar(EMPTY + st), ph ^ 1u, abort_flag)) {
             if (!*abort_flag) atomicExch(g.err, 1);
             abort_sh = 1;
@@ -595,14 +651,13 @@ __global__ void __maxnreg__(96) oz_gemm_kernel(const OzGemmArgs g) {
           }
           const uint32_t base = smem_u32(smem + st * Cfg::STAGE);
           mbar_expect_tx(bar(FULL + st), Cfg::STAGE);
-          const int64_t kc = t.c0 + c;
 #pragma unroll
           for (int s = 0; s < S; ++s) {
-            bulk_g2s(base + s * Cfg::A_SL, a_sl + (((int64_t)s * g.a_nkc + kc) * g.a_nrb + arb) * OZ_TILE,
-                     Cfg::A_SL, bar(FULL + st));
-            bulk_g2s(base + S * Cfg::A_SL + s * Cfg::B_SL,
-                     b_sl + (((int64_t)s * g.b_nkc + kc) * g.b_nrb + brb) * OZ_TILE, Cfg::B_SL, bar(FULL + st));
+            bulk_g2s(base + s * Cfg::A_SL, ap + s * asl, Cfg::A_SL, bar(FULL + st));
+            bulk_g2s(base + S * Cfg::A_SL + s * Cfg::B_SL, bp + s * bsl, Cfg::B_SL, bar(FULL + st));
           }
+          ap += (int64_t)g.a_nrb * OZ_TILE;
+          bp += (int64_t)g.b_nrb * OZ_TILE;
           last_full_parity[st] = (int)ph;
           if (++st == NST) {
             st = 0;
@@ -613,43 +668,45 @@ __global__ void __maxnreg__(96) oz_gemm_kernel(const OzGemmArgs g) {
     producer_done:;
     }
   } else if (warp == 1) {
-    // ---- MMA issuer ----
-    if (lane == 0) {
-      // D F32, A/B BF16, K-major both, M = 128; N is set per instruction
-      const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(OZ_BM >> 4) << 24);
-      // no-swizzle K-major: core matrices of 8 rows x 16 bytes; LBO steps K (128 B),
-      // SBO steps 8 rows (8 x 32 K x 2 B = 512 B)
-      const uint32_t lbo = 128u, sbo = 512u;
-      int st = 0, b = 0;
-      uint32_t ph = 0, tph[2] = {0u, 0u};
-      for (int64_t L = blockIdx.x; L < ntiles; L += gridDim.x) {
-        OzTile t;
-        if (!oz_tile_at(g, L, t) || t.nch == 0) continue;
-        uint32_t fresh = 0;  // 1 while the group's accumulators are still to be overwritten
-        for (int64_t c = 0; c < t.nch; ++c) {
-          const bool gstart = (c % OZ_GROUP) == 0;
-          const bool gend = ((c + 1) % OZ_GROUP) == 0 || c == t.nch - 1;
-          if (gstart) {
-            if (!oz_wait(bar(TEMPTY + b), tph[b] ^ 1u, abort_flag)) {
-              if (!*abort_flag) atomicExch(g.err, 2);
-              abort_sh = 1;
-              goto mma_done;
-            }
-            tc_fence_after();
-            fresh = 1;
-          }
-          if (!oz_wait(bar(FULL + st), ph, abort_flag)) {
+    // ---- MMA issuer: the whole warp walks the chunks, one elected lane issues ----
+    // (Warp-uniform control flow keeps descriptors and barrier addresses in uniform
+    // registers; with everything inside one lane's branch an instruction took 84 to
+    // 100 cycles to issue, longer than the tensor pipe takes to run it.)
+    // D F32, A/B BF16, K-major both, M = 128; N is set per instruction
+    const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(OZ_BM >> 4) << 24);
+    // no-swizzle K-major: core matrices of 8 rows x 16 bytes; LBO steps K (128 B),
+    // SBO steps 8 rows (8 x 32 K x 2 B = 512 B). Slices, K steps and stages are offsets
+    // in 16-byte units (shared addresses stay below 2^18, so the 14-bit address field
+    // never carries).
+    const uint64_t adesc = umma_desc(smem_u32(smem), 128u, 512u);
+    const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0);
+    const bool leader = elect_one();
+    int st = 0, b = 0;
+    uint32_t ph = 0, tph = 0;  // tph bit b: parity of accumulator set b
+    for (int L = blockIdx.x; L < ntiles; L += gridDim.x) {
+      OzTile t;
+      if (!oz_tile_at(g, L, t) || t.nch == 0) continue;
+      uint32_t acc = 0;  // 0 while the group's accumulators are still to be overwritten
+      for (int c = 0; c < t.nch; ++c) {
+        const bool gend = ((c + 1) & (OZ_GROUP - 1)) == 0 || c == t.nch - 1;
+        if ((c & (OZ_GROUP - 1)) == 0) {
+          if (!oz_wait(bar(TEMPTY + b), ((tph >> b) & 1u) ^ 1u, abort_flag)) {
             if (!*abort_flag) atomicExch(g.err, 2);
             abort_sh = 1;
             goto mma_done;
           }
-          tc_fence_after();
-          const uint32_t abase = smem_u32(smem + st * Cfg::STAGE);
-          const uint32_t bbase = abase + S * Cfg::A_SL;
-          // Descriptors of the stage; slices and K steps are offsets in 16-byte units
-          // (shared addresses stay below 2^18, so the 14-bit address field never carries).
-          const uint64_t ad0 = umma_desc(abase, lbo, sbo), bd0 = umma_desc(bbase, lbo, sbo);
-          const uint32_t d0 = tmem + (uint32_t)(b * OZ_NACC * OZ_BN);
+          acc = 0;
+        }
+        if (!oz_wait(bar(FULL + st), ph, abort_flag)) {
+          if (!*abort_flag) atomicExch(g.err, 2);
+          abort_sh = 1;
+          goto mma_done;
+        }
+        tc_fence_after();
+        const uint64_t ad0 = adesc + (uint64_t)((uint32_t)st * (uint32_t)(Cfg::STAGE >> 4));
+        const uint64_t bd0 = ad0 + (uint64_t)((S * Cfg::A_SL) >> 4);
+        const uint32_t d0 = tm + (uint32_t)(b * OZ_NACC * OZ_BN);
+        if (leader) {
 #pragma unroll
           for (int kk = 0; kk < OZ_TK / 16; ++kk) {
 #pragma unroll
@@ -662,7 +719,7 @@ __global__ void __maxnreg__(96) oz_gemm_kernel(const OzGemmArgs g) {
               if (ti < OZ_NACC)
                 umma_bf16(d0 + (uint32_t)(ti * OZ_BN), ad, bd0 + (uint64_t)((kk * 256) >> 4),
                           idesc | ((uint32_t)((OZ_NACC - ti) * OZ_BN >> 3) << 17),
-                          (kk == 0 && ti == 0) ? (fresh ^ 1u) : 1u);
+                          (kk == 0 && ti == 0) ? acc : 1u);
               // the remaining products of levels > 3 go one by one into the last accumulator
 #pragma unroll
               for (int ui = ti < OZ_NACC ? OZ_NACC - ti : 0; ui < S; ++ui) {
@@ -673,22 +730,23 @@ __global__ void __maxnreg__(96) oz_gemm_kernel(const OzGemmArgs g) {
               }
             }
           }
-          fresh = 0;
-          mma_issued = true;
           umma_commit(bar(EMPTY + st));
-          if (++st == NST) {
-            st = 0;
-            ph ^= 1u;
-          }
-          if (gend) {
-            umma_commit(bar(TFULL + b));
-            tph[b] ^= 1u;
-            b ^= 1;
-          }
+          if (gend) umma_commit(bar(TFULL + b));
+        }
+        __syncwarp();
+        acc = 1u;
+        mma_issued = true;
+        if (++st == NST) {
+          st = 0;
+          ph ^= 1u;
+        }
+        if (gend) {
+          tph ^= 1u << b;
+          b ^= 1;
         }
       }
-    mma_done:;
     }
+  mma_done:;
   } else {
     // ---- epilogue: warps 2..17 drain TMEM lanes 32 (warp % 4).., 16 columns each ----
     const int quarter = warp & 3, part = (warp - 2) >> 2;
@@ -698,37 +756,53 @@ __global__ void __maxnreg__(96) oz_gemm_kernel(const OzGemmArgs g) {
     const bool unit = (g.alpha == 1.0 || g.alpha == -1.0) && (g.beta == 0.0 || g.beta == 1.0);
     const bool beta0 = g.beta == 0.0, beta1 = g.beta == 1.0;
     const uint32_t negmask = g.alpha < 0.0 ? 0x80000000u : 0u;
-    for (int64_t L = blockIdx.x; L < ntiles; L += gridDim.x) {
+    for (int L = blockIdx.x; L < ntiles; L += gridDim.x) {
       OzTile t;
       if (!oz_tile_at(g, L, t)) continue;
-      const int64_t my_row = t.row0 + quarter * 32 + lane;
-      const bool row_ok = my_row < g.M;
-      const int64_t col_base = t.col0 + part * OZ_EPI_COLS;
-      double *crow = g.C + t.z * g.c_bs + my_row;
-      // this thread's C values, loaded before the accumulators are ready so that
-      // the loads overlap the MMAs
-      double cv[OZ_EPI_COLS];
+      const int my_row = t.row0 + quarter * 32 + lane;
+      const int col_base = t.col0 + part * OZ_EPI_COLS;
+      // this thread's columns: those inside C and, of a lower-only product, left of
+      // the diagonal (0 outside the rows)
+      int ncol = my_row < g.M ? min(OZ_EPI_COLS, g.N - col_base) : 0;
+      if (g.lower_only) ncol = min(ncol, my_row - col_base + 1);
+      double *cp = g.C + t.z * g.c_bs + my_row + (int64_t)col_base * g.ldc;
+      // The first half of this thread's C values is loaded before the accumulators are
+      // ready, so that the loads overlap the MMAs; the second half is only brought to
+      // L2 (16 values at a time would not leave the accumulation its registers).
+      constexpr int HALF = OZ_EPI_COLS / 2;
+      double cv[HALF];
+      auto load_c = [&](int j0) {
+        const double *cr = cp + j0 * g.ldc;
 #pragma unroll
-      for (int j = 0; j < OZ_EPI_COLS; ++j)
-        cv[j] = (row_ok && !beta0 && col_base + j < g.N) ? crow[(col_base + j) * g.ldc] : 0.0;
+        for (int j = 0; j < HALF; ++j) {
+          cv[j] = j0 + j < ncol ? *cr : 0.0;
+          cr += g.ldc;
+        }
+      };
+      if (!beta0) {
+        load_c(0);
+        const double *cr = cp + HALF * g.ldc;
+#pragma unroll
+        for (int j = 0; j < HALF; ++j) {
+          if (HALF + j < ncol) asm volatile("prefetch.global.L2 [%0];" ::"l"(cr));
+          cr += g.ldc;
+        }
+      }
       if (t.nch == 0) {  // nothing accumulated: C = beta C
-        if (row_ok && !beta1)
-#pragma unroll
-          for (int j = 0; j < OZ_EPI_COLS; ++j) {
-            const int64_t col = col_base + j;
-            if (col < g.N && !(g.lower_only && my_row < col)) crow[col * g.ldc] = g.beta * cv[j];
-          }
+        if (!beta1)
+          for (int j = 0; j < ncol; ++j) cp[j * g.ldc] = beta0 ? 0.0 : g.beta * cp[j * g.ldc];
         continue;
       }
-      const int *a_ex = g.a_ex + t.z * g.a_bs_ex;
-      const int *b_ex = g.b_ex + t.z * g.b_bs_ex + g.b_rb0 * OZ_TR;
-      const int ea = row_ok ? a_ex[g.a_rb0 * OZ_TR + my_row] : 0;
-      const int64_t ngr = (t.nch + OZ_GROUP - 1) / OZ_GROUP;
+      // exponents: the row's, and the 16 columns' one to a lane
+      const int ea = my_row < g.M ? g.a_ex[t.z * g.a_bs_ex + g.a_rb0 * OZ_TR + my_row] : 0;
+      const int eb = lane < OZ_EPI_COLS && col_base + lane < g.N
+                         ? g.b_ex[t.z * g.b_bs_ex + g.b_rb0 * OZ_TR + col_base + lane] : 0;
+      const int ngr = (t.nch + OZ_GROUP - 1) / OZ_GROUP;
       // the tile's sum over its K groups, in double-float (level-0 units)
       float hi[OZ_EPI_COLS], lo[OZ_EPI_COLS];
 #pragma unroll
       for (int j = 0; j < OZ_EPI_COLS; ++j) hi[j] = lo[j] = 0.f;
-      for (int64_t gi = 0; gi < ngr; ++gi) {
+      for (int gi = 0; gi < ngr; ++gi) {
         int ok = 1;
         if (lane == 0) ok = oz_wait(bar(TFULL + b), tph[b], abort_flag) ? 1 : 0;
         ok = __shfl_sync(0xffffffffu, ok, 0);
@@ -740,21 +814,21 @@ __global__ void __maxnreg__(96) oz_gemm_kernel(const OzGemmArgs g) {
           goto epi_done;
         }
         tc_fence_after();
+        const uint32_t ta = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(b * OZ_NACC * OZ_BN + part * OZ_EPI_COLS);
 #pragma unroll
-        for (int cb = 0; cb < OZ_EPI_COLS / 8; ++cb) {
-          uint32_t r[OZ_NACC][8];
+        for (int cb = 0; cb < OZ_EPI_COLS / 8; ++cb)
 #pragma unroll
-          for (int acc = 0; acc < OZ_NACC; ++acc)
-            tmem_ld8(tmem + ((uint32_t)(quarter * 32) << 16) +
-                         (uint32_t)((b * OZ_NACC + acc) * OZ_BN + part * OZ_EPI_COLS + cb * 8),
-                     r[acc]);
-          tmem_ld_wait();
+          for (int ac = 0; ac < OZ_NACC; ac += 2) {  // two accumulators at a time: 16 registers
+            uint32_t r[2][8];
+            tmem_ld8(ta + (uint32_t)(ac * OZ_BN + cb * 8), r[0]);
+            tmem_ld8(ta + (uint32_t)((ac + 1) * OZ_BN + cb * 8), r[1]);
+            tmem_ld_wait();
 #pragma unroll
-          for (int j = 0; j < 8; ++j) {
-#pragma unroll
-            for (int acc = 0; acc < OZ_NACC; ++acc) df_add(hi[cb * 8 + j], lo[cb * 8 + j], __uint_as_float(r[acc][j]));
+            for (int j = 0; j < 8; ++j) {
+              df_add(hi[cb * 8 + j], lo[cb * 8 + j], __uint_as_float(r[0][j]));
+              df_add(hi[cb * 8 + j], lo[cb * 8 + j], __uint_as_float(r[1][j]));
+            }
           }
-        }
         // every load of this set has completed: hand it back to the MMA warp
         tc_fence_before();
         __syncwarp();
@@ -763,25 +837,43 @@ __global__ void __maxnreg__(96) oz_gemm_kernel(const OzGemmArgs g) {
         b ^= 1;
       }
       // C = alpha 2^(e_i + f_j - 16) (hi + lo) + beta C
-      if (row_ok) {
+      if (unit) {
+        // EC columns at a time without a branch between them, so that their
+        // conversions overlap; a pair outside the fast range (subnormal, overflow)
+        // sends them through the general conversion
+        constexpr int EC = 4;
+        double *cw = cp;
+#pragma unroll
+        for (int j0 = 0; j0 < OZ_EPI_COLS; j0 += EC) {
+          if (j0 == HALF && !beta0) load_c(HALF);
+          double v[EC];
+          bool slow = false;
+#pragma unroll
+          for (int j = 0; j < EC; ++j) {
+            // the sign of alpha goes onto the FP32 pair
+            hi[j0 + j] = __uint_as_float(__float_as_uint(hi[j0 + j]) ^ negmask);
+            lo[j0 + j] = __uint_as_float(__float_as_uint(lo[j0 + j]) ^ negmask);
+            const int sh = ea + __shfl_sync(0xffffffffu, eb, j0 + j) - 16;
+            v[j] = df2d_try(hi[j0 + j], lo[j0 + j], sh, slow);
+          }
+          if (__any_sync(0xffffffffu, slow)) {
+#pragma unroll
+            for (int j = 0; j < EC; ++j)
+              v[j] = df2d_scaled(hi[j0 + j], lo[j0 + j], ea + __shfl_sync(0xffffffffu, eb, j0 + j) - 16);
+          }
+#pragma unroll
+          for (int j = 0; j < EC; ++j) {
+            if (!beta0) v[j] = cv[(j0 + j) % HALF] + v[j];
+            if (j0 + j < ncol) *cw = v[j];
+            cw += g.ldc;
+          }
+        }
+      } else {
 #pragma unroll
         for (int j = 0; j < OZ_EPI_COLS; ++j) {
-          const int64_t col = col_base + j;
-          if (col < g.N && !(g.lower_only && my_row < col)) {
-            const int sh = ea + b_ex[col] - 16;
-            double out;
-            if (unit) {
-              // the sign of alpha goes onto the FP32 pair
-              const float h = __uint_as_float(__float_as_uint(hi[j]) ^ negmask);
-              const float l = __uint_as_float(__float_as_uint(lo[j]) ^ negmask);
-              const double v = df2d_scaled(h, l, sh);
-              out = beta0 ? v : cv[j] + v;
-            } else {
-              const double v = f2d_scaled(hi[j], sh) + f2d_scaled(lo[j], sh);
-              out = beta0 ? g.alpha * v : fma(g.alpha, v, g.beta * cv[j]);
-            }
-            crow[col * g.ldc] = out;
-          }
+          const int sh = ea + __shfl_sync(0xffffffffu, eb, j) - 16;
+          const double v = f2d_scaled(hi[j], sh) + f2d_scaled(lo[j], sh);
+          if (j < ncol) cp[j * g.ldc] = beta0 ? g.alpha * v : fma(g.alpha, v, g.beta * cp[j * g.ldc]);
         }
       }
     }
@@ -792,7 +884,7 @@ __global__ void __maxnreg__(96) oz_gemm_kernel(const OzGemmArgs g) {
   if (abort_sh) {
     // a wait ran out: let what was issued land (bounded) before the shared memory
     // and TMEM are released
-    if (warp == 1 && lane == 0 && mma_issued) {
+    if (warp == 1 && mma_issued && elect_one()) {
       umma_commit(bar(DRAIN));
       mbar_wait_bounded(bar(DRAIN), 0);
     }
@@ -827,19 +919,19 @@ void oz_gemm_batched(cudaStream_t s, const OzSplit &A, int64_t a_row0, const OzS
   OzGemmArgs g;
   g.a_sl = A.sl;
   g.a_ex = A.ex;
-  g.a_nrb = A.nrb;
-  g.a_nkc = 2 * A.nkb;
-  g.a_rb0 = a_row0 / OZ_TR;
+  g.a_nrb = (int)A.nrb;
+  g.a_nkc = (int)(2 * A.nkb);
+  g.a_rb0 = (int)(a_row0 / OZ_TR);
   g.b_sl = B.sl;
   g.b_ex = B.ex;
-  g.b_nrb = B.nrb;
-  g.b_nkc = 2 * B.nkb;
-  g.b_rb0 = b_row0 / OZ_TR;
-  g.M = M;
-  g.N = N;
+  g.b_nrb = (int)B.nrb;
+  g.b_nkc = (int)(2 * B.nkb);
+  g.b_rb0 = (int)(b_row0 / OZ_TR);
+  g.M = (int)M;
+  g.N = (int)N;
   // callers count K in 64-wide blocks; the kernel in 32-wide chunks
-  g.kc0 = 2 * kc0;
-  g.kc1 = std::min<int64_t>(2 * kc1, std::min(g.a_nkc, g.b_nkc));
+  g.kc0 = (int)(2 * kc0);
+  g.kc1 = (int)std::min<int64_t>(2 * kc1, std::min(g.a_nkc, g.b_nkc));
   g.kmode = kmode;
   g.alpha = alpha;
   g.beta = beta;
@@ -854,28 +946,27 @@ void oz_gemm_batched(cudaStream_t s, const OzSplit &A, int64_t a_row0, const OzS
   g.b_bs_ex = B.bstride_ex;
   g.c_bs = sC;
   g.status_bs = status_bs;
-  g.gx = (M + OZ_BM - 1) / OZ_BM;
-  g.gy = (N + OZ_BN - 1) / OZ_BN;
-  g.batch = batch;
-  const int64_t ntiles = g.gx * g.gy * batch;
-  const int64_t cap = tl_oz_grid_cap > 0 ? std::min(tl_oz_grid_cap, oz_sm_count()) : oz_sm_count();
-  const int64_t grid = std::min<int64_t>(ntiles, cap);
+  const int64_t gx = (M + OZ_BM - 1) / OZ_BM, gy = (N + OZ_BN - 1) / OZ_BN;
+  if (gx * gy * batch >= (int64_t)1 << 31 || M >= (int64_t)1 << 30 || N >= (int64_t)1 << 30)
+    throw CudaError{cudaErrorInvalidValue, "oz_gemm: too many tiles", __LINE__};
+  g.gx = (int)gx;
+  g.gy = (int)gy;
+  g.order = lower_only ? OZ_LOWER : kmode == 3 ? OZ_ROWS_UP : OZ_COLS;
+  g.per = lower_only ? oz_lower_tiles(g.gx, g.gy) : g.gx * g.gy;
+  g.ntiles = (int)(g.per * batch);
+  const int cap = tl_oz_grid_cap > 0 ? std::min(tl_oz_grid_cap, oz_sm_count()) : oz_sm_count();
+  const int grid = std::min(g.ntiles, cap);
   double fl = 0.0;
   if (tl_kt) {
-    // executed MMA arithmetic of the tiles the launch runs (the kernel's own tile
-    // skipping and K ranges; failed problems are not known on the host)
+    // executed MMA arithmetic of the tiles the launch runs (failed problems are not
+    // known on the host)
     const int prods = A.S == 5 ? 19 : 13;
-    for (int64_t bx = 0; bx < g.gx; ++bx)
-      for (int64_t by = 0; by < g.gy; ++by) {
-        const int64_t row0 = bx * OZ_BM, col0 = by * OZ_BN;
-        if (lower_only && col0 > row0 + OZ_BM - 1) continue;
-        const int64_t grow0 = g.a_rb0 * OZ_TR + row0, gcol0 = g.b_rb0 * OZ_TR + col0;
-        int64_t k0 = g.kc0, k1 = g.kc1;
-        if (kmode == 1) k0 = std::max(k0, std::max(grow0, gcol0) / OZ_TK);
-        if (kmode == 2) k0 = std::max(k0, gcol0 / OZ_TK);
-        if (kmode == 3) k1 = std::min(k1, (grow0 + OZ_BM + OZ_TK - 1) / OZ_TK);
-        if (k1 > k0) fl += 2.0 * OZ_BM * OZ_BN * OZ_TK * (double)(k1 - k0) * prods;
-      }
+    for (int r = 0; r < g.per; ++r) {
+      int bx, by, k0, k1;
+      oz_tile_xy(g.order, g.gx, g.gy, r, &bx, &by);
+      oz_krange(kmode, g.a_rb0 * OZ_TR + bx * OZ_BM, g.b_rb0 * OZ_TR + by * OZ_BN, g.kc0, g.kc1, &k0, &k1);
+      if (k1 > k0) fl += 2.0 * OZ_BM * OZ_BN * OZ_TK * (double)(k1 - k0) * prods;
+    }
     fl *= (double)batch;
   }
   {
@@ -896,7 +987,6 @@ void oz_gemm(cudaStream_t s, const OzSplit &A, int64_t a_row0, const OzSplit &B,
   oz_gemm_batched(s, A, a_row0, B, b_row0, M, N, kc0, kc1, kmode, alpha, beta, C, ldc, 0, lower_only,
                   err, status, 0, 1);
 }
-
 
 }  // namespace gpgp
 
