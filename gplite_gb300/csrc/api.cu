@@ -236,6 +236,8 @@ int64_t factor_and_solve(gpgp_model *m, Work &w, const double *zvec, double *alp
     Phase ph(ctx, GPGP_PHASE_POTRF);
     if (mixed)
       potrf_mixed(st, m->L.p, n, n, m->Winv.p, w.logdet_part.p, w.status.p, m->errflag.p, &ctx->side);
+    else if (n >= SLICED_MIN)
+      potrf_mixed(st, m->L.p, n, n, m->Winv.p, w.logdet_part.p, w.status.p, m->errflag.p, &ctx->side, OZ_FP64);
     else
       potrf(st, m->L.p, n, n, m->Winv.p, w.logdet_part.p, w.status.p, 1);
   }
@@ -297,6 +299,8 @@ void compute_linv(gpgp_model *m) {
   Phase ph(m->ctx, GPGP_PHASE_TRTRI);
   if (m->opts.precision == GPGP_PREC_MIXED) {
     trtri_mixed(st, m->L.p, n, n, m->Winv.p, m->Linv.p, n, m->errflag.p);
+  } else if (n >= SLICED_MIN) {
+    trtri_mixed(st, m->L.p, n, n, m->Winv.p, m->Linv.p, n, m->errflag.p, OZ_FP64);
   } else {
     DBuf tmp;
     tmp.alloc(st, (size_t)NB * n);
@@ -1190,7 +1194,10 @@ static gpgp_status pred_impl(gpgp_model *m, const double *xt, int64_t mt, uint32
         if (mixed) {
           trmv_sumsq_mixed(s, m->Linv.p, n, n, R.p, mc, n, csum.p + c0, m->errflag.p);
         } else {
-          trsm_lower(s, m->L.p, n, n, m->Winv.p, R.p, mc, n, tmp.p, status.p);
+          if (n >= SLICED_MIN)
+            trsm_sliced(s, m->L.p, n, n, m->Winv.p, R.p, mc, n, m->errflag.p, OZ_FP64);
+          else
+            trsm_lower(s, m->L.p, n, n, m->Winv.p, R.p, mc, n, tmp.p, status.p);
           col_sumsq(s, R.p, n, mc, n, csum.p + c0);
         }
       }
@@ -1331,6 +1338,8 @@ gpgp_status gpgp_model_grad(gpgp_model *m, double *grad_terms, double *grad_lik_
       Phase ph(ctx, GPGP_PHASE_LAUUM);
       if (m->opts.precision == GPGP_PREC_MIXED)
         lauum_mixed(s, m->Linv.p, n, n, Bi.p, n, m->errflag.p);
+      else if (n >= SLICED_MIN)
+        lauum_mixed(s, m->Linv.p, n, n, Bi.p, n, m->errflag.p, OZ_FP64);
       else
         gemm64(s, true, false, n, n, n, 1.0, m->Linv.p, n, m->Linv.p, n, 0.0, Bi.p, n, true, 1);
     }

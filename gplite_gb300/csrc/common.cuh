@@ -294,12 +294,17 @@ void getrs(cudaStream_t s, const double *LU, int64_t n, int64_t lda, const int *
 // ---------------------------------------------------------------------------
 // mixed precision (mixed.cu / mixed_la.cu): BF16-sliced operands for tcgen05
 // ---------------------------------------------------------------------------
+constexpr int OZ_FP64 = 8;
+#ifndef GPGP_SLICED_MIN
+#define GPGP_SLICED_MIN 960
+#endif
+constexpr int64_t SLICED_MIN = GPGP_SLICED_MIN;
 struct OzSplit {
   int *ex = nullptr;        // per-row power-of-two exponents (rows padded)
   uint16_t *sl = nullptr;   // BF16 slices, pre-tiled for UMMA
   int64_t rows = 0, K = 0, nrb = 0, nkb = 0;
   int64_t bstride_ex = 0, bstride_sl = 0;  // batched operands: per-problem strides
-  int S = 4;  // slices (8S-bit fixed point); both operands of a product use the same S
+  int S = 4;  // slices (4, 5: 8S-bit fixed point; OZ_FP64: 63-bit); both operands of a product use the same S
 };
 int64_t oz_nrb(int64_t rows);
 size_t oz_split_bytes(int64_t rows, int64_t K, int S = 4);
@@ -339,16 +344,21 @@ void oz_gemm_batched(cudaStream_t s, const OzSplit &A, int64_t a_row0, const OzS
                      double beta, double *C, int64_t ldc, int64_t sC, bool lower_only, int *err,
                      const int *status, int64_t status_bs, int64_t batch);
 
-// Mixed-precision factorisation and inverses (same outputs as the FP64 versions).
+// Sliced factorisation and inverses (same outputs as the FP64 pipe's): with S = 4 the
+// mixed precision, with S = OZ_FP64 (63 bits below each row's largest entry, as accurate as
+// the FP64 pipe) the FP64 path of n >= SLICED_MIN.
 // With a side stream, panel p + 1 is factored on it while the main stream
 // finishes the trailing update of panel p (identical results).
 void potrf_mixed(cudaStream_t s, double *A, int64_t n, int64_t lda, double *Winv,
-                 double *logdet_part, int *status, int *err, const SideStream *side = nullptr);
+                 double *logdet_part, int *status, int *err, const SideStream *side = nullptr, int S = 4);
 void trtri_mixed(cudaStream_t s, const double *L, int64_t n, int64_t lda, const double *Winv,
-                 double *W, int64_t ldw, int *err);
+                 double *W, int64_t ldw, int *err, int S = 4);
 // Binv (lower) = W^T W for lower-triangular W
 void lauum_mixed(cudaStream_t s, const double *W, int64_t n, int64_t ldw, double *Binv,
-                 int64_t ldb, int *err);
+                 int64_t ldb, int *err, int S = 4);
+// X = L^-1 R in place (n x m, leading dimension ldr)
+void trsm_sliced(cudaStream_t s, const double *L, int64_t n, int64_t lda, const double *Winv, double *R, int64_t m,
+                 int64_t ldr, int *err, int S);
 // T = W R (W lower n x n, R n x m), then out[j] = sum_i T_ij^2
 void trmv_sumsq_mixed(cudaStream_t s, const double *W, int64_t n, int64_t ldw, const double *R,
                       int64_t m, int64_t ldr, double *out, int *err);

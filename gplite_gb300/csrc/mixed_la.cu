@@ -35,14 +35,14 @@ struct SplitBuf {
   void *p = nullptr;
   cudaStream_t s = nullptr;
   OzSplit sp;
-  SplitBuf(cudaStream_t st, int64_t rows, int64_t K) : s(st) {
-    const size_t b = oz_split_bytes(rows, K);
+  SplitBuf(cudaStream_t st, int64_t rows, int64_t K, int S) : s(st) {
+    const size_t b = oz_split_bytes(rows, K, S);
     if (cudaMallocAsync(&p, b, st) != cudaSuccess) {
       p = nullptr;
       (void)cudaGetLastError();
       throw std::bad_alloc();
     }
-    oz_split_bind(p, rows, K, &sp);
+    oz_split_bind(p, rows, K, &sp, S);
   }
   ~SplitBuf() {
     if (p) cudaFreeAsync(p, s);
@@ -118,10 +118,10 @@ void factor_panel(cudaStream_t x, cudaStream_t y, const SideStream *sd, double *
 }  // namespace
 
 void potrf_mixed(cudaStream_t s, double *A, int64_t n, int64_t lda, double *Winv,
-                 double *logdet_part, int *status, int *err, const SideStream *side) {
-  SplitBuf a(s, n, NBO);   // panel operand (rows below the current block)
-  SplitBuf w(s, NB, NB);   // inverse of the diagonal block
-  SplitBuf lp(s, NBO, NB);  // the block's rows inside the panel
+                 double *logdet_part, int *status, int *err, const SideStream *side, int S) {
+  SplitBuf a(s, n, NBO, S);    // panel operand (rows below the current block)
+  SplitBuf w(s, NB, NB, S);    // inverse of the diagonal block
+  SplitBuf lp(s, NBO, NB, S);  // the block's rows inside the panel
   cudaStreamCaptureStatus cap_st = cudaStreamCaptureStatusNone;
   GPGP_CUDA(cudaStreamIsCapturing(s, &cap_st));
   // Per-kernel timers (tl_kt) time each launch alone, so a profiled call runs the
@@ -145,7 +145,7 @@ void potrf_mixed(cudaStream_t s, double *A, int64_t n, int64_t lda, double *Winv
   // (event a), and then applies p to the rest of the trailing matrix while panel
   // p + 1 is factored beside it (the two touch disjoint columns). Every product
   // is the one the plain schedule computes, so the factor is the same.
-  SplitBuf t(s, n, NBO);  // panel p as the trailing update's operand
+  SplitBuf t(s, n, NBO, S);  // panel p as the trailing update's operand
   cudaStream_t x = side->s;
   GPGP_CUDA(cudaEventRecord(side->fork, s));
   GPGP_CUDA(cudaStreamWaitEvent(x, side->fork, 0));
@@ -218,14 +218,14 @@ struct SplitBatch {
   void *p = nullptr;
   cudaStream_t s = nullptr;
   OzSplit sp;
-  SplitBatch(cudaStream_t st, int64_t rows, int64_t K, int64_t count) : s(st) {
-    const size_t per = (oz_split_bytes(rows, K) + 1023) / 1024 * 1024;
+  SplitBatch(cudaStream_t st, int64_t rows, int64_t K, int64_t count, int S) : s(st) {
+    const size_t per = (oz_split_bytes(rows, K, S) + 1023) / 1024 * 1024;
     if (cudaMallocAsync(&p, per * count, st) != cudaSuccess) {
       p = nullptr;
       (void)cudaGetLastError();
       throw std::bad_alloc();
     }
-    oz_split_bind(p, rows, K, &sp);
+    oz_split_bind(p, rows, K, &sp, S);
     sp.bstride_ex = (int64_t)(per / sizeof(int));
     sp.bstride_sl = (int64_t)(per / sizeof(uint16_t));
   }
@@ -238,17 +238,17 @@ struct SplitBatch {
 // offsets k b (k < count), whose two halves are already inverted:
 // W21 = -W22 (L21 W11), all blocks of the level in two batched GEMMs.
 static void trtri_level(cudaStream_t s, const double *L, int64_t lda, double *W, int64_t ldw, int64_t b,
-                        int64_t count, double *T, int *err) {
+                        int64_t count, double *T, int *err, int S) {
   const int64_t h = b / 2;
   {
-    SplitBatch a(s, h, h, count), bb(s, h, h, count);
+    SplitBatch a(s, h, h, count, S), bb(s, h, h, count, S);
     oz_split_batched(s, L + h, lda, b * (lda + 1), 0, h, h, &a.sp, count);
     oz_split_batched(s, W, ldw, b * (ldw + 1), 1, h, h, &bb.sp, count);
     oz_gemm_batched(s, a.sp, 0, bb.sp, 0, h, h, 0, bb.sp.nkb, 2, 1.0, 0.0, T, h, h * h, false, err, nullptr, 0,
                     count);
   }
   {
-    SplitBatch a(s, h, h, count), bb(s, h, h, count);
+    SplitBatch a(s, h, h, count, S), bb(s, h, h, count, S);
     oz_split_batched(s, W + h + h * ldw, ldw, b * (ldw + 1), 0, h, h, &a.sp, count);
     oz_split_batched(s, T, h, h * h, 1, h, h, &bb.sp, count);
     oz_gemm_batched(s, a.sp, 0, bb.sp, 0, h, h, 0, a.sp.nkb, 3, -1.0, 0.0, W + h, ldw, b * (ldw + 1), false, err,
@@ -261,24 +261,24 @@ static void trtri_level(cudaStream_t s, const double *L, int64_t lda, double *W,
 // blocks from the batched levels) are skipped; above the base the split points
 // are multiples of the base so that its blocks line up.
 static void trtri_rec(cudaStream_t s, const double *L, int64_t n, int64_t lda, int64_t off, int64_t ntot,
-                      double *W, int64_t ldw, double *T, int *err) {
+                      double *W, int64_t ldw, double *T, int *err, int S) {
   if (n <= NB) return;
   if ((n == 128 || n == 256 || n == TRTRI_BASE) && off % n == 0 && off + n <= ntot) return;
   const int64_t g = n > TRTRI_BASE ? TRTRI_BASE : NB;
   const int64_t n1 = ((n / 2) + g - 1) / g * g;
   const int64_t n2 = n - n1;
-  trtri_rec(s, L, n1, lda, off, ntot, W, ldw, T, err);
-  trtri_rec(s, L + n1 + n1 * lda, n2, lda, off + n1, ntot, W + n1 + n1 * ldw, ldw, T, err);
+  trtri_rec(s, L, n1, lda, off, ntot, W, ldw, T, err, S);
+  trtri_rec(s, L + n1 + n1 * lda, n2, lda, off + n1, ntot, W + n1 + n1 * ldw, ldw, T, err, S);
   // T = L21 W11  (n2 x n1): A = L21 (rows n2, K n1), B rows j = columns of W11 (W11[k, j], k >= j)
   {
-    SplitBuf a(s, n2, n1), b(s, n1, n1);
+    SplitBuf a(s, n2, n1, S), b(s, n1, n1, S);
     oz_split(s, L + n1, lda, 0, n2, n1, &a.sp);
     oz_split(s, W, ldw, 1, n1, n1, &b.sp);
     oz_gemm(s, a.sp, 0, b.sp, 0, n2, n1, 0, b.sp.nkb, 2, 1.0, 0.0, T, n2, false, err);
   }
   // W21 = -W22 T  (n2 x n1): A = W22 (rows n2, K n2, lower: k <= i), B rows j = columns of T
   {
-    SplitBuf a(s, n2, n2), b(s, n1, n2);
+    SplitBuf a(s, n2, n2, S), b(s, n1, n2, S);
     oz_split(s, W + n1 + n1 * ldw, ldw, 0, n2, n2, &a.sp);
     oz_split(s, T, n2, 1, n1, n2, &b.sp);
     oz_gemm(s, a.sp, 0, b.sp, 0, n2, n1, 0, a.sp.nkb, 3, -1.0, 0.0, W + n1, ldw, false, err);
@@ -293,7 +293,7 @@ __global__ void zero_upper_kernel(double *W, int64_t n, int64_t ldw) {
 }
 
 void trtri_mixed(cudaStream_t s, const double *L, int64_t n, int64_t lda, const double *Winv,
-                 double *W, int64_t ldw, int *err) {
+                 double *W, int64_t ldw, int *err, int S) {
   if (n <= 0) return;
   dim3 g((unsigned)std::min<int64_t>((n + 255) / 256, 64), (unsigned)std::min<int64_t>(n, 65535));
   zero_upper_kernel<<<g, 256, 0, s>>>(W, n, ldw);
@@ -309,8 +309,8 @@ void trtri_mixed(cudaStream_t s, const double *L, int64_t n, int64_t lda, const 
   try {
     // the full aligned diagonal blocks of 128, 256 and 512, all blocks of a size at once
     for (int64_t b = 2 * NB; b <= TRTRI_BASE; b *= 2)
-      if (n / b > 0) trtri_level(s, L, lda, W, ldw, b, n / b, T, err);
-    trtri_rec(s, L, n, lda, 0, n, W, ldw, T, err);
+      if (n / b > 0) trtri_level(s, L, lda, W, ldw, b, n / b, T, err, S);
+    trtri_rec(s, L, n, lda, 0, n, W, ldw, T, err, S);
   } catch (...) {
     cudaFreeAsync(T, s);
     throw;
@@ -319,11 +319,48 @@ void trtri_mixed(cudaStream_t s, const double *L, int64_t n, int64_t lda, const 
 }
 
 void lauum_mixed(cudaStream_t s, const double *W, int64_t n, int64_t ldw, double *Binv,
-                 int64_t ldb, int *err) {
+                 int64_t ldb, int *err, int S) {
   // Binv_ij = sum_k W_ki W_kj (k >= max(i, j)); operand rows = columns of W
-  SplitBuf a(s, n, n);
+  SplitBuf a(s, n, n, S);
   oz_split(s, W, ldw, 1, n, n, &a.sp);
   oz_gemm(s, a.sp, 0, a.sp, 0, n, n, 0, a.sp.nkb, 1, 1.0, 0.0, Binv, ldb, true, err);
+}
+
+// X = L^-1 R in place (n x m), right-looking on two levels: a 64-row block is
+// multiplied by its diagonal block's inverse and updates the rest of its outer block of
+// TRSM_OUTER rows (K = 64); the rows below take one product with K = TRSM_OUTER, so
+// that they are rewritten n / TRSM_OUTER times. Inverses of larger diagonal blocks would
+// need fewer launches, but 128-row ones made the predictive variance 1.6 times and
+// 512-row ones 4 times less accurate.
+constexpr int64_t TRSM_OUTER = 512;
+
+void trsm_sliced(cudaStream_t s, const double *L, int64_t n, int64_t lda, const double *Winv, double *R, int64_t m,
+                 int64_t ldr, int *err, int S) {
+  if (n <= 0 || m <= 0) return;
+  const int64_t nblk = (n + NB - 1) / NB;
+  SplitBatch w(s, NB, NB, nblk, S);  // the diagonal blocks' inverses, split at once
+  oz_split_batched(s, Winv, NB, NB * NB, 0, NB, NB, &w.sp, nblk);
+  SplitBuf a(s, n, TRSM_OUTER, S), x(s, m, TRSM_OUTER, S);
+  for (int64_t o0 = 0; o0 < n; o0 += TRSM_OUTER) {
+    const int64_t oend = std::min<int64_t>(o0 + TRSM_OUTER, n);
+    for (int64_t k0 = o0; k0 < oend; k0 += NB) {
+      const int64_t kb = std::min<int64_t>(NB, n - k0), rest = oend - k0 - kb;
+      OzSplit wk = w.sp;
+      wk.ex += k0 / NB * wk.bstride_ex;
+      wk.sl += k0 / NB * wk.bstride_sl;
+      oz_split(s, R + k0, ldr, 1, m, kb, &x.sp);
+      oz_gemm(s, wk, 0, x.sp, 0, kb, m, 0, 1, 0, 1.0, 0.0, R + k0, ldr, false, err);
+      if (rest <= 0) break;
+      oz_split(s, R + k0, ldr, 1, m, kb, &x.sp);
+      oz_split(s, L + (k0 + kb) + k0 * lda, lda, 0, rest, kb, &a.sp);
+      oz_gemm(s, a.sp, 0, x.sp, 0, rest, m, 0, 1, 0, -1.0, 1.0, R + k0 + kb, ldr, false, err);
+    }
+    const int64_t below = n - oend;
+    if (below <= 0) break;
+    oz_split(s, R + o0, ldr, 1, m, oend - o0, &x.sp);
+    oz_split(s, L + oend + o0 * lda, lda, 0, below, oend - o0, &a.sp);
+    oz_gemm(s, a.sp, 0, x.sp, 0, below, m, 0, a.sp.nkb, 0, -1.0, 1.0, R + oend, ldr, false, err);
+  }
 }
 
 void trmv_sumsq_mixed(cudaStream_t s, const double *W, int64_t n, int64_t ldw, const double *R,
@@ -335,7 +372,7 @@ void trmv_sumsq_mixed(cudaStream_t s, const double *W, int64_t n, int64_t ldw, c
     throw std::bad_alloc();
   }
   {
-    SplitBuf a(s, n, n), b(s, m, n);
+    SplitBuf a(s, n, n, 4), b(s, m, n, 4);
     oz_split(s, W, ldw, 0, n, n, &a.sp);
     oz_split(s, R, ldr, 1, m, n, &b.sp);
     oz_gemm(s, a.sp, 0, b.sp, 0, n, m, 0, a.sp.nkb, 3, 1.0, 0.0, T, n, false, err);
@@ -391,7 +428,7 @@ __global__ void max_abs_kernel(const double *a, const double *b, int64_t n, doub
 extern "C" gpgp_status gpgp_mixed_selftest(gpgp_ctx *ctx, int64_t M, int64_t N, int64_t K,
                                            int32_t slices, double *max_rel_err) {
   using namespace gpgp;
-  if (!ctx || M < 1 || N < 1 || K < 1 || !max_rel_err || (slices != 4 && slices != 5))
+  if (!ctx || M < 1 || N < 1 || K < 1 || !max_rel_err || (slices != 4 && slices != 5 && slices != OZ_FP64))
     return GPGP_EINVAL;
   cudaStream_t s = (cudaStream_t)gpgp_stream(ctx);
   KTBind bind(ctx);

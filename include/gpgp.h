@@ -494,7 +494,8 @@ gpgp_status gpgp_fit_gaussian_noalloc(gpgp_ctx *ctx, const gpgp_kernel *k, doubl
  *      M x K and N x K operands with entries spread over 2^8 in magnitude,
  *      computed with the BF16-sliced tensor-core GEMM and with the FP64 GEMM;
  *      returns max |difference| / max |C|. slices is 4 (32-bit fixed point,
- *      the factorisation path) or 5 (40-bit, the batched path). ---- */
+ *      the mixed factorisation), 5 (40-bit, the batched path) or 8 (63-bit, the
+ *      FP64 path of large n). ---- */
 gpgp_status gpgp_mixed_selftest(gpgp_ctx *ctx, int64_t M, int64_t N, int64_t K, int32_t slices,
                                 double *max_rel_err);
 
