@@ -1298,8 +1298,11 @@ static gpgp_status loo_impl(gpgp_model *m, int32_t quad_order, int64_t draws, co
       lik_loo_gh(s, m->lk, n, quad_order, ghx.p, ghw.p, mp, vp, m->y.p,
                  m->has_trials ? m->trials.p : nullptr, m->has_offset ? m->offset.p : nullptr, out.p);
     }
+    int herr = 0;
+    GPGP_CUDA(cudaMemcpyAsync(&herr, m->errflag.p, sizeof(int), cudaMemcpyDeviceToHost, s));
     GPGP_CUDA(cudaMemcpyAsync(loos, out.p, n * sizeof(double), cudaMemcpyDeviceToHost, s));
     GPGP_CUDA(cudaStreamSynchronize(s));
+    if (herr) return fail(ctx, GPGP_ETIMEOUT, "a tensor-core kernel wait timed out");
     if (loo_sum) {
       double acc = 0.0;
       for (int64_t i = 0; i < n; ++i) acc += loos[i];

@@ -263,7 +263,7 @@ void trsv_flow(cudaStream_t s, const double *L, int64_t n, int64_t lda, const do
 // backsolve: rows of the n x M matrix B (mode 0: X = B L^-T, mode 1: X = B L^-1),
 // and vectors (x = L^-1 b, or L^-T b when trans).
 void tri_rows(cudaStream_t s, const double *L, int64_t M, int64_t ldl, const double *B, int64_t ldb,
-              double *X, int64_t ldx, int64_t n, int mode);
+              double *X, int64_t ldx, int64_t n, int mode, int *err = nullptr);
 void tri_vec(cudaStream_t s, const double *L, int64_t M, int64_t ldl, const double *b, double *x,
              bool trans);
 // B <- L^-1 B (n x m, ldb); tmp holds NB * m doubles.
@@ -309,9 +309,46 @@ struct OzSplit {
 int64_t oz_nrb(int64_t rows);
 size_t oz_split_bytes(int64_t rows, int64_t K, int S = 4);
 void oz_split_bind(void *mem, int64_t rows, int64_t K, OzSplit *out, int S = 4);
+// Stream-ordered scratch for a split operand (freed when the scope ends).
+struct SplitBuf {
+  void *p = nullptr;
+  cudaStream_t s = nullptr;
+  OzSplit sp;
+  explicit SplitBuf(cudaStream_t st) : s(st) {}
+  SplitBuf(cudaStream_t st, int64_t rows, int64_t K, int S) : s(st) { bind(rows, K, S); }
+  SplitBuf(const SplitBuf &) = delete;
+  SplitBuf &operator=(const SplitBuf &) = delete;
+  void bind(int64_t rows, int64_t K, int S) {
+    const size_t b = oz_split_bytes(rows, K, S);
+    if (cudaMallocAsync(&p, b, s) != cudaSuccess) {
+      p = nullptr;
+      (void)cudaGetLastError();
+      throw std::bad_alloc();
+    }
+    oz_split_bind(p, rows, K, &sp, S);
+  }
+  ~SplitBuf() {
+    if (p) cudaFreeAsync(p, s);
+  }
+};
 // rows x K operand: element (r, k) = P[r + k*ld] (trans 0) or P[k + r*ld] (trans 1)
 void oz_split(cudaStream_t s, const double *P, int64_t ld, int trans, int64_t rows, int64_t K,
               OzSplit *out);
+// C = alpha A B^T + beta C for many rows (n x N, alpha 1 or -1, beta 0 or 1)
+void rows_times_bt(cudaStream_t s, int64_t n, int64_t N, int64_t K, double alpha, const double *A, int64_t lda,
+                   const double *B, int64_t ldb, double beta, double *C, int64_t ldc, int *err);
+// C = A^T B (M x N) for tall A (n x M) and B (n x N), at FP64 accuracy: n split over the
+// SMs, 8-slice products, partials summed in a fixed order
+void gram_sliced(cudaStream_t s, const double *A, int64_t lda, const double *B, int64_t ldb, int64_t n, int64_t M,
+                 int64_t N, double *C, int64_t ldc, int *err);
+// C = alpha sum_z P_z + beta C over nz M x N partials (fixed order)
+void splitk_reduce(cudaStream_t s, int64_t M, int64_t N, int nz, const double *P, double alpha, double beta,
+                   double *C, int64_t ldc, bool lower_only);
+// rows from which a product of many rows with a 64-wide K takes the tensor cores at FP64
+// accuracy (4096 x 192: 84 us on the FP64 pipe, ~20 with the two splits; 1000 rows: 20 us)
+constexpr int64_t SLICED_ROWS = 1024;
+// rows from which a Gram product takes gram_sliced
+constexpr int64_t GRAM_SLICED_MIN = 4096;
 // C = alpha A B^T + beta C on K chunks [kc0, kc1) (64 wide); a_row0/b_row0 multiples of 64.
 // kmode: 0 all chunks; 1 start at max(row, col); 2 start at col; 3 stop after row.
 // status (optional): the launch is skipped for a problem whose word is nonzero; the

@@ -137,6 +137,13 @@ __global__ void splitk_reduce_kernel(int64_t M, int64_t N, int nz, const double 
   }
 }
 
+void splitk_reduce(cudaStream_t s, int64_t M, int64_t N, int nz, const double *P, double alpha, double beta,
+                   double *C, int64_t ldc, bool lower_only) {
+  splitk_reduce_kernel<<<(unsigned)std::min<int64_t>((M * N + 255) / 256, 4096), 256, 0, s>>>(
+      M, N, nz, P, alpha, beta, C, ldc, lower_only ? 1 : 0);
+  GPGP_CHECK_LAUNCH();
+}
+
 template <bool TA, bool TB>
 static void launch_gemm64(cudaStream_t s, dim3 grid, int64_t M, int64_t N, int64_t K, double alpha,
                           const double *A, int64_t lda, const double *B, int64_t ldb, double beta, double *C,
@@ -215,10 +222,7 @@ void gemm64_batched(cudaStream_t s, bool ta, bool tb, int64_t M, int64_t N, int6
     GPGP_CUDA(cudaMallocAsync((void **)&P, (size_t)nz * M * N * sizeof(double), s));
     dim3 g2(grid.x, grid.y, (unsigned)nz);
     gemm64_dispatch(s, ta, tb, g2, M, N, K, 1.0, A, lda, B, ldb, 0.0, P, M, 0, tri_mode, 0, 0, M * N, kchunk);
-    const int64_t MN = M * N;
-    splitk_reduce_kernel<<<(unsigned)std::min<int64_t>((MN + 255) / 256, 4096), 256, 0, s>>>(
-        M, N, (int)nz, P, alpha, beta, C, ldc, lo);
-    GPGP_CHECK_LAUNCH();
+    splitk_reduce(s, M, N, (int)nz, P, alpha, beta, C, ldc, lower_only);
     GPGP_CUDA(cudaFreeAsync(P, s));
     return;
   }
@@ -432,9 +436,191 @@ __global__ void __launch_bounds__(DIAG_THREADS) potrf_diag_kernel(double *__rest
   if (tid == 0) *logdet_part = lg[0];
 }
 
-// panel: L21 = A21 L11^-T by forward substitution, one row per thread (in place).
-// Substitution keeps the factorisation backward stable when a diagonal block is
-// ill-conditioned (FITC's K_z); the inverse W is used by the solves instead.
+// ---------------------------------------------------------------------------
+// substitution solves for small factors (M x M lower L), as R's forwardsolve /
+// backsolve do, on the rows of a column-major n x M matrix
+// ---------------------------------------------------------------------------
+// mode 0: X = B L^-T (x L^T = b, forward); mode 1: X = B L^-1 (x L = b, backward).
+// Blocked in TB columns: a block's columns are solved by substitution, then the columns
+// still to come take one product with them, so that most of the n M^2 / 2 multiply-adds
+// are a GEMM's. (One thread per row over all M columns, as before, is one chain of M^2 / 2
+// FP64 instructions: 1.6 ms for 256 rows of M = 256, and 65536 rows took 8.1 ms.)
+constexpr int TB = 64;
+
+// One block: rows of X (n x kb, in place) against the kb x kb lower block L. The lanes
+// of a warp share few rows: lane q of a group of eight owns columns q, q + 8, .. of its
+// row, so that an FP64 instruction (64 cycles of its sub-partition, whatever the number
+// of active lanes) works on four rows and eight columns.
+template <int MODE>
+__global__ void __launch_bounds__(128) tri_block_kernel(const double *__restrict__ L, int64_t ldl, int kb,
+                                                        double *__restrict__ X, int64_t ldx, int64_t n,
+                                                        const int *__restrict__ status) {
+  if (status && *(volatile const int *)status != 0) return;
+  __shared__ double Ls[TB][TB + 1];  // [c][r] = L(r, c): a step reads one column (mode 0) or row (mode 1)
+  __shared__ double rd[TB];
+  for (int idx = threadIdx.x; idx < TB * TB; idx += 128) {
+    const int r = idx % TB, c = idx / TB;
+    Ls[c][r] = (r < kb && c < kb && r >= c) ? L[r + c * ldl] : 0.0;
+  }
+  __syncthreads();
+  if (threadIdx.x < TB) rd[threadIdx.x] = threadIdx.x < kb ? 1.0 / Ls[threadIdx.x][threadIdx.x] : 0.0;
+  __syncthreads();
+  const int lane = threadIdx.x & 31, q = lane & 7;
+  const int64_t i = ((int64_t)blockIdx.x * 4 + (threadIdx.x >> 5)) * 4 + (lane >> 3);
+  double x[TB / 8];
+#pragma unroll
+  for (int t = 0; t < TB / 8; ++t) {
+    const int c = 8 * t + q;
+    x[t] = (i < n && c < kb) ? X[i + c * ldx] : 0.0;
+  }
+#pragma unroll
+  for (int s0 = 0; s0 < TB / 8; ++s0) {
+    const int t0 = MODE == 0 ? s0 : TB / 8 - 1 - s0;  // the eight columns 8 t0 ..
+#pragma unroll
+    for (int s1 = 0; s1 < 8; ++s1) {
+      const int cq = MODE == 0 ? s1 : 7 - s1, c = 8 * t0 + cq;
+      // the owner's value scaled by 1 / L(c, c); a column past kb holds zeros and has rd = 0
+      const double xc = __shfl_sync(0xffffffffu, x[t0] * rd[c], cq, 8);
+      if (q == cq) x[t0] = xc;
+      else if (MODE == 0 ? q > cq : q < cq) x[t0] = fma(-xc, MODE == 0 ? Ls[c][8 * t0 + q] : Ls[8 * t0 + q][c], x[t0]);
+#pragma unroll
+      for (int t = MODE == 0 ? t0 + 1 : 0; t < (MODE == 0 ? TB / 8 : t0); ++t)
+        x[t] = fma(-xc, MODE == 0 ? Ls[c][8 * t + q] : Ls[8 * t + q][c], x[t]);
+    }
+  }
+  if (i < n)
+#pragma unroll
+    for (int t = 0; t < TB / 8; ++t) {
+      const int c = 8 * t + q;
+      if (c < kb) X[i + c * ldx] = x[t];
+    }
+}
+
+// C = alpha A B^T + beta C (n x N, alpha 1 or -1, beta 0 or 1) for many rows n: on the
+// tensor cores at FP64 accuracy from SLICED_ROWS rows on.
+void rows_times_bt(cudaStream_t s, int64_t n, int64_t N, int64_t K, double alpha, const double *A, int64_t lda,
+                   const double *B, int64_t ldb, double beta, double *C, int64_t ldc, int *err) {
+  if (n < SLICED_ROWS) {
+    gemm64(s, false, true, n, N, K, alpha, A, lda, B, ldb, beta, C, ldc);
+    return;
+  }
+  SplitBuf a(s, n, K, OZ_FP64), b(s, N, K, OZ_FP64);
+  oz_split(s, A, lda, 0, n, K, &a.sp);
+  oz_split(s, B, ldb, 0, N, K, &b.sp);
+  oz_gemm(s, a.sp, 0, b.sp, 0, n, N, 0, a.sp.nkb, 0, alpha, beta, C, ldc, false, err);
+}
+
+// X may alias B. err (optional): the products of many rows then go through the sliced
+// tensor-core GEMM, whose bounded waits report there.
+void tri_rows(cudaStream_t s, const double *L, int64_t M, int64_t ldl, const double *B, int64_t ldb,
+              double *X, int64_t ldx, int64_t n, int mode, int *err) {
+  if (n <= 0 || M <= 0) return;
+  if (X != B)
+    GPGP_CUDA(cudaMemcpy2DAsync(X, ldx * sizeof(double), B, ldb * sizeof(double), n * sizeof(double), M,
+                                cudaMemcpyDeviceToDevice, s));
+  const unsigned grid = (unsigned)((n + 15) / 16);
+  const bool sliced = err && n >= SLICED_ROWS;
+  SplitBuf xs(s), ls(s);
+  if (sliced && M > TB) {
+    xs.bind(n, TB, OZ_FP64);
+    ls.bind(M, TB, OZ_FP64);
+  }
+  const int64_t nblk = (M + TB - 1) / TB;
+  for (int64_t b = 0; b < nblk; ++b) {
+    const int64_t k0 = (mode == 0 ? b : nblk - 1 - b) * TB;
+    const int kb = (int)std::min<int64_t>(TB, M - k0);
+    double *Xk = X + k0 * ldx;
+    if (mode == 0) tri_block_kernel<0><<<grid, 128, 0, s>>>(L + k0 * (ldl + 1), ldl, kb, Xk, ldx, n, nullptr);
+    else tri_block_kernel<1><<<grid, 128, 0, s>>>(L + k0 * (ldl + 1), ldl, kb, Xk, ldx, n, nullptr);
+    GPGP_CHECK_LAUNCH();
+    // the columns after the block (mode 0: X_rest -= X_k L_rest,k^T) or before it
+    // (mode 1: X_rest -= X_k L_k,rest)
+    const int64_t rest = mode == 0 ? M - k0 - kb : k0;
+    if (rest <= 0) continue;
+    double *Xr = mode == 0 ? X + (k0 + kb) * ldx : X;
+    const double *Lr = mode == 0 ? L + (k0 + kb) + k0 * ldl : L + k0;
+    if (sliced) {
+      oz_split(s, Xk, ldx, 0, n, kb, &xs.sp);
+      oz_split(s, Lr, ldl, mode == 0 ? 0 : 1, rest, kb, &ls.sp);
+      oz_gemm(s, xs.sp, 0, ls.sp, 0, n, rest, 0, 1, 0, -1.0, 1.0, Xr, ldx, false, err);
+    } else {
+      gemm64(s, false, mode == 0, n, rest, kb, -1.0, Xk, ldx, Lr, ldl, 1.0, Xr, ldx);
+    }
+  }
+}
+
+// x = L^-1 b (trans = 0) or x = L^-T b (trans = 1), x may alias b: one CTA, 32 rows at a
+// time. Warp 0 solves the diagonal block in registers (one row per lane) while the other
+// rows' entries of the block's columns are already in flight; then every row still to
+// come takes its 32 multiply-adds at once. (A row's dot product by one warp, row after
+// row, was a chain of shuffles and FP64 latencies: 500 us at M = 256.)
+constexpr int TV = 32, TV_THREADS = 256;
+
+__global__ void __launch_bounds__(TV_THREADS) tri_vec_kernel(const double *__restrict__ L, int64_t M, int64_t ldl,
+                                                             const double *b, double *x, int trans) {
+  __shared__ double D[TV][TV + 1];  // the diagonal block, D[c][r] = L(r, c)
+  __shared__ double xs[TV];
+  const int tid = threadIdx.x, lane = tid & 31;
+  if (x != b)
+    for (int64_t r = tid; r < M; r += TV_THREADS) x[r] = b[r];
+  const int64_t nblk = (M + TV - 1) / TV;
+  for (int64_t st = 0; st < nblk; ++st) {
+    const int64_t k0 = (trans ? nblk - 1 - st : st) * TV;
+    const int kb = (int)(M - k0 < TV ? M - k0 : TV);
+    for (int idx = tid; idx < TV * TV; idx += TV_THREADS) {
+      const int r = idx % TV, c = idx / TV;
+      D[c][r] = (r < kb && c < kb && r >= c) ? L[(k0 + r) + (k0 + c) * ldl] : 0.0;
+    }
+    // rows after the block (trans: before it); this thread's first row is loaded now
+    const int64_t r0 = trans ? 0 : k0 + kb, r1 = trans ? k0 : M;
+    const int64_t r = r0 + tid;
+    double l[TV];
+#pragma unroll
+    for (int c = 0; c < TV; ++c)
+      l[c] = (r < r1 && c < kb) ? (trans ? L[(k0 + c) + r * ldl] : L[r + (k0 + c) * ldl]) : 0.0;
+    __syncthreads();
+    if (tid < 32) {
+      double v = lane < kb ? x[k0 + lane] : 0.0;
+      const double rd = lane < kb ? 1.0 / D[lane][lane] : 0.0;
+      for (int t = 0; t < kb; ++t) {
+        const int c = trans ? kb - 1 - t : t;
+        const double xc = __shfl_sync(0xffffffffu, v * rd, c);
+        if (lane == c) v = xc;
+        else if (trans ? lane < c : lane > c) v = fma(-xc, trans ? D[lane][c] : D[c][lane], v);
+      }
+      xs[lane] = v;
+      if (lane < kb) x[k0 + lane] = v;
+    }
+    __syncthreads();
+    if (r < r1) {
+      double a[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+      for (int c = 0; c < TV; ++c) a[c & 3] = fma(l[c], xs[c], a[c & 3]);
+      x[r] -= (a[0] + a[1]) + (a[2] + a[3]);
+    }
+    for (int64_t rr = r + TV_THREADS; rr < r1; rr += TV_THREADS) {
+      double a[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+      for (int c = 0; c < TV; ++c)
+        if (c < kb) a[c & 3] = fma(trans ? L[(k0 + c) + rr * ldl] : L[rr + (k0 + c) * ldl], xs[c], a[c & 3]);
+      x[rr] -= (a[0] + a[1]) + (a[2] + a[3]);
+    }
+    __syncthreads();
+  }
+}
+
+void tri_vec(cudaStream_t s, const double *L, int64_t M, int64_t ldl, const double *b, double *x,
+             bool trans) {
+  if (M <= 0) return;
+  tri_vec_kernel<<<1, TV_THREADS, 0, s>>>(L, M, ldl, b, x, trans ? 1 : 0);
+  GPGP_CHECK_LAUNCH();
+}
+
+// panel: L21 = A21 L11^-T by forward substitution, one row per thread (in place), for
+// the many rows of a batch (a single matrix's panel takes tri_block_kernel, whose rows
+// are 12 us instead of this one's 62 to 116 while they are few). Substitution keeps the
+// factorisation backward stable when a diagonal block is ill-conditioned (FITC's K_z);
+// the inverse W is used by the solves instead.
 __global__ void __launch_bounds__(128) potrf_panel_kernel(double *__restrict__ A21, int64_t m, int kb,
                                                           int64_t lda, const double *__restrict__ L11,
                                                           const int *__restrict__ status, int64_t sA) {
@@ -515,7 +701,7 @@ void potrf(cudaStream_t s, double *A, int64_t n, int64_t lda, double *Winv, doub
       if (panel_mode == 1)
         potrf_panel_inv_kernel<<<(unsigned)((m + 3) / 4), 256, 0, s>>>(A21, m, kb, lda, W, status);
       else
-        potrf_panel_kernel<<<(unsigned)((m + 127) / 128), 128, 0, s>>>(A21, m, kb, lda, Akk, status, 0);
+        tri_block_kernel<0><<<(unsigned)((m + 15) / 16), 128, 0, s>>>(Akk, lda, kb, A21, lda, m, status);
       GPGP_CHECK_LAUNCH();
       double *A22 = A + (k0 + kb) + (k0 + kb) * lda;
       gemm64(s, false, true, m, m, kb, -1.0, A21, lda, A21, lda, 1.0, A22, lda, true, 0);
@@ -880,68 +1066,6 @@ void trsv_flow(cudaStream_t s, const double *L, int64_t n, int64_t lda, const do
 }
 
 // ---------------------------------------------------------------------------
-// substitution solves for small factors (M x M lower L), as R's forwardsolve /
-// backsolve do: rows of a column-major n x M matrix, one thread per row
-// ---------------------------------------------------------------------------
-// mode 0: X = B L^-T (x L^T = b, forward); mode 1: X = B L^-1 (x L = b, backward).
-// X may alias B.
-__global__ void tri_rows_kernel(const double *__restrict__ L, int64_t M, int64_t ldl, const double *B,
-                                int64_t ldb, double *X, int64_t ldx, int64_t n, int mode) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  if (mode == 0) {
-    for (int64_t c = 0; c < M; ++c) {
-      double s = B[i + c * ldb];
-      for (int64_t k = 0; k < c; ++k) s = fma(-X[i + k * ldx], L[c + k * ldl], s);
-      X[i + c * ldx] = s / L[c + c * ldl];
-    }
-  } else {
-    for (int64_t c = M - 1; c >= 0; --c) {
-      double s = B[i + c * ldb];
-      for (int64_t k = c + 1; k < M; ++k) s = fma(-X[i + k * ldx], L[k + c * ldl], s);
-      X[i + c * ldx] = s / L[c + c * ldl];
-    }
-  }
-}
-
-void tri_rows(cudaStream_t s, const double *L, int64_t M, int64_t ldl, const double *B, int64_t ldb,
-              double *X, int64_t ldx, int64_t n, int mode) {
-  if (n <= 0 || M <= 0) return;
-  tri_rows_kernel<<<(unsigned)((n + 127) / 128), 128, 0, s>>>(L, M, ldl, B, ldb, X, ldx, n, mode);
-  GPGP_CHECK_LAUNCH();
-}
-
-// one warp: x = L^-1 b (trans = 0) or x = L^-T b (trans = 1), x may alias b
-__global__ void tri_vec_kernel(const double *__restrict__ L, int64_t M, int64_t ldl, const double *b,
-                               double *x, int trans) {
-  const int lane = threadIdx.x & 31;
-  if (!trans) {
-    for (int64_t r = 0; r < M; ++r) {
-      double s = 0.0;
-      for (int64_t k = lane; k < r; k += 32) s = fma(L[r + k * ldl], x[k], s);
-      for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-      if (lane == 0) x[r] = (b[r] - s) / L[r + r * ldl];
-      __syncwarp();
-    }
-  } else {
-    for (int64_t r = M - 1; r >= 0; --r) {
-      double s = 0.0;
-      for (int64_t k = r + 1 + lane; k < M; k += 32) s = fma(L[k + r * ldl], x[k], s);
-      for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-      if (lane == 0) x[r] = (b[r] - s) / L[r + r * ldl];
-      __syncwarp();
-    }
-  }
-}
-
-void tri_vec(cudaStream_t s, const double *L, int64_t M, int64_t ldl, const double *b, double *x,
-             bool trans) {
-  if (M <= 0) return;
-  tri_vec_kernel<<<1, 32, 0, s>>>(L, M, ldl, b, x, trans ? 1 : 0);
-  GPGP_CHECK_LAUNCH();
-}
-
-// ---------------------------------------------------------------------------
 // multi-RHS solve and triangular inverse
 // ---------------------------------------------------------------------------
 void trsm_lower(cudaStream_t s, const double *L, int64_t n, int64_t lda, const double *Winv,
@@ -1044,9 +1168,37 @@ __global__ void gemv_n_kernel(int64_t M, int64_t N, const double *__restrict__ A
   const int64_t c0 = (int64_t)blockIdx.y * GV_COLS;
   const int64_t c1 = (c0 + GV_COLS < N) ? c0 + GV_COLS : N;
   if (r >= M) return;
-  double s = 0.0;
-  for (int64_t c = c0; c < c1; ++c) s = fma(A[r + c * lda], x[c], s);
-  part[r + blockIdx.y * M] = s;
+  // four chains, so that the FP64 latency of one row's sum is hidden by its own loads
+  double s[4] = {0.0, 0.0, 0.0, 0.0};
+  int64_t c = c0;
+  for (; c + 4 <= c1; c += 4)
+#pragma unroll
+    for (int u = 0; u < 4; ++u) s[u] = fma(A[r + (c + u) * lda], x[c + u], s[u]);
+  for (; c < c1; ++c) s[0] = fma(A[r + c * lda], x[c], s[0]);
+  part[r + blockIdx.y * M] = (s[0] + s[1]) + (s[2] + s[3]);
+}
+
+// A^T x of a tall A with too few columns for a warp each to fill the GPU: a warp takes
+// GT_ROWS rows of a column, and the partials are summed in order (gemv_reduce_kernel).
+// 65536 x 256: 452 us with one warp per column.
+constexpr int64_t GT_ROWS = 2048;
+__global__ void gemv_t_part_kernel(int64_t M, int64_t N, const double *__restrict__ A, int64_t lda,
+                                   const double *__restrict__ x, double *__restrict__ part) {
+  const int lane = threadIdx.x & 31;
+  const int64_t c = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (c >= N) return;
+  const int64_t r0 = (int64_t)blockIdx.y * GT_ROWS;
+  const int64_t r1 = r0 + GT_ROWS < M ? r0 + GT_ROWS : M;
+  double s0 = 0.0, s1 = 0.0;
+  int64_t r = r0 + lane;
+  for (; r + 32 < r1; r += 64) {
+    s0 = fma(A[r + c * lda], x[r], s0);
+    s1 = fma(A[r + 32 + c * lda], x[r + 32], s1);
+  }
+  if (r < r1) s0 = fma(A[r + c * lda], x[r], s0);
+  double s = s0 + s1;
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+  if (lane == 0) part[c + blockIdx.y * N] = s;
 }
 
 __global__ void gemv_t_kernel(int64_t M, int64_t N, const double *__restrict__ A, int64_t lda,
@@ -1120,6 +1272,17 @@ void gemv64(cudaStream_t s, bool trans, int64_t M, int64_t N, double alpha, cons
             int64_t lda, const double *x, double beta, double *y) {
   if (trans) {
     if (N == 0) return;
+    if (M >= 4 * GT_ROWS && N < 8 * device_sms()) {  // fewer than two warps to a sub-partition
+      const int64_t nch = (M + GT_ROWS - 1) / GT_ROWS;
+      double *part = nullptr;
+      GPGP_CUDA(cudaMallocAsync((void **)&part, (size_t)N * nch * sizeof(double), s));
+      gemv_t_part_kernel<<<dim3((unsigned)((N * 32 + 255) / 256), (unsigned)nch), 256, 0, s>>>(M, N, A, lda, x, part);
+      GPGP_CHECK_LAUNCH();
+      gemv_reduce_kernel<<<(unsigned)((N + 255) / 256), 256, 0, s>>>(N, (int)nch, part, alpha, beta, y);
+      GPGP_CHECK_LAUNCH();
+      GPGP_CUDA(cudaFreeAsync(part, s));
+      return;
+    }
     gemv_t_kernel<<<(unsigned)((N * 32 + 255) / 256), 256, 0, s>>>(M, N, A, lda, x, y, alpha, beta);
     GPGP_CHECK_LAUNCH();
     return;

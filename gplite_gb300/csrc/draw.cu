@@ -69,9 +69,12 @@ gpgp_status gpgp_pred_cov(gpgp_model *m, const double *xt, int64_t mt, uint32_t 
       C.alloc(s, (size_t)mt * mt);
       gpgp_status st = pred_cov_fitc(m, Ft.p, mt, gm, jitter, dmean.p, C.p);
       if (st != GPGP_OK) return st;
+      int herr = 0;
+      GPGP_CUDA(cudaMemcpyAsync(&herr, m->errflag.p, sizeof(int), cudaMemcpyDeviceToHost, s));
       GPGP_CUDA(cudaMemcpyAsync(mean, dmean.p, mt * sizeof(double), cudaMemcpyDeviceToHost, s));
       GPGP_CUDA(cudaMemcpyAsync(cov, C.p, (size_t)mt * mt * sizeof(double), cudaMemcpyDeviceToHost, s));
       GPGP_CUDA(cudaStreamSynchronize(s));
+      if (herr) return fail(ctx, GPGP_ETIMEOUT, "a tensor-core kernel wait timed out");
       return GPGP_OK;
     }
     cov_matvec(s, m->dk, gm, Ft.p, mt, mt, m->F.p, n, n, m->alpha.p, dmean.p);

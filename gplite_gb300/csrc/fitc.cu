@@ -10,11 +10,13 @@
 // (R/gp_pred.R:234-296). Every product is O(n M^2) or less; n x n matrices
 // never appear. Solves with the M x M factors of K_z and of the lemma's
 // C_m = K_z + U^T S^-1 U are substitutions, as forwardsolve/backsolve do,
-// applied to the rows of n x M matrices (one thread per row, coalesced):
+// applied to the rows of n x M matrices (tri_rows):
 // X = K(x, z) L_z^-T is the transpose of the reference's
 // forwardsolve(Kz_chol, t(Kxz)). Explicit inverses of these often
-// ill-conditioned factors would cost accuracy. The n x M Gram product
-// U^T S^-1 U uses the sliced tensor-core GEMM in mixed precision.
+// ill-conditioned factors would cost accuracy. The products of n rows run on the tensor
+// cores at FP64 accuracy (gram_sliced, rows_times_bt): at n = 65536, M = 256 a Laplace
+// fit with 256 predictions spent 77 of 131 ms in the FP64 pipe's Gram products, 18 in
+// one-warp solves with the M x M factors and 14 in row-per-thread substitution.
 #include <math.h>
 
 #include <algorithm>
@@ -28,11 +30,16 @@ namespace {
 
 // out[i, m] = X[i, m] / v[i]  (n x M, column-major)
 __global__ void div_rows_kernel(int64_t n, int64_t M, const double *__restrict__ X,
-                                const double *__restrict__ v, double *__restrict__ out) {
+                                const double *__restrict__ v, const double *__restrict__ rv,
+                                double *__restrict__ out) {
   for (int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < n * M;
        idx += (int64_t)gridDim.x * blockDim.x) {
+    // the quotient by the reciprocal with one correction: three FP64 instructions where
+    // the division takes about ten (the kernel is bound by them)
     const int64_t i = idx % n;
-    out[idx] = X[idx] / v[i];
+    const double x = X[idx], d = v[i], r = rv[i];
+    const double q = x * r;
+    out[idx] = fma(fma(-q, d, x), r, q);
   }
 }
 
@@ -232,16 +239,17 @@ int64_t chol_small(gpgp_ctx *ctx, double *A, int64_t M, double *Wblk, double *lo
 void rows_times_cminv(gpgp_model *m, const double *B, double *X, int64_t n) {
   FitcState &f = *m->fitc;
   cudaStream_t st = m->ctx->stream;
-  tri_rows(st, f.Lm.p, f.M, f.M, B, n, X, n, n, 0);
-  tri_rows(st, f.Lm.p, f.M, f.M, X, n, X, n, n, 1);
+  tri_rows(st, f.Lm.p, f.M, f.M, B, n, X, n, n, 0, m->errflag.p);
+  tri_rows(st, f.Lm.p, f.M, f.M, X, n, X, n, n, 1, m->errflag.p);
 }
 
-// U^T B for U = Kxz, B both n x M, on the FP64 pipe in both precisions: the
-// lemma's C_m inherits K_z's conditioning (~1e4 and more), so BF16-sliced
-// products move its log-determinant by ~1e-5 relative at n = 65536, and the
-// Gram (2 n M^2 flops, split over K) is a small part of a FITC fit anyway.
+// A^T B for A, B both n x M, at FP64 accuracy in both precisions: the lemma's C_m
+// inherits K_z's conditioning (~1e4 and more), so products of 4 or 5 slices move its
+// log-determinant by ~1e-5 relative at n = 65536. Eight slices are as accurate as the
+// FP64 pipe, which small n keep (the split operands' launches cost more there).
 void gram_tn(gpgp_model *m, const double *A, const double *B, int64_t n, int64_t M, double *C) {
-  gemm64(m->ctx->stream, true, false, M, M, n, 1.0, A, n, B, n, 0.0, C, M);
+  if (n >= GRAM_SLICED_MIN) gram_sliced(m->ctx->stream, A, n, B, n, n, M, M, C, M, m->errflag.p);
+  else gemm64(m->ctx->stream, true, false, M, M, n, 1.0, A, n, B, n, 0.0, C, M);
 }
 
 // The lemma for the current S (R/linear_algebra.R:3-43): iDU = Kxz / S, C_m and its
@@ -251,7 +259,11 @@ bool lemma_get(gpgp_model *m, Red &red, double logdet_z) {
   FitcState &f = *m->fitc;
   cudaStream_t st = m->ctx->stream;
   const int64_t n = m->n, M = f.M;
-  div_rows_kernel<<<gs(n * M), 256, 0, st>>>(n, M, f.Kxz.p, f.S.p, f.iDU.p);
+  DBuf rS;
+  rS.alloc(st, n);
+  recip2_kernel<<<g1(n), 256, 0, st>>>(n, f.S.p, rS.p);
+  GPGP_CHECK_LAUNCH();
+  div_rows_kernel<<<gs(n * M), 256, 0, st>>>(n, M, f.Kxz.p, f.S.p, rS.p, f.iDU.p);
   GPGP_CHECK_LAUNCH();
   DBuf VDU;
   VDU.alloc(st, (size_t)M * M);
@@ -356,7 +368,11 @@ gpgp_status fitc_nlc_terms(gpgp_model *m, Red &red, double logdet_z, bool ep, co
   axpy_vec_kernel<<<g1(ng), 256, 0, st>>>(ng, Dg.p, 1.0, Vg.p, Sg.p);
   GPGP_CHECK_LAUNCH();
   iDUg.alloc(st, ng * M);
-  div_rows_kernel<<<gs(ng * M), 256, 0, st>>>(ng, M, Ug.p, Sg.p, iDUg.p);
+  DBuf rSg;
+  rSg.alloc(st, ng);
+  recip2_kernel<<<g1(ng), 256, 0, st>>>(ng, Sg.p, rSg.p);
+  GPGP_CHECK_LAUNCH();
+  div_rows_kernel<<<gs(ng * M), 256, 0, st>>>(ng, M, Ug.p, Sg.p, rSg.p, iDUg.p);
   GPGP_CHECK_LAUNCH();
   VDU.alloc(st, M * M);
   gemm64(st, true, false, M, M, ng, 1.0, Ug.p, ng, iDUg.p, ng, 0.0, VDU.p, M);
@@ -515,7 +531,7 @@ gpgp_status fit_fitc(gpgp_model *m, gpgp_fit_result *res, const double *inducing
   {
     Phase ph(ctx, GPGP_PHASE_SOLVE);
     // X = Kxz Lz^-T, the transpose of forwardsolve(Kz_chol, t(Kxz)) (R/gp_fit.R:110)
-    tri_rows(st, f.Lz.p, M, M, f.Kxz.p, n, f.X.p, n, n, 0);
+    tri_rows(st, f.Lz.p, M, M, f.Kxz.p, n, f.X.p, n, n, 0, m->errflag.p);
   }
   // D = (diag K(x, x) + jitter) - colSums(forwardsolve(...)^2)  (R/gp_fit.R:109-110)
   {
@@ -619,7 +635,7 @@ gpgp_status fit_fitc(gpgp_model *m, gpgp_fit_result *res, const double *inducing
   // Y = X Lz^-1: the transpose of inv_Kz_Kzx = backsolve(t(Kz_chol), forwardsolve(Kz_chol, t(Kxz)))
   DBuf Y, VU, Qt, lhsU, auxT, d1, d2;
   Y.alloc(st, (size_t)n * M);
-  tri_rows(st, f.Lz.p, M, M, f.X.p, n, Y.p, n, n, 1);
+  tri_rows(st, f.Lz.p, M, M, f.X.p, n, Y.p, n, n, 1, m->errflag.p);
   VU.alloc(st, (size_t)n * M);
   Qt.alloc(st, (size_t)n * M);
   lhsU.alloc(st, (size_t)M * M);
@@ -670,12 +686,12 @@ gpgp_status fit_fitc(gpgp_model *m, gpgp_fit_result *res, const double *inducing
       scale_rows_kernel<<<gs(n * M), 256, 0, st>>>(n, M, f.iDU.p, m->V.p, VU.p);
       GPGP_CHECK_LAUNCH();
       rows_times_cminv(m, VU.p, Qt.p, n);
-      gemm64(st, true, false, M, M, n, 1.0, Y.p, n, f.iDU.p, n, 0.0, lhsU.p, M);  // inv_Kz_Kzx iDU
+      gram_tn(m, Y.p, f.iDU.p, n, M, lhsU.p);  // inv_Kz_Kzx iDU
       div_vec_kernel<<<g1(n), 256, 0, st>>>(n, m->V.p, f.S.p, tmpn.p);              // V / S
       GPGP_CHECK_LAUNCH();
       scale_rows_kernel<<<gs(n * M), 256, 0, st>>>(n, M, Y.p, tmpn.p, auxT.p);
       GPGP_CHECK_LAUNCH();
-      gemm64(st, false, true, n, M, M, -1.0, Qt.p, n, lhsU.p, M, 1.0, auxT.p, n);
+      rows_times_bt(st, n, M, M, -1.0, Qt.p, n, lhsU.p, M, 1.0, auxT.p, n, m->errflag.p);
       rowdot_nn_kernel<<<g1(n), 256, 0, st>>>(M, n, f.Kxz.p, auxT.p, d1.p);          // diag1
       GPGP_CHECK_LAUNCH();
       rowdot_nn_kernel<<<g1(n), 256, 0, st>>>(M, n, f.iDU.p, Qt.p, d2.p);
@@ -743,8 +759,8 @@ static void fitc_pred_cache(gpgp_model *m) {
   GPGP_CHECK_LAUNCH();
   scale_rows_kernel<<<gs(n * M), 256, 0, st>>>(n, M, f.X.p, rs.p, XS.p);
   GPGP_CHECK_LAUNCH();
-  gemm64(st, true, false, M, M, n, 1.0, XS.p, n, f.X.p, n, 0.0, f.Sig1.p, M);
-  gemm64(st, true, false, M, M, n, 1.0, f.X.p, n, f.iDU.p, n, 0.0, f.P.p, M);
+  gram_tn(m, XS.p, f.X.p, n, M, f.Sig1.p);
+  gram_tn(m, f.X.p, f.iDU.p, n, M, f.P.p);
   // Z = P C_m^-1 (rows of P), sol = Sig1 - Z P^T
   Z.alloc(st, (size_t)M * M);
   rows_times_cminv(m, f.P.p, Z.p, M);
@@ -762,7 +778,7 @@ gpgp_status pred_fitc(gpgp_model *m, const double *Ft, int64_t mt, uint32_t gm, 
   X2.alloc(st, (size_t)mt * M);
   v1.alloc(st, M);
   cov_matrix(st, m->dk, gm, Ft, mt, mt, f.Fz.p, M, M, Ktz.p, mt, COV_FULL, 0, 0, 0.0, nullptr);
-  tri_rows(st, f.Lz.p, M, M, Ktz.p, mt, X2.p, mt, mt, 0);        // X2 = Ktz Lz^-T (= Kt_aux2^T)
+  tri_rows(st, f.Lz.p, M, M, Ktz.p, mt, X2.p, mt, mt, 0, m->errflag.p);        // X2 = Ktz Lz^-T (= Kt_aux2^T)
   gemv64(st, true, n, M, 1.0, f.X.p, n, m->alpha.p, 0.0, v1.p);  // Kt_aux1 alpha
   gemv64(st, false, mt, M, 1.0, X2.p, mt, v1.p, 0.0, mean);      // t(Kt_aux2) (Kt_aux1 alpha)
   if (!var) return GPGP_OK;
@@ -776,7 +792,7 @@ gpgp_status pred_fitc(gpgp_model *m, const double *Ft, int64_t mt, uint32_t gm, 
   vec_axpby(st, mt, -1.0, cs.p, 1.0, Dt.p);
   // prior_var = rowSums(Ktz * t(Kz^-1 Ktz^T)) + Dt, (Kz^-1 Ktz^T)^T = X2 Lz^-1
   Y2.alloc(st, (size_t)mt * M);
-  tri_rows(st, f.Lz.p, M, M, X2.p, mt, Y2.p, mt, mt, 1);
+  tri_rows(st, f.Lz.p, M, M, X2.p, mt, Y2.p, mt, mt, 1, m->errflag.p);
   pv.alloc(st, mt);
   rowdot_nn_kernel<<<g1(mt), 256, 0, st>>>(M, mt, Ktz.p, Y2.p, pv.p);
   GPGP_CHECK_LAUNCH();
@@ -808,7 +824,7 @@ gpgp_status pred_cov_fitc(gpgp_model *m, const double *Ft, int64_t mt, uint32_t 
   X2.alloc(st, (size_t)mt * M);
   v1.alloc(st, M);
   cov_matrix(st, m->dk, gm, Ft, mt, mt, f.Fz.p, M, M, Ktz.p, mt, COV_FULL, 0, 0, 0.0, nullptr);
-  tri_rows(st, f.Lz.p, M, M, Ktz.p, mt, X2.p, mt, mt, 0);        // X2 = Ktz Lz^-T
+  tri_rows(st, f.Lz.p, M, M, Ktz.p, mt, X2.p, mt, mt, 0, m->errflag.p);        // X2 = Ktz Lz^-T
   gemv64(st, true, n, M, 1.0, f.X.p, n, m->alpha.p, 0.0, v1.p);  // Kt_aux1 alpha
   gemv64(st, false, mt, M, 1.0, X2.p, mt, v1.p, 0.0, mean);
   // Dt = diag K(xt, xt) - colSums(Kt_aux2^2)
@@ -849,7 +865,7 @@ gpgp_status loo_fitc_posteriors(gpgp_model *m, double *lmean, double *lvar) {
   GPGP_CHECK_LAUNCH();
   // prior_var = rowSums(Kxz * (X Lz^-1)) + Dt
   Y.alloc(st, (size_t)n * M);
-  tri_rows(st, f.Lz.p, M, M, f.X.p, n, Y.p, n, n, 1);
+  tri_rows(st, f.Lz.p, M, M, f.X.p, n, Y.p, n, n, 1, m->errflag.p);
   pv.alloc(st, n);
   rowdot_nn_kernel<<<g1(n), 256, 0, st>>>(M, n, f.Kxz.p, Y.p, pv.p);
   GPGP_CHECK_LAUNCH();
@@ -858,7 +874,7 @@ gpgp_status loo_fitc_posteriors(gpgp_model *m, double *lmean, double *lvar) {
   CiU.alloc(st, (size_t)n * M);
   rows_times_cminv(m, f.iDU.p, CiU.p, n);
   iCP.alloc(st, (size_t)n * M);
-  gemm64(st, false, true, n, M, M, 1.0, CiU.p, n, f.P.p, M, 0.0, iCP.p, n);
+  rows_times_bt(st, n, M, M, 1.0, CiU.p, n, f.P.p, M, 0.0, iCP.p, n, m->errflag.p);
   ds.alloc(st, n);
   div_vec_kernel<<<g1(n), 256, 0, st>>>(n, Dt.p, f.S.p, ds.p);  // Dt / S
   GPGP_CHECK_LAUNCH();
@@ -866,7 +882,7 @@ gpgp_status loo_fitc_posteriors(gpgp_model *m, double *lmean, double *lvar) {
   auxT.alloc(st, (size_t)n * M);
   scale_rows_kernel<<<gs(n * M), 256, 0, st>>>(n, M, f.X.p, ds.p, auxT.p);
   GPGP_CHECK_LAUNCH();
-  gemm64(st, false, true, n, M, M, 1.0, f.X.p, n, f.Sig1.p, M, 1.0, auxT.p, n);
+  rows_times_bt(st, n, M, M, 1.0, f.X.p, n, f.Sig1.p, M, 1.0, auxT.p, n, m->errflag.p);
   DBuf DiCP;
   DiCP.alloc(st, (size_t)n * M);
   scale_rows_kernel<<<gs(n * M), 256, 0, st>>>(n, M, iCP.p, Dt.p, DiCP.p);

@@ -135,16 +135,23 @@ void estimate(const gpgp_server *s, Req *r) {
   }
   if (r->meth.kind == GPGP_METHOD_FITC) {
     const double M = (double)r->meth.num_inducing;
-    r->bytes = (int64_t)(8.0 * (8.0 * n * M + 12.0 * M * M + 3.0 * m * M + 40.0 * n) + (4 << 20));
+    // beside the fit, the Gram product's two split operands (16 bytes an entry with its
+    // row padding, at most 128 MB each) or those of the substitution (n x 64)
+    const double gram = std::max(std::min(32.0 * n * (M + 128.0), 2.7e8), 16.0 * n * 80.0);
+    r->bytes = (int64_t)(8.0 * (8.0 * n * M + 12.0 * M * M + 3.0 * m * M + 40.0 * n) + gram + (4 << 20));
     r->resident = (int64_t)(8.0 * (5.0 * n * M + 8.0 * M * M + 20.0 * n));
     r->work = 4.0 * n * M * M;
     return;
   }
   const double iters = r->lik.kind == GPGP_LIK_GAUSSIAN ? 1.0 : 8.0;
-  // n x 64 diagonal inverses; mixed adds two n x 256 four-slice panel operands
-  // (the Cholesky's panel and its lookahead trailing update), 256 n doubles each
-  r->bytes = (int64_t)(8.0 * ((mixed ? 5.0 : 3.0) * n * n + 2.0 * n * std::min(m, 4096.0) +
-                              (mixed ? 576.0 : 64.0) * n + 20.0 * n) + (4 << 20));
+  // n x 64 diagonal inverses; two n x 384 split panel operands (the Cholesky's panel and
+  // its lookahead trailing update: 8 bytes an entry of mixed, 16 of FP64); in FP64 also
+  // the operands of the variance's solve (n x 512 and m x 512) or, for EP, L^-1 with the
+  // operands of its products (2.5 n^2 doubles)
+  const bool sliced = !mixed && r->n >= SLICED_MIN;
+  const double extra = mixed ? 900.0 * n : sliced ? 2700.0 * n + 1100.0 * std::min(m, 4096.0) : 64.0 * n;
+  const double nn = mixed ? 5.0 : sliced && r->ap.kind == GPGP_APPROX_EP ? 5.5 : 3.0;
+  r->bytes = (int64_t)(8.0 * (nn * n * n + 2.0 * n * std::min(m, 4096.0) + extra + 20.0 * n) + (4 << 20));
   r->resident = (int64_t)(8.0 * (2.0 * n * n + 64.0 * n + 12.0 * n));
   r->work = iters * n * n * n / 3.0 + n * n * m;
 }

@@ -54,3 +54,25 @@ def test_a_nan_entry_of_the_matrix_is_refused(n):
     x[n // 2] = 1e200
     with pytest.raises((L.GpgpError, np.linalg.LinAlgError)):
         G.gp_fit(G.gp_init(G.cf_matern52(lscale=0.5), G.lik_gaussian(sigma=0.1)), x, rng.standard_normal(n))
+
+
+@pytest.mark.parametrize("n,M", [(1023, 65), (1024, 64), (4095, 33), (4096, 128), (4353, 63), (9001, 129), (8500, 1)])
+def test_fitc_either_side_of_the_sliced_sizes(n, M):
+    """FITC fits and predictions around the row counts where the Gram products and the
+    substitution's products move to the tensor cores, at inducing counts around the
+    block sizes. The Matern 3/2 kernel at scattered inducing inputs keeps K_z's condition
+    number below ~1e4, so 64-bit sums of up to 1e4 terms agree to ~1e-10; 1e-9 here."""
+    rng = np.random.default_rng(n + M)
+    x = rng.uniform(-2, 2, (n, 2))
+    y = np.sin(2 * x[:, 0]) * np.cos(x[:, 1]) + 0.1 * rng.standard_normal(n)
+    z = x[rng.choice(n, M, replace=False)]
+    xt = rng.uniform(-2, 2, (70, 2))
+    g = G.gp_fit(G.gp_init(G.cf_matern32(lscale=0.3), G.lik_gaussian(sigma=0.2), G.method_fitc(inducing=z)), x, y)
+    o = R.gp_fit(R.gp_init([R.cf("matern32", lscale=0.3, magn=1.0)], R.lik("gaussian", sigma=0.2),
+                           R.method_fitc(z)), x, y)
+    assert abs(g.fit["log_evidence"] - o.fit["log_evidence"]) <= 1e-9 * abs(o.fit["log_evidence"])
+    p, q = G.gp_pred(g, xt, var=True), R.gp_pred(o, xt, var=True)
+    assert np.allclose(p["mean"], q["mean"], rtol=1e-9, atol=1e-9)
+    assert np.allclose(p["var"], q["var"], rtol=1e-8, atol=1e-9)
+    if n < 5000:
+        assert np.allclose(G.gp_loo(g, x, y)["loos"], R.gp_loo(o, x, y)["loos"], rtol=1e-8, atol=1e-8)
