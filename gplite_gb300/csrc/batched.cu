@@ -25,12 +25,6 @@
 
 namespace gpgp {
 
-// potrf_diag_kernel lives in dense.cu
-__global__ void potrf_diag_kernel(double *__restrict__ A, int kb, int64_t lda,
-                                  double *__restrict__ Winv, double *__restrict__ logdet_part,
-                                  int *__restrict__ status, int64_t k0, int64_t sA, int64_t sW,
-                                  int64_t sL);
-
 namespace {
 
 constexpr int PRM = 8;  // doubles per problem: n, m, d, kind, lscale, magn, sigma, -
@@ -495,13 +489,7 @@ void run_bucket(gpgp_batch *b, Bucket &k, cudaStream_t st) {
       for (int64_t j0 = k0; j0 < k0 + kbo; j0 += NB) {
         const int64_t blk = j0 / NB;
         double *Akk = k.Bm.p + j0 + j0 * nb;
-        {
-          KTScope kts(GPGP_KPROF_POTRF_DIAG, st, 2.0 * NB * NB * NB / 3 * (double)P);
-          potrf_diag_kernel<<<(unsigned)P, DIAG_THREADS, 0, st>>>(Akk, NB, nb, k.Winv.p + blk * NB * NB,
-                                                                  k.ldp.p + blk, k.status.p, j0, nb * nb, nb * NB,
-                                                                  nbl);
-        }
-        GPGP_CHECK_LAUNCH();
+        potrf_diag(st, Akk, NB, nb, k.Winv.p + blk * NB * NB, k.ldp.p + blk, k.status.p, j0, nb * nb, nb * NB, nbl, P);
         const int64_t m = nb - j0 - NB;
         if (m <= 0) continue;
         double *A21 = k.Bm.p + (j0 + NB) + j0 * nb;

@@ -267,4 +267,40 @@ __device__ __forceinline__ double df2d_try(float hi, float lo, int sh, bool &slo
 }
 __device__ __forceinline__ double f2_to_double(f2 a) { return df2d_scaled(a.h, a.l, 0); }
 
+// 2^sh 2^-14 (hi 2^-24 + lo 2^-48) of a fixed-point sum, 0 <= lo < 2^24, rounded to a double with
+// integer instructions (a 64-bit integer conversion would go through the FP64 pipe);
+// slow is set (and the result void) where that is subnormal, overflows, or the operand
+// was marked non-finite.
+__device__ __forceinline__ double fixed_to_double(long long hi, int lo, int sh, uint32_t negmask, bool &slow) {
+  // sign and magnitude of hi 2^24 + lo, 0 <= lo < 2^24
+  const bool neg = hi < 0;
+  unsigned long long h = (unsigned long long)hi;
+  uint32_t l = (uint32_t)lo;
+  if (neg) {
+    l = (0x1000000u - l) & 0xFFFFFFu;
+    h = (l == 0u ? 0ull : ~0ull) - h;  // -hi - (lo != 0)
+  }
+  int e = sh - 38;
+  if (h == 0ull) {
+    h = l;
+    l = 0u;
+    e -= 24;
+  }
+  const int z = __clzll((long long)h);
+  // top 64 bits of the number: hi shifted up, lo's 24 bits following it
+  unsigned long long m = (h << (z & 63)) | (((unsigned long long)l << 39) >> (63 - (z & 63)));
+  m = (m >> 11) + ((m >> 10) & 1ull);  // 53 bits, rounded to nearest (ties away)
+  const int ed = e + 63 - z + 1023;
+  const bool zero = h == 0ull;
+  slow |= sh > 4096 || (!zero && (ed <= 1 || ed >= 2046));
+  const unsigned long long b = ((unsigned long long)(uint32_t)(ed - 1) << 52) + m;  // m's leading bit adds 1 to ed - 1
+  const uint32_t sb = (neg ? 0x80000000u : 0u) ^ negmask;
+  return __longlong_as_double(zero ? 0ll : (long long)(b | ((unsigned long long)sb << 32)));
+}
+static __device__ __noinline__ double fixed_to_double_slow(long long hi, int lo, int sh, uint32_t negmask) {
+  if (sh > 4096) return __longlong_as_double(0x7FF8000000000000ll);  // a non-finite operand
+  const double v = ldexp(ldexp((double)hi, -24) + ldexp((double)lo, -48), sh - 14);
+  return negmask ? -v : v;
+}
+
 }  // namespace gpgp

@@ -598,42 +598,6 @@ __device__ __forceinline__ bool oz_wait(uint32_t bar, uint32_t parity, volatile 
   return false;
 }
 
-// 2^sh 2^-14 (hi 2^-24 + lo 2^-48) of the fixed-point sums of S = 8, rounded to a double with
-// integer instructions (a 64-bit integer conversion would go through the FP64 pipe);
-// slow is set (and the result void) where that is subnormal, overflows, or the operand
-// was marked non-finite.
-__device__ __forceinline__ double oz_fixed_to_double(long long hi, int lo, int sh, uint32_t negmask, bool &slow) {
-  // sign and magnitude of hi 2^24 + lo, 0 <= lo < 2^24
-  const bool neg = hi < 0;
-  unsigned long long h = (unsigned long long)hi;
-  uint32_t l = (uint32_t)lo;
-  if (neg) {
-    l = (0x1000000u - l) & 0xFFFFFFu;
-    h = (l == 0u ? 0ull : ~0ull) - h;  // -hi - (lo != 0)
-  }
-  int e = sh - 38;
-  if (h == 0ull) {
-    h = l;
-    l = 0u;
-    e -= 24;
-  }
-  const int z = __clzll((long long)h);
-  // top 64 bits of the number: hi shifted up, lo's 24 bits following it
-  unsigned long long m = (h << (z & 63)) | (((unsigned long long)l << 39) >> (63 - (z & 63)));
-  m = (m >> 11) + ((m >> 10) & 1ull);  // 53 bits, rounded to nearest (ties away)
-  const int ed = e + 63 - z + 1023;
-  const bool zero = h == 0ull;
-  slow |= sh > 4096 || (!zero && (ed <= 1 || ed >= 2046));
-  const unsigned long long b = ((unsigned long long)(uint32_t)(ed - 1) << 52) + m;  // m's leading bit adds 1 to ed - 1
-  const uint32_t sb = (neg ? 0x80000000u : 0u) ^ negmask;
-  return __longlong_as_double(zero ? 0ll : (long long)(b | ((unsigned long long)sb << 32)));
-}
-__device__ __noinline__ double oz_fixed_to_double_slow(long long hi, int lo, int sh, uint32_t negmask) {
-  if (sh > 4096) return __longlong_as_double(0x7FF8000000000000ll);  // a non-finite operand
-  const double v = ldexp(ldexp((double)hi, -24) + ldexp((double)lo, -48), sh - 14);
-  return negmask ? -v : v;
-}
-
 template <int S>
 // 576 threads: the register cap keeps the block inside one SM's register file
 __global__ void __maxnreg__(96) oz_gemm_kernel(const OzGemmArgs g) {
@@ -945,7 +909,7 @@ __global__ void __maxnreg__(96) oz_gemm_kernel(const OzGemmArgs g) {
         for (int j = 0; j < EC; ++j) {
           const int sh = ea + __shfl_sync(0xffffffffu, eb, j0 + j);
           if constexpr (Cfg::FP64) {
-            v[j] = oz_fixed_to_double(hi[j0 + j], lo[j0 + j], sh, negmask, slow);
+            v[j] = fixed_to_double(hi[j0 + j], lo[j0 + j], sh, negmask, slow);
           } else {
             // the sign of alpha goes onto the FP32 pair
             hi[j0 + j] = __uint_as_float(__float_as_uint(hi[j0 + j]) ^ negmask);
@@ -957,7 +921,7 @@ __global__ void __maxnreg__(96) oz_gemm_kernel(const OzGemmArgs g) {
 #pragma unroll
           for (int j = 0; j < EC; ++j) {
             const int sh = ea + __shfl_sync(0xffffffffu, eb, j0 + j);
-            if constexpr (Cfg::FP64) v[j] = oz_fixed_to_double_slow(hi[j0 + j], lo[j0 + j], sh, negmask);
+            if constexpr (Cfg::FP64) v[j] = fixed_to_double_slow(hi[j0 + j], lo[j0 + j], sh, negmask);
             else v[j] = df2d_scaled(hi[j0 + j], lo[j0 + j], sh - 16);
           }
         }

@@ -20,11 +20,7 @@
 
 namespace gpgp {
 
-// potrf_diag_kernel and potrf_panel_inv_kernel live in dense.cu
-__global__ void potrf_diag_kernel(double *__restrict__ A, int kb, int64_t lda,
-                                  double *__restrict__ Winv, double *__restrict__ logdet_part,
-                                  int *__restrict__ status, int64_t k0, int64_t sA, int64_t sW,
-                                  int64_t sL);
+// potrf_panel_inv_kernel lives in dense.cu
 __global__ void potrf_panel_inv_kernel(double *__restrict__ A21, int64_t m, int kb, int64_t lda,
                                        const double *__restrict__ W, const int *__restrict__ status);
 
@@ -60,12 +56,7 @@ void factor_panel(cudaStream_t x, cudaStream_t y, const SideStream *sd, double *
     const int jb = (int)std::min<int64_t>(NB, pend - j0);
     const int64_t blk = j0 / NB;
     double *Wb = Winv + blk * NB * NB;
-    {
-      KTScope kts(GPGP_KPROF_POTRF_DIAG, x, 2.0 * jb * jb * jb / 3);
-      potrf_diag_kernel<<<1, DIAG_THREADS, 0, x>>>(A + j0 + j0 * lda, jb, lda, Wb, logdet_part + blk, status, j0, 0,
-                                                   0, 0);
-    }
-    GPGP_CHECK_LAUNCH();
+    potrf_diag(x, A + j0 + j0 * lda, jb, lda, Wb, logdet_part + blk, status, j0, 0, 0, 0, 1);
     const int64_t mp = pend - (j0 + jb);  // panel rows below the block
     double *Ap = A + (j0 + jb) + j0 * lda;
     if (mp > 0) {
