@@ -812,7 +812,8 @@ gpgp_status gpgp_create(gpgp_ctx **out, int device) {
     GPGP_CUDA(cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking));
     GPGP_CUDA(cudaStreamCreateWithFlags(&c->side.s, cudaStreamNonBlocking));
     GPGP_CUDA(cudaStreamCreateWithFlags(&c->side.s2, cudaStreamNonBlocking));
-    for (cudaEvent_t *e : {&c->side.fork, &c->side.a, &c->side.l, &c->side.c, &c->side.b})
+    GPGP_CUDA(cudaStreamCreateWithFlags(&c->side.s3, cudaStreamNonBlocking));
+    for (cudaEvent_t *e : {&c->side.fork, &c->side.a, &c->side.l, &c->side.c, &c->side.b, &c->side.e})
       GPGP_CUDA(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
     GPGP_CUDA(cudaMallocHost((void **)&c->h_pinned, 64 * sizeof(double)));
     return GPGP_OK;
@@ -828,12 +829,12 @@ gpgp_status gpgp_destroy(gpgp_ctx *ctx) {
     cudaStreamSynchronize(ctx->stream);
     cudaStreamDestroy(ctx->stream);
   }
-  for (cudaStream_t x : {ctx->side.s, ctx->side.s2})
+  for (cudaStream_t x : {ctx->side.s, ctx->side.s2, ctx->side.s3})
     if (x) {
       cudaStreamSynchronize(x);
       cudaStreamDestroy(x);
     }
-  for (cudaEvent_t e : {ctx->side.fork, ctx->side.a, ctx->side.l, ctx->side.c, ctx->side.b})
+  for (cudaEvent_t e : {ctx->side.fork, ctx->side.a, ctx->side.l, ctx->side.c, ctx->side.b, ctx->side.e})
     if (e) cudaEventDestroy(e);
   if (ctx->h_pinned) cudaFreeHost(ctx->h_pinned);
   delete ctx;

@@ -220,11 +220,14 @@ void cov_matvec_df(cudaStream_t s, const DevKernel &dk, uint32_t gmask, const do
 // ---------------------------------------------------------------------------
 constexpr int NB = 64;  // block size of the blocked factorisations
 constexpr int DIAG_THREADS = 512;  // threads of the diagonal-block kernel (potrf_diag_kernel)
+// D -= L L^T (lower triangle) for L = m x 64, m <= 64, both of leading dimension lda
+void syrk_block(cudaStream_t s, const double *Ln, int64_t lda, int m, double *D);
 // Factor and inverse of the kb x kb (kb <= 64) diagonal block of each of `batch` problems
 // (matrices sA, inverses sW, log-determinant parts sL apart, one status word each); a
-// pivot that is not positive sets the status to its number, k0 + 1 ...
+// pivot that is not positive sets the status to its number, k0 + 1 ... (rank1: the FP64
+// pipe's rounding that the mixed precision is kept at.)
 void potrf_diag(cudaStream_t s, double *A, int kb, int64_t lda, double *Winv, double *logdet_part, int *status,
-                int64_t k0, int64_t sA, int64_t sW, int64_t sL, int64_t batch);
+                int64_t k0, int64_t sA, int64_t sW, int64_t sL, int64_t batch, bool rank1 = false);
 
 // C = alpha * op(A) op(B) + beta * C. lower_only: only tiles on/below the
 // diagonal of C are computed (SYRK-style). tri_k: A and B are triangular so
@@ -300,6 +303,11 @@ void getrs(cudaStream_t s, const double *LU, int64_t n, int64_t lda, const int *
 // mixed precision (mixed.cu / mixed_la.cu): BF16-sliced operands for tcgen05
 // ---------------------------------------------------------------------------
 constexpr int OZ_FP64 = 8;
+// Size from which the FP64 path's factorisation, inverses and B^-1 take the tensor cores
+// with 8 slices. Optimiser step / fit and predict / EP fit in ms, FP64 pipe against slices:
+// n = 800: 2.92 / 2.16 / 19.1 against 2.28 / 2.28 / 19.9; n = 900: 3.58 / 2.72 / 21.0
+// against 2.38 / 2.54 / 18.6 (n <= 768 has one outer panel's lookahead too few: 2.76 /
+// 2.03 / 18.2 against 2.61 / 2.65 / 22.7 at 760).
 #ifndef GPGP_SLICED_MIN
 #define GPGP_SLICED_MIN 960
 #endif
@@ -370,12 +378,17 @@ struct OzGridCap {
   ~OzGridCap() { tl_oz_grid_cap = old; }
 };
 int oz_sms();  // SMs of the current device
-// Two more streams with their events, owned by a context, for work that runs
+// One 64-wide block column (at j0) of the Cholesky: rows [r0, r1) become L = A W^T (W the
+// diagonal block's inverse) and update the next q1 64-wide column blocks by L L_q^T, L_q the
+// finished rows j0 + 64 (q + 1) .. of the block column (S = 4 or OZ_FP64).
+void panel_block(cudaStream_t s, int S, double *A, int64_t lda, int64_t r0, int64_t r1, int64_t j0, const double *W,
+                 int q1, int *err, const int *status);
+// Three more streams with their events, owned by a context, for work that runs
 // beside its main stream (the mixed Cholesky: s factors the diagonal chain of the
-// next panel, s2 the panel's rows below it).
+// next panel, s2 the rows below it, s3 the rest of the panel's own rows).
 struct SideStream {
-  cudaStream_t s = nullptr, s2 = nullptr;
-  cudaEvent_t fork = nullptr, a = nullptr, l = nullptr, c = nullptr, b = nullptr;
+  cudaStream_t s = nullptr, s2 = nullptr, s3 = nullptr;
+  cudaEvent_t fork = nullptr, a = nullptr, l = nullptr, c = nullptr, b = nullptr, e = nullptr;
 };
 // Batched versions: problem z uses P + z sP and the split's batch strides (set
 // bstride_ex / bstride_sl before splitting); C + z sC; status + z status_bs.

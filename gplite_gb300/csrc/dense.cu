@@ -595,15 +595,210 @@ __global__ void __launch_bounds__(DIAG_THREADS) potrf_diag_kernel(double *__rest
   }
 }
 
+// The same block on the FP64 pipe alone, column by column: the kernel of the mixed
+// precision. There the trailing updates cut their operands to 32 (batched: 40) bits, so
+// any other rounding of an entry here draws the whole truncation of the factor anew, and
+// predicted variances, whose error is 2e-8 of their scale, move by up to 2e-9 of it: with
+// this kernel mixed results stay the same to the bit. It costs 65 us a block where the
+// kernel above costs 51.
+// On this part the FP64 pipe retires about 2 lane operations per clock per SM,
+// and a warp instruction occupies it whether 1 or 32 lanes are active, so the
+// kernel issues as few FP64 warp instructions as it can, each with all lanes on
+// distinct entries, and runs the factor and the inverse in one loop with one
+// barrier per column:
+//  - factor, right-looking: warp 0 takes the pivots one column ahead (column
+//    j+1 gets its update from column j, then its inverse square root,
+//    rsqrt_fast) while the update warps apply the rank-1 update of column j to
+//    the trailing triangle c >= j+2. The trailing triangle's entries are
+//    numbered by column, last column first, so that step j's entries are the
+//    first (kb-2-j)(kb-1-j)/2 of one fixed list. The warps that share warp 0's
+//    sub-partition take no update work; the other twelve (three per
+//    sub-partition, enough to cover the FP64 latency) share it evenly.
+//  - inverse: W = L^-1 = D^-1 V with D = diag(L) and V the unit lower triangular
+//    inverse of the column-scaled factor L D^-1:
+//      V(i, c) = -sum_{k=c..i-1} (L(i, k) / L(k, k)) V(k, c),  V(c, c) = 1.
+//    The k = c term is written by the pivot of column c (V(i, c) starts as
+//    -L(i, c) / L(c, c)); the terms k > c are added right-looking, step k adding
+//    V(i, k) V(k, c) to every (i > k, c < k) while V(i, k) still holds only its
+//    first term. Step k needs column k of L and rows <= k of V final, so it runs
+//    beside the factor's step k + 1 in the same loop iteration. Every inverse
+//    entry costs one FMA; the row scaling by 1 / L(i, i) happens once, on the
+//    way out.
+//  - log L_jj summed in a fixed tree order.
+__device__ __forceinline__ int div_small(int e, int d, int magic) {
+  // e / d for e < 4096, 1 <= d <= 64, magic = ceil(2^20 / d): exact on that range
+  return (int)(((unsigned)e * (unsigned)magic) >> 20);
+}
+
+__global__ void __launch_bounds__(DIAG_THREADS) potrf_diag_rank1_kernel(double *__restrict__ A, int kb, int64_t lda,
+                                                         double *__restrict__ Winv,
+                                                         double *__restrict__ logdet_part,
+                                                         int *__restrict__ status, int64_t k0,
+                                                         int64_t sA, int64_t sW, int64_t sL) {
+  // batched: problem blockIdx.x (strides sA, sW, sL; status has one word per problem)
+  A += blockIdx.x * sA;
+  Winv += blockIdx.x * sW;
+  logdet_part += blockIdx.x * sL;
+  status += blockIdx.x;
+  __shared__ double S[NB][NB + 1];
+  __shared__ double V[NB][NB + 1];
+  __shared__ double rdiag[NB];
+  __shared__ double lg[NB];
+  __shared__ unsigned short pairs[NB * (NB + 1) / 2];  // (r | c << 8), column-major from the last column
+  __shared__ int failed;
+  if (*(volatile int *)status != 0) return;
+  const int tid = threadIdx.x;
+  const int lane = tid & 31, warp = tid >> 5;
+  for (int idx = tid; idx < NB * NB; idx += DIAG_THREADS) {
+    const int r = idx % NB, c = idx / NB;
+    // held negated until its column is pivoted (see the update loop)
+    S[r][c] = (r < kb && c < kb && r >= c) ? neg_bits(A[r + c * lda]) : 0.0;
+    V[r][c] = 0.0;
+  }
+  // entry e of the kb x kb triangle: u = kb - 1 - c is the largest u with
+  // u (u + 1) / 2 <= e; r = c + e - u (u + 1) / 2 (a partial block lists only its
+  // own entries)
+  for (int e = tid; e < kb * (kb + 1) / 2; e += DIAG_THREADS) {
+    int u = (int)((sqrtf(8.0f * (float)e + 1.0f) - 1.0f) * 0.5f);
+    while (u * (u + 1) / 2 > e) --u;
+    while ((u + 1) * (u + 2) / 2 <= e) ++u;
+    const int c = kb - 1 - u, r = c + (e - u * (u + 1) / 2);
+    pairs[e] = (unsigned short)(r | (c << 8));
+  }
+  if (tid == 0) failed = 0;
+  __syncthreads();
+  // Warp 0 keeps the current scaled column in registers: lane l owns rows l and
+  // l + 32, and lreg[u] holds L(l + 32 u, j) once column j is pivoted. Rows below
+  // 32 drop out after column 31, so their FP64 work is skipped from then on (a
+  // warp instruction costs the same with one lane or 32).
+  double lreg[2] = {0.0, 0.0};
+  // pivot of column j by warp 0 from t[u] = -S(l + 32 u, j) after all updates:
+  // L_jj, the scaled column below it (stored positive, and kept in lreg) and the
+  // first term of column j of V
+  auto pivot = [&](int j, const double (&t)[2]) {
+    const double dj = neg_bits(__shfl_sync(0xffffffffu, j < 32 ? t[0] : t[1], j & 31));
+    // not positive (sign bit or zero) or not finite, tested on the bits
+    const long long djb = __double_as_longlong(dj);
+    if (djb <= 0ll || (djb >> 52) >= 0x7FFll) {
+      if (lane == 0) {
+        failed = 1;
+        atomicCAS(status, 0, (int)(k0 + j + 1));
+      }
+      return;
+    }
+    const double rp = rsqrt_fast(dj);
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      if (u == 1 || j < 31) {
+        const int r = lane + 32 * u;
+        if (r > j && r < kb) {
+          const double l = -(t[u] * rp);
+          S[r][j] = l;
+          V[r][j] = -(l * rp);
+          lreg[u] = l;
+        }
+      }
+    }
+    if (lane == (j & 31)) {
+      S[j][j] = dj * rp;
+      rdiag[j] = rp;
+    }
+  };
+  if (warp == 0) {
+    double t0[2];
+#pragma unroll
+    for (int u = 0; u < 2; ++u) t0[u] = (lane + 32 * u < kb) ? S[lane + 32 * u][0] : 0.0;
+    pivot(0, t0);
+  }
+  __syncthreads();
+  if (failed) return;
+  // update workers: every warp off sub-partition 0 (warps 4, 8, 12 share warp 0's)
+  constexpr int NUPD = DIAG_THREADS / 32 - DIAG_THREADS / 128;  // 12 update warps
+  const int uw = warp - 1 - (warp >> 2);
+  const int ut = uw * 32 + lane;
+  for (int j = 0; j < kb; ++j) {
+    if (warp == 0) {
+      if (j + 1 < kb) {
+        // column j + 1 takes its last update, from column j, then its pivot
+        const double l = __shfl_sync(0xffffffffu, (j + 1) < 32 ? lreg[0] : lreg[1], (j + 1) & 31);
+        double t[2] = {0.0, 0.0};
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          if (u == 1 || j < 31) {
+            const int r = lane + 32 * u;
+            if (r > j && r < kb) t[u] = fma(lreg[u], l, S[r][j + 1]);
+          }
+        }
+        pivot(j + 1, t);
+      }
+    } else if ((warp & 3) != 0) {
+      // factor step j: entries (r, c), c >= j + 2, of the fixed list; inverse step
+      // k = j - 1: entries (i, c), k < i < kb, c < k, row-major by i. Both are
+      // dst += a b with a, b >= sign-free operands (the trailing matrix is held
+      // negated), so that each entry is exactly one FP64 instruction.
+      const int cf = j < kb - 2 ? (kb - 2 - j) * (kb - 1 - j) / 2 : 0;
+      const int k = j - 1;
+      const int ci = k >= 1 ? (kb - 1 - k) * k : 0;
+      const int magic = k >= 1 ? ((1 << 20) + k - 1) / k : 0;
+      for (int e = ut; e < cf + ci; e += NUPD * 32) {
+        const double *pa, *pb;
+        double *dst;
+        if (e < cf) {
+          const unsigned short pc = pairs[e];
+          const int r = pc & 0xFF, c = pc >> 8;
+          dst = &S[r][c];
+          pa = &S[r][j];
+          pb = &S[c][j];
+        } else {
+          const int e2 = e - cf;
+          const int q = div_small(e2, k, magic);
+          const int c = e2 - q * k, i = k + 1 + q;
+          dst = &V[i][c];
+          pa = &V[i][k];
+          pb = &V[k][c];
+        }
+        *dst = fma(*pa, *pb, *dst);
+      }
+    }
+    __syncthreads();
+    if (failed) return;
+  }
+  // write the factor back (lower part of the block)
+  for (int idx = tid; idx < kb * kb; idx += DIAG_THREADS) {
+    const int r = idx % kb, c = idx / kb;
+    if (r >= c) A[r + c * lda] = S[r][c];
+  }
+  if (tid < NB) lg[tid] = tid < kb ? log(S[tid][tid]) : 0.0;
+  __syncthreads();
+  // W = D^-1 V
+  for (int idx = tid; idx < NB * NB; idx += DIAG_THREADS) {
+    const int r = idx % NB, c = idx / NB;
+    double wv = 0.0;
+    if (r < kb && c <= r) wv = (r == c) ? rdiag[r] : rdiag[r] * V[r][c];
+    Winv[r + c * NB] = wv;
+  }
+  for (int st = NB / 2; st > 0; st >>= 1) {
+    if (tid < st) lg[tid] += lg[tid + st];
+    __syncthreads();
+  }
+  if (tid == 0) *logdet_part = lg[0];
+}
+
 void potrf_diag(cudaStream_t s, double *A, int kb, int64_t lda, double *Winv, double *logdet_part, int *status,
-                int64_t k0, int64_t sA, int64_t sW, int64_t sL, int64_t batch) {
+                int64_t k0, int64_t sA, int64_t sW, int64_t sL, int64_t batch, bool rank1) {
+  KTScope kts(GPGP_KPROF_POTRF_DIAG, s, 2.0 * kb * kb * kb / 3 * (double)batch);
+  if (rank1) {
+    potrf_diag_rank1_kernel<<<(unsigned)batch, DIAG_THREADS, 0, s>>>(A, kb, lda, Winv, logdet_part, status, k0, sA,
+                                                                     sW, sL);
+    GPGP_CHECK_LAUNCH();
+    return;
+  }
   static PerDevice attr;
   per_device(attr, [] {
     GPGP_CUDA(cudaFuncSetAttribute(potrf_diag_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    (int)sizeof(DiagShared)));
     return 1;
   });
-  KTScope kts(GPGP_KPROF_POTRF_DIAG, s, 2.0 * kb * kb * kb / 3 * (double)batch);
   potrf_diag_kernel<<<(unsigned)batch, DIAG_THREADS, sizeof(DiagShared), s>>>(A, kb, lda, Winv, logdet_part, status,
                                                                               k0, sA, sW, sL);
   GPGP_CHECK_LAUNCH();
@@ -829,23 +1024,30 @@ __global__ void __launch_bounds__(128) potrf_panel_kernel(double *__restrict__ A
 
 // panel by the diagonal block's inverse: L21 = A21 W11^T, L21(r, c) = sum_{k <= c}
 // A21(r, k) W11(c, k). A CTA takes 4 rows (one element per thread), staged in
-// shared memory with W11, so the FP64 work spreads over m / 4 CTAs. For the
-// well-conditioned diagonal blocks of B = I + S K S the error is that of the
+// shared memory with W11, so the FP64 work spreads over m / 4 CTAs; the four warps of a
+// sub-partition pair hold columns c and 63 - c, whose sums add up to the same length. For
+// the well-conditioned diagonal blocks of B = I + S K S the error is that of the
 // substitution to within the block's condition number.
 __global__ void __launch_bounds__(256) potrf_panel_inv_kernel(double *__restrict__ A21, int64_t m, int kb,
                                                               int64_t lda, const double *__restrict__ W,
                                                               const int *__restrict__ status) {
   __shared__ double Ws[NB][NB + 1];
   __shared__ double As[4][NB + 1];
-  if (*(volatile const int *)status != 0) return;
+  if (status && *(volatile const int *)status != 0) return;
   const int64_t r0 = (int64_t)blockIdx.x * 4;
-  for (int idx = threadIdx.x; idx < NB * NB; idx += 256) Ws[idx % NB][idx / NB] = W[idx];
+#pragma unroll
+  for (int t = 0; t < NB * NB / 256; ++t) {
+    const int idx = threadIdx.x + 256 * t;
+    Ws[idx % NB][idx / NB] = W[idx];
+  }
   {
     const int rr = threadIdx.x & 3, c = threadIdx.x >> 2;
     As[rr][c] = (r0 + rr < m && c < kb) ? A21[r0 + rr + c * lda] : 0.0;
   }
   __syncthreads();
-  const int rr = threadIdx.x & 3, c = threadIdx.x >> 2;
+  // warps w and w + 4 share a sub-partition: columns 8w.. and 56 - 8w..
+  const int w = threadIdx.x >> 5, cg = w < 4 ? w : 11 - w;
+  const int rr = threadIdx.x & 3, c = 8 * cg + ((threadIdx.x & 31) >> 2);
   if (r0 + rr >= m || c >= kb) return;
   double s0 = 0.0, s1 = 0.0;
   int k = 0;
@@ -855,6 +1057,44 @@ __global__ void __launch_bounds__(256) potrf_panel_inv_kernel(double *__restrict
   }
   if (k <= c) s0 = fma(As[rr][k], Ws[c][k], s0);
   A21[r0 + rr + c * lda] = s0 + s1;
+}
+
+// The next diagonal block's update, D -= L L^T (lower triangle) for its m <= 64 rows L
+// (m x 64): 32 CTAs share the 2080 entries, two threads to an entry (even and odd
+// terms, as the small GEMM sums them), so that each sub-partition runs one warp of 32 FP64
+// multiply-adds (the chain of the Cholesky waits for this: 5 us, against 12 as a small
+// GEMM whose every operand came from L2).
+constexpr int SU_CTAS = 32, SU_ENT = (NB * (NB + 1) / 2 + SU_CTAS - 1) / SU_CTAS;  // 65 entries
+
+__global__ void __launch_bounds__(160) syrk_block_kernel(const double *__restrict__ Ln, int64_t lda, int m,
+                                                         double *__restrict__ D) {
+  __shared__ double Ls[NB][NB + 1];  // [k][r]
+  const int tid = threadIdx.x;
+  const int e = blockIdx.x * SU_ENT + (tid >> 1), half = tid & 1;
+  int r = (int)((sqrtf(8.0f * (float)e + 1.0f) - 1.0f) * 0.5f);
+  if (r * (r + 1) / 2 > e) --r;
+  if ((r + 1) * (r + 2) / 2 <= e) ++r;
+  const int c = e - r * (r + 1) / 2;
+  const bool mine = (tid >> 1) < SU_ENT && r < m;
+  const double d = mine && half == 0 ? D[r + c * lda] : 0.0;
+#pragma unroll
+  for (int t = 0; t < (NB * NB + 159) / 160; ++t) {
+    const int idx = tid + 160 * t, lr = idx % NB, lk = idx / NB;
+    if (idx < NB * NB) Ls[lk][lr] = lr < m ? Ln[lr + lk * lda] : 0.0;
+  }
+  __syncthreads();
+  double s = 0.0;
+  if (mine)
+#pragma unroll 8
+    for (int k = half; k < NB; k += 2) s = fma(Ls[k][r], Ls[k][c], s);
+  s += __shfl_xor_sync(0xffffffffu, s, 1);
+  if (mine && half == 0) D[r + c * lda] = d - s;
+}
+
+void syrk_block(cudaStream_t s, const double *Ln, int64_t lda, int m, double *D) {
+  if (m <= 0) return;
+  syrk_block_kernel<<<SU_CTAS, 160, 0, s>>>(Ln, lda, m, D);
+  GPGP_CHECK_LAUNCH();
 }
 
 void potrf(cudaStream_t s, double *A, int64_t n, int64_t lda, double *Winv, double *logdet_part,

@@ -104,54 +104,53 @@ __device__ __forceinline__ double oz_elem(const double *P, int64_t ld, int trans
   return trans ? P[k + r * ld] : P[r + k * ld];
 }
 
-// Row exponents and slices are computed from the FP64 bit patterns with
-// integer instructions only (the FP64 pipe of this part is slow).
+// Row exponents and slices are computed from the FP64 bit patterns with integer and FP32
+// instructions only (the FP64 pipe of this part is slow).
 
-// bf16 bits of q 2^-8t, |q| <= 256 (exact: at most 8 significant bits)
-__device__ __forceinline__ uint32_t bf16_of_digit(int q, int t) {
-  if (q == 0) return 0u;
-  const uint32_t sgn = q < 0 ? 0x8000u : 0u;
-  const uint32_t a = (uint32_t)(q < 0 ? -q : q);
-  const int p = 31 - __clz(a);
-  const uint32_t mant = p <= 7 ? ((a << (7 - p)) & 0x7Fu) : ((a >> (p - 7)) & 0x7Fu);
-  return sgn | ((uint32_t)(127 + p - 8 * t) << 7) | mant;
-}
-
-// Fixed point |x| 2^BITS (rounded to nearest) of x = P 2^-e, as balanced base-256
-// digits d0..d(S-1) carrying the sign of P (|d0| <= 256, of S = 8 <= 128; the others
-// <= 128)
+// Two neighbouring entries v0, v1 of a row with power of two e, as the S slices' packed
+// BF16 pairs. |x| 2^BITS (rounded to nearest) of x = v 2^-e is written in balanced
+// base-256 digits d0..d(S-1) (|d0| <= 256, of S = 8 <= 128; the others in [-128, 127])
+// carrying the sign of v; slice t holds d_t 2^-8t (S = 8: d_t, as every level has its own
+// accumulator). With 128 added to every byte but the first, the digits are the bytes
+// minus 128, and a byte under the exponent of 2^23 is a float: two instructions a digit
+// where a count of leading zeros and shifts took ten.
 template <int S>
-__device__ __forceinline__ void oz_digits(double v, int e, int d[S]) {
-  const unsigned long long b = (unsigned long long)__double_as_longlong(v);
-  const int E = (int)((b >> 52) & 0x7FF);
-  unsigned long long X = 0ull;
-  if (E != 0 && E != 2047) {
-    const unsigned long long mnt = (b & 0xFFFFFFFFFFFFFull) | (1ull << 52);
-    const int rsh = 1075 + e - E - OzCfg<S>::BITS;  // >= 53 - BITS because |v| < 2^e
-    if (OzCfg<S>::BITS > 52 && rsh <= 0) X = mnt << -rsh;
-    else if (rsh < 64) X = (mnt + (1ull << (rsh - 1))) >> rsh;
-  }
-  int u[S];
+__device__ __forceinline__ void oz_pair(double v0, double v1, int e, uint32_t (&out)[S]) {
+  constexpr int BITS = OzCfg<S>::BITS;
+  // the top digit at byte S - 1
+  constexpr unsigned long long BIAS = 0x8080808080808080ull >> (8 * (9 - S));
+  uint32_t half[2][S];
 #pragma unroll
-  for (int t = 0; t < S; ++t) u[t] = (int)((X >> (8 * (S - 1 - t))) & 255ull);
-  u[0] = (int)(X >> (8 * (S - 1)));
-#pragma unroll
-  for (int t = S - 1; t >= 1; --t)
-    if (u[t] >= 128) {
-      u[t] -= 256;
-      u[t - 1] += 1;
+  for (int i = 0; i < 2; ++i) {
+    const unsigned long long b = (unsigned long long)__double_as_longlong(i ? v1 : v0);
+    const int E = (int)((b >> 52) & 0x7FF);
+    unsigned long long X = 0ull;
+    if (E != 0 && E != 2047) {
+      const unsigned long long mnt = (b & 0xFFFFFFFFFFFFFull) | (1ull << 52);
+      const int rsh = 1075 + e - E - BITS;  // >= 53 - BITS because |v| < 2^e
+      if (BITS > 52 && rsh <= 0) X = mnt << -rsh;
+      else if (rsh < 64) X = (mnt + (1ull << (rsh - 1))) >> rsh;
     }
-  const int sg = (b >> 63) ? -1 : 1;
+    X += BIAS;
+    const uint32_t lo = (uint32_t)X, hi = (uint32_t)(X >> 32);
+    const uint32_t sgn = (uint32_t)(b >> 63) << 31;
 #pragma unroll
-  for (int t = 0; t < S; ++t) d[t] = sg * u[t];
-}
-
-// two neighbouring digits of slice t as BF16 (S = 8: plain integers, as every level has
-// its own accumulator)
-template <int S>
-__device__ __forceinline__ uint32_t oz_pack(int d0, int d1, int t) {
-  const int w = OzCfg<S>::FP64 ? 0 : t;
-  return bf16_of_digit(d0, w) | (bf16_of_digit(d1, w) << 16);
+    for (int t = 0; t < S; ++t) {
+      const int byte = S - 1 - t;
+      float f;
+      if (t == 0) {
+        // the top digit, up to 256 (S = 4: 32-bit numbers and one more)
+        f = (float)(int)(X >> (8 * (S - 1)));
+      } else {
+        const uint32_t w = byte >= 4 ? hi : lo;
+        f = __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7650u | (byte & 3))) - 8388736.0f;
+      }
+      if (!OzCfg<S>::FP64 && t > 0) f *= __uint_as_float((uint32_t)(127 - 8 * t) << 23);
+      half[i][t] = __float_as_uint(f) ^ sgn;
+    }
+  }
+#pragma unroll
+  for (int t = 0; t < S; ++t) out[t] = __byte_perm(half[0][t], half[1][t], 0x7632);
 }
 
 // The exponent of a row from its largest biased exponent field E: the row's largest
@@ -242,11 +241,10 @@ __global__ void __launch_bounds__(256) oz_split_kernel(const double *__restrict_
     uint32_t packed[S][4];
 #pragma unroll
     for (int j = 0; j < 8; j += 2) {
-      int d0[S], d1[S];
-      oz_digits<S>(T[rl][8 * gl + j], e, d0);
-      oz_digits<S>(T[rl][8 * gl + j + 1], e, d1);
+      uint32_t w[S];
+      oz_pair<S>(T[rl][8 * gl + j], T[rl][8 * gl + j + 1], e, w);
 #pragma unroll
-      for (int t = 0; t < S; ++t) packed[t][j / 2] = oz_pack<S>(d0[t], d1[t], t);
+      for (int t = 0; t < S; ++t) packed[t][j / 2] = w[t];
     }
     const int64_t rb = r / OZ_TR, rr = r % OZ_TR;
     const int64_t kc = k0 / TK, kk = k0 % TK;
@@ -344,11 +342,10 @@ __global__ void __launch_bounds__(256) oz_slice_kernel(const double *__restrict_
   uint32_t packed[S][4];
 #pragma unroll
   for (int j = 0; j < 8; j += 2) {
-    int d0[S], d1[S];
-    oz_digits<S>(T[rl][8 * gl + j], e, d0);
-    oz_digits<S>(T[rl][8 * gl + j + 1], e, d1);
+    uint32_t w[S];
+    oz_pair<S>(T[rl][8 * gl + j], T[rl][8 * gl + j + 1], e, w);
 #pragma unroll
-    for (int t = 0; t < S; ++t) packed[t][j / 2] = oz_pack<S>(d0[t], d1[t], t);
+    for (int t = 0; t < S; ++t) packed[t][j / 2] = w[t];
   }
   constexpr int TK = OzCfg<S>::TK;
   const int64_t nkc = (64 / TK) * nkb;
@@ -482,6 +479,101 @@ __device__ __forceinline__ void df_add(float &hi, float &lo, float v) {
   const float e = __fadd_rn(__fsub_rn(hi, __fsub_rn(s, bp)), __fsub_rn(v, bp));
   hi = s;
   lo = __fadd_rn(lo, e);
+}
+
+// The slice products of KS K steps (16 K each, 256 bytes apart in an operand) into the
+// accumulators at column d0: ad, bd describe slice 0 of the operands, a_sl and b_sl are the
+// bytes from slice to slice. acc 0: overwrite the accumulators.
+template <int S, int KS>
+__device__ __forceinline__ void oz_issue(uint64_t ad0, uint64_t bd0, int a_sl, int b_sl, uint32_t d0, uint32_t acc) {
+  using Cfg = OzCfg<S>;
+  constexpr int NACC = Cfg::NACC;
+  // D F32, A/B BF16, K-major both, M = 128; N is set per instruction
+  const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(OZ_BM >> 4) << 24);
+#pragma unroll
+  for (int kk = 0; kk < KS; ++kk) {
+#pragma unroll
+    for (int ti = 0; ti < S; ++ti) {
+      const uint64_t ad = ad0 + (uint64_t)((ti * a_sl + kk * 256) >> 4);
+      // The B slices lie back to back with one 8-row stride, so slices
+      // 0..NACC-1-ti read as one operand of 64 (NACC - ti) rows: an MMA puts
+      // A_ti B_u^T (level ti + u) into accumulators ti.., which are adjacent
+      // column blocks (N of at most 256: two MMAs where there are more). The
+      // first slice's, first in a group, overwrite all of them.
+#pragma unroll
+      for (int o = 0; o < OZ_BN * (NACC - ti); o += 256) {
+        const int nn = OZ_BN * (NACC - ti) - o < 256 ? OZ_BN * (NACC - ti) - o : 256;
+        umma_bf16(d0 + (uint32_t)(ti * OZ_BN + o), ad, bd0 + (uint64_t)((o / OZ_BN * b_sl + kk * 256) >> 4),
+                  idesc | ((uint32_t)(nn >> 3) << 17), (kk == 0 && ti == 0) ? acc : 1u);
+      }
+      // S = 4, 5: the remaining products of levels > 3 go one by one into the
+      // last accumulator
+      if (!Cfg::FP64)
+#pragma unroll
+        for (int ui = ti < NACC ? NACC - ti : 0; ui < S; ++ui) {
+          if (ti + ui > S) continue;
+          umma_bf16(d0 + (uint32_t)((NACC - 1) * OZ_BN), ad, bd0 + (uint64_t)((ui * b_sl + kk * 256) >> 4),
+                    idesc | ((uint32_t)(OZ_BN >> 3) << 17), 1u);
+        }
+    }
+  }
+}
+
+// The sum over one exactly accumulated group of NC columns: added to hi, lo (double-float,
+// level-0 units; of S = 8 fixed point, hi in units of level 3, lo, 0 <= lo < 2^24, of level 6)
+template <int S>
+struct OzSum {
+  using Hi = typename std::conditional<OzCfg<S>::FP64, long long, float>::type;
+  using Lo = typename std::conditional<OzCfg<S>::FP64, int, float>::type;
+};
+template <int S, int NC>
+__device__ __forceinline__ void oz_drain(uint32_t ta, typename OzSum<S>::Hi *hi, typename OzSum<S>::Lo *lo) {
+  constexpr int NACC = OzCfg<S>::NACC;
+  if constexpr (OzCfg<S>::FP64) {
+#pragma unroll
+    for (int cb = 0; cb < NC; cb += 4) {
+      // an accumulator of level l holds an integer of at most (l + 1) 2^22: levels
+      // 0..3 exactly, the deeper ones to a unit of theirs
+      uint32_t r[4][4];
+#pragma unroll
+      for (int l = 0; l < 4; ++l) tmem_ld4(ta + (uint32_t)(l * OZ_BN + cb), r[l]);
+      tmem_ld_wait();
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        long long x = hi[cb + j] + __float2int_rn(__uint_as_float(r[3][j]));
+        x += (long long)__float2int_rn(__uint_as_float(r[2][j])) * 256;
+        x += (long long)__float2int_rn(__uint_as_float(r[1][j])) * 65536;
+        x += (long long)__float2int_rn(__uint_as_float(r[0][j])) * 16777216;
+        hi[cb + j] = x;
+      }
+#pragma unroll
+      for (int l = 4; l < NACC; ++l) tmem_ld4(ta + (uint32_t)(l * OZ_BN + cb), r[l - 4]);
+      tmem_ld_wait();
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int i4 = __float2int_rn(__uint_as_float(r[0][j])), i5 = __float2int_rn(__uint_as_float(r[1][j]));
+        int y = lo[cb + j] + ((i4 & 255) << 16) + ((i5 & 65535) << 8) + __float2int_rn(__uint_as_float(r[2][j]));
+        y += __float2int_rn(__uint_as_float(r[3][j]) * 0x1p-8f);
+        hi[cb + j] += (i4 >> 8) + (i5 >> 16) + (y >> 24);
+        lo[cb + j] = y & 0xFFFFFF;
+      }
+    }
+  } else {
+#pragma unroll
+    for (int cb = 0; cb < NC; cb += 8)
+#pragma unroll
+      for (int ac = 0; ac < NACC; ac += 2) {  // two accumulators at a time: 16 registers
+        uint32_t r[2][8];
+        tmem_ld8(ta + (uint32_t)(ac * OZ_BN + cb), r[0]);
+        tmem_ld8(ta + (uint32_t)((ac + 1) * OZ_BN + cb), r[1]);
+        tmem_ld_wait();
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          df_add(hi[cb + j], lo[cb + j], __uint_as_float(r[0][j]));
+          df_add(hi[cb + j], lo[cb + j], __uint_as_float(r[1][j]));
+        }
+      }
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -686,8 +778,6 @@ __global__ void __maxnreg__(96) oz_gemm_kernel(const OzGemmArgs g) {
     // (Warp-uniform control flow keeps descriptors and barrier addresses in uniform
     // registers; with everything inside one lane's branch an instruction took 84 to
     // 100 cycles to issue, longer than the tensor pipe takes to run it.)
-    // D F32, A/B BF16, K-major both, M = 128; N is set per instruction
-    const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(OZ_BM >> 4) << 24);
     // no-swizzle K-major: core matrices of 8 rows x 16 bytes; LBO steps K (128 B),
     // SBO steps 8 rows (8 x TK x 2 B). Slices, K steps and stages are offsets
     // in 16-byte units (shared addresses stay below 2^18, so the 14-bit address field
@@ -721,35 +811,7 @@ __global__ void __maxnreg__(96) oz_gemm_kernel(const OzGemmArgs g) {
         const uint64_t bd0 = ad0 + (uint64_t)((S * Cfg::A_SL) >> 4);
         const uint32_t d0 = tm + (uint32_t)(b * NACC * OZ_BN);
         if (leader) {
-#pragma unroll
-          for (int kk = 0; kk < Cfg::TK / 16; ++kk) {
-#pragma unroll
-            for (int ti = 0; ti < S; ++ti) {
-              const uint64_t ad = ad0 + (uint64_t)((ti * Cfg::A_SL + kk * 256) >> 4);
-              // The B slices lie back to back with one 8-row stride, so slices
-              // 0..NACC-1-ti read as one operand of 64 (NACC - ti) rows: an MMA puts
-              // A_ti B_u^T (level ti + u) into accumulators ti.., which are adjacent
-              // column blocks (N of at most 256: two MMAs where there are more). The
-              // first slice's, first in a group, overwrite all of them.
-#pragma unroll
-              for (int o = 0; o < OZ_BN * (NACC - ti); o += 256) {
-                const int nn = OZ_BN * (NACC - ti) - o < 256 ? OZ_BN * (NACC - ti) - o : 256;
-                umma_bf16(d0 + (uint32_t)(ti * OZ_BN + o), ad,
-                          bd0 + (uint64_t)((o / OZ_BN * Cfg::B_SL + kk * 256) >> 4),
-                          idesc | ((uint32_t)(nn >> 3) << 17), (kk == 0 && ti == 0) ? acc : 1u);
-              }
-              // S = 4, 5: the remaining products of levels > 3 go one by one into the
-              // last accumulator
-              if (!Cfg::FP64)
-#pragma unroll
-                for (int ui = ti < NACC ? NACC - ti : 0; ui < S; ++ui) {
-                  if (ti + ui > S) continue;
-                  umma_bf16(d0 + (uint32_t)((NACC - 1) * OZ_BN), ad,
-                            bd0 + (uint64_t)((ui * Cfg::B_SL + kk * 256) >> 4),
-                            idesc | ((uint32_t)(OZ_BN >> 3) << 17), 1u);
-                }
-            }
-          }
+          oz_issue<S, Cfg::TK / 16>(ad0, bd0, Cfg::A_SL, Cfg::B_SL, d0, acc);
           umma_commit(bar(EMPTY + st));
           if (gend) umma_commit(bar(TFULL + b));
         }
@@ -819,12 +881,9 @@ __global__ void __maxnreg__(96) oz_gemm_kernel(const OzGemmArgs g) {
       const int eb = lane < OZ_EPI_COLS && col_base + lane < g.N
                          ? g.b_ex[t.z * g.b_bs_ex + g.b_rb0 * OZ_TR + col_base + lane] : 0;
       const int ngr = (t.nch + GROUP - 1) / GROUP;
-      // the tile's sum over its K groups: in double-float (level-0 units); of S = 8 in
-      // fixed point, hi in units of level 3 (2^-24) and lo, 0 <= lo < 2^24, of level 6 (2^-48)
-      using Hi = typename std::conditional<Cfg::FP64, long long, float>::type;
-      using Lo = typename std::conditional<Cfg::FP64, int, float>::type;
-      Hi hi[OZ_EPI_COLS];
-      Lo lo[OZ_EPI_COLS];
+      // the tile's sum over its K groups
+      typename OzSum<S>::Hi hi[OZ_EPI_COLS];
+      typename OzSum<S>::Lo lo[OZ_EPI_COLS];
 #pragma unroll
       for (int j = 0; j < OZ_EPI_COLS; ++j) {
         hi[j] = 0;
@@ -843,51 +902,7 @@ __global__ void __maxnreg__(96) oz_gemm_kernel(const OzGemmArgs g) {
         }
         tc_fence_after();
         const uint32_t ta = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(b * NACC * OZ_BN + part * OZ_EPI_COLS);
-        if constexpr (Cfg::FP64) {
-#pragma unroll
-          for (int cb = 0; cb < OZ_EPI_COLS; cb += 4) {
-            // an accumulator of level l holds an integer of at most (l + 1) 2^22: levels
-            // 0..3 exactly, the deeper ones to a unit of theirs
-            uint32_t r[4][4];
-#pragma unroll
-            for (int l = 0; l < 4; ++l) tmem_ld4(ta + (uint32_t)(l * OZ_BN + cb), r[l]);
-            tmem_ld_wait();
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              long long x = hi[cb + j] + __float2int_rn(__uint_as_float(r[3][j]));
-              x += (long long)__float2int_rn(__uint_as_float(r[2][j])) * 256;
-              x += (long long)__float2int_rn(__uint_as_float(r[1][j])) * 65536;
-              x += (long long)__float2int_rn(__uint_as_float(r[0][j])) * 16777216;
-              hi[cb + j] = x;
-            }
-#pragma unroll
-            for (int l = 4; l < NACC; ++l) tmem_ld4(ta + (uint32_t)(l * OZ_BN + cb), r[l - 4]);
-            tmem_ld_wait();
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              const int i4 = __float2int_rn(__uint_as_float(r[0][j])), i5 = __float2int_rn(__uint_as_float(r[1][j]));
-              int y = lo[cb + j] + ((i4 & 255) << 16) + ((i5 & 65535) << 8) + __float2int_rn(__uint_as_float(r[2][j]));
-              y += __float2int_rn(__uint_as_float(r[3][j]) * 0x1p-8f);
-              hi[cb + j] += (i4 >> 8) + (i5 >> 16) + (y >> 24);
-              lo[cb + j] = y & 0xFFFFFF;
-            }
-          }
-        } else {
-#pragma unroll
-          for (int cb = 0; cb < OZ_EPI_COLS / 8; ++cb)
-#pragma unroll
-            for (int ac = 0; ac < NACC; ac += 2) {  // two accumulators at a time: 16 registers
-              uint32_t r[2][8];
-              tmem_ld8(ta + (uint32_t)(ac * OZ_BN + cb * 8), r[0]);
-              tmem_ld8(ta + (uint32_t)((ac + 1) * OZ_BN + cb * 8), r[1]);
-              tmem_ld_wait();
-#pragma unroll
-              for (int j = 0; j < 8; ++j) {
-                df_add(hi[cb * 8 + j], lo[cb * 8 + j], __uint_as_float(r[0][j]));
-                df_add(hi[cb * 8 + j], lo[cb * 8 + j], __uint_as_float(r[1][j]));
-              }
-            }
-        }
+        oz_drain<S, OZ_EPI_COLS>(ta, hi, lo);
         // every load of this set has completed: hand it back to the MMA warp
         tc_fence_before();
         __syncwarp();
@@ -1049,6 +1064,229 @@ void oz_gemm(cudaStream_t s, const OzSplit &A, int64_t a_row0, const OzSplit &B,
              double *C, int64_t ldc, bool lower_only, int *err, const int *status) {
   oz_gemm_batched(s, A, a_row0, B, b_row0, M, N, kc0, kc1, kmode, alpha, beta, C, ldc, 0, lower_only,
                   err, status, 0, 1);
+}
+
+// ---------------------------------------------------------------------------
+// a 64-wide block column of the Cholesky's outer panel, in one kernel
+// ---------------------------------------------------------------------------
+// Rows [r0, r1) of the block column at j0, 128 to a CTA:
+//   L = A W^T (W: the diagonal block's inverse), written over A, then
+//   A_q -= L L_q^T for the panel's next q1 64-wide column blocks, L_q the rows j0 + 64 (q + 1)
+//   .. of the block column (finished before).
+// Every operand is 64 K wide, so it is split where it is used: the rows' exponents and
+// slices go from registers to shared memory and on to the tensor cores, and neither the
+// slices nor L in slices pass through memory. As split, split, product, split, split,
+// product the block took six launches and ~280 us of a 32-SM share at n = 16384 for work
+// of ~20 us. The products, their order and their rounding are those of oz_split and
+// oz_gemm. (One loop body serves every
+// round: its phases run once or a few times, and with a copy for each product the warps
+// spent 44% of their time waiting for instructions.)
+constexpr int PB_THREADS = 512;
+constexpr int PB_SBO = 1024;  // 8 rows x 64 K x 2 bytes
+
+template <int S>
+struct PbCfg {
+  static constexpr int A_SL = OZ_BM * 64 * 2, B_SL = OZ_BN * 64 * 2;  // a slice of 64 K
+  static constexpr int SMEM = S * (A_SL + B_SL) + 1024;
+  static constexpr uint32_t TMEM_COLS = OzCfg<S>::NACC * OZ_BN;  // 256 or 512
+};
+
+// NV entries (a multiple of 8) of row r, K 8 kg0 .., as slices at base. Rolled over the
+// pairs: the kernel's phases run once or a few times each, and with everything unrolled
+// its warps spent 44% of their time waiting for instructions.
+template <int S, int NV>
+__device__ __forceinline__ void pb_put(uint8_t *base, int sl, int r, int kg0, const double *v, int e) {
+  uint8_t *dst = base + (r >> 3) * PB_SBO + kg0 * 128 + (r & 7) * 16;
+#pragma unroll
+  for (int g = 0; g < NV / 8; ++g)
+#pragma unroll
+    for (int j = 0; j < 8; j += 2) {
+      uint32_t w[S];
+      oz_pair<S>(v[8 * g + j], v[8 * g + j + 1], e, w);
+#pragma unroll
+      for (int t = 0; t < S; ++t) *reinterpret_cast<uint32_t *>(dst + t * sl + g * 128 + 2 * j) = w[t];
+    }
+}
+
+__device__ __forceinline__ int pb_field(double v) {
+  return (int)(((unsigned long long)__double_as_longlong(v) >> 52) & 0x7FF);
+}
+
+template <int S>
+__global__ void __launch_bounds__(PB_THREADS) panel_block_kernel(double *__restrict__ A, int64_t lda, int64_t r0,
+                                                                 int64_t r1, int64_t j0,
+                                                                 const double *__restrict__ W, int q1, int *err,
+                                                                 const int *__restrict__ status) {
+  using Cfg = PbCfg<S>;
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  uint8_t *As = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023), *Bs = As + S * Cfg::A_SL;
+  __shared__ int amax[OZ_BM], bmax[OZ_BN];
+  __shared__ uint64_t bar;
+  __shared__ uint32_t tmem_sh;
+  if (status && *(volatile const int *)status != 0) return;
+  const int tid = threadIdx.x, warp = tid >> 5;
+  if (tid == 0) {
+    mbar_init(smem_u32(&bar), 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_sh)),
+                 "r"(Cfg::TMEM_COLS));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = tmem_sh;
+  // this thread's row of the tile and its 16 columns of a 64-wide block; in the second
+  // operand its row and 8 columns
+  const int row = tid & 127, part = tid >> 7, brow = tid & 63, bpart = tid >> 6;
+  const uint32_t ta = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(part * 16);
+  const uint64_t ad = umma_desc(smem_u32(As), 128u, PB_SBO), bd = umma_desc(smem_u32(Bs), 128u, PB_SBO);
+  uint32_t ph = 0;
+  bool ok = true;
+  // operands in shared memory -> products in TMEM (false: the wait ran out)
+  auto product = [&]() -> bool {
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 0) {
+      tc_fence_after();
+      if (elect_one()) {
+        oz_issue<S, 4>(ad, bd, Cfg::A_SL, Cfg::B_SL, tmem, 0u);
+        umma_commit(smem_u32(&bar));
+      }
+      __syncwarp();
+    }
+    const bool done = mbar_wait_bounded(smem_u32(&bar), ph);
+    ph ^= 1u;
+    tc_fence_after();
+    return !__syncthreads_or(!done);
+  };
+  // TMEM -> 16 doubles of this thread's row (power of two ea) and columns (bmax)
+  auto results = [&](double (&v)[16], int ea, uint32_t negmask) {
+#pragma unroll
+    for (int h = 0; h < 16; h += 8) {
+      typename OzSum<S>::Hi hi[8];
+      typename OzSum<S>::Lo lo[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        hi[j] = 0;
+        lo[j] = 0;
+      }
+      oz_drain<S, 8>(ta + (uint32_t)h, hi, lo);
+      bool slow = false;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const int sh = ea + oz_exponent<S>(bmax[part * 16 + h + j]);
+        if constexpr (OzCfg<S>::FP64) {
+          v[h + j] = fixed_to_double(hi[j], lo[j], sh, negmask, slow);
+        } else {
+          hi[j] = __uint_as_float(__float_as_uint(hi[j]) ^ negmask);
+          lo[j] = __uint_as_float(__float_as_uint(lo[j]) ^ negmask);
+          v[h + j] = df2d_try(hi[j], lo[j], sh - 16, slow);
+        }
+      }
+      if (__any_sync(0xffffffffu, slow)) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const int sh = ea + oz_exponent<S>(bmax[part * 16 + h + j]);
+          if constexpr (OzCfg<S>::FP64) v[h + j] = fixed_to_double_slow(hi[j], lo[j], sh, negmask);
+          else v[h + j] = df2d_scaled(hi[j], lo[j], sh - 16);
+        }
+      }
+    }
+    tc_fence_before();
+  };
+  // the second operand: 64 rows of P (leading dimension ld)
+  auto load_b = [&](const double *P, int64_t ld) {
+    double b[8];
+    int mx = 0;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      b[k] = P[brow + (8 * bpart + k) * ld];
+      mx = max(mx, pb_field(b[k]));
+    }
+    atomicMax(&bmax[brow], mx);
+    __syncthreads();
+    pb_put<S, 8>(Bs, Cfg::B_SL, brow, bpart, b, oz_exponent<S>(bmax[brow]));
+  };
+  // the first operand: this thread's 16 entries of its row; returns the row's power of two
+  auto put_a = [&](const double (&v)[16]) -> int {
+    int mx = 0;
+#pragma unroll
+    for (int k = 0; k < 16; ++k) mx = max(mx, pb_field(v[k]));
+    atomicMax(&amax[row], mx);
+    __syncthreads();
+    const int e = oz_exponent<S>(amax[row]);
+    pb_put<S, 16>(As, Cfg::A_SL, row, 2 * part, v, e);
+    return e;
+  };
+  for (int64_t t0 = r0 + (int64_t)blockIdx.x * OZ_BM; ok && t0 < r1; t0 += (int64_t)gridDim.x * OZ_BM) {
+    const int64_t gr = t0 + row;
+    const bool in = gr < r1;
+    double v[16];
+    double *ar = A + gr + (j0 + 16 * part) * lda;
+#pragma unroll
+    for (int k = 0; k < 16; ++k) v[k] = in ? ar[k * lda] : 0.0;
+    int ea = 0;
+    // round -1: L = A W^T; round q: the update of column block q
+#pragma unroll 1
+    for (int q = -1; q < q1; ++q) {
+      __syncthreads();
+      if (tid < OZ_BN) bmax[tid] = 0;
+      if (q <= 0 && tid >= 128 && tid < 128 + OZ_BM) amax[tid - 128] = 0;
+      __syncthreads();
+      if (q <= 0) ea = put_a(v);
+      const double *P = q < 0 ? W : A + j0 + 64 * (q + 1) + j0 * lda;
+      load_b(P, q < 0 ? NB : lda);
+      double *cr = A + gr + (j0 + 64 * (q + 1) + 16 * part) * lda;
+      double c[16];
+#pragma unroll
+      for (int k = 0; k < 16; ++k) c[k] = q >= 0 && in ? cr[k * lda] : 0.0;
+      if (!(ok = product())) break;
+      double u[16];
+      results(u, ea, q < 0 ? 0u : 0x80000000u);
+#pragma unroll
+      for (int k = 0; k < 16; ++k) {
+        if (q < 0) v[k] = u[k];
+        else u[k] += c[k];
+        if (in) cr[k * lda] = u[k];
+      }
+    }
+  }
+  if (!ok && tid == 0) atomicExch(err, 5);
+  __syncthreads();
+  if (warp == 0) {
+    __syncwarp();
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(Cfg::TMEM_COLS));
+  }
+}
+
+template <int S>
+static void launch_panel_block(cudaStream_t s, double *A, int64_t lda, int64_t r0, int64_t r1, int64_t j0,
+                               const double *W, int q1, int *err, const int *status) {
+  static PerDevice attr;
+  per_device(attr, [] {
+    GPGP_CUDA(cudaFuncSetAttribute(panel_block_kernel<S>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   PbCfg<S>::SMEM));
+    return 1;
+  });
+  const int cap = tl_oz_grid_cap > 0 ? std::min(tl_oz_grid_cap, oz_sm_count()) : oz_sm_count();
+  const int64_t tiles = (r1 - r0 + OZ_BM - 1) / OZ_BM;
+  const double fl = 2.0 * OZ_BM * OZ_BN * 64 * (double)tiles * (1 + q1) * OzCfg<S>::PRODUCTS;
+  KTScope kts(GPGP_KPROF_OZ_GEMM, s, fl);
+  panel_block_kernel<S><<<(unsigned)std::min<int64_t>(tiles, cap), PB_THREADS, PbCfg<S>::SMEM, s>>>(
+      A, lda, r0, r1, j0, W, q1, err, status);
+  GPGP_CHECK_LAUNCH();
+}
+
+void panel_block(cudaStream_t s, int S, double *A, int64_t lda, int64_t r0, int64_t r1, int64_t j0, const double *W,
+                 int q1, int *err, const int *status) {
+  if (r1 <= r0) return;
+  if (S == OZ_FP64) launch_panel_block<OZ_FP64>(s, A, lda, r0, r1, j0, W, q1, err, status);
+  else launch_panel_block<4>(s, A, lda, r0, r1, j0, W, q1, err, status);
 }
 
 }  // namespace gpgp

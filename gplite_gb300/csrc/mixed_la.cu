@@ -5,11 +5,9 @@
 // of 32-bit fixed-point row slices, accumulated exactly, summed in FP64).
 //
 // Cholesky is two-level right-looking: outer panels of NBO columns (384: faster
-// at n = 16384 than 256 or 512), each factored with the 64-wide FP64 diagonal
-// kernel of dense.cu, a sliced GEMM for the panel solve L21 = A21 W11^T and
-// sliced GEMMs for the updates inside the panel; one sliced SYRK with K = NBO
-// then updates the trailing matrix, so every trailing element is rewritten in
-// FP64 once per outer panel.
+// at n = 16384 than 256 or 512), each factored in 64-wide blocks (factor_panel); one
+// sliced SYRK with K = NBO then updates the trailing matrix, so every trailing element is
+// rewritten in FP64 once per outer panel.
 #include <math.h>
 
 #include <algorithm>
@@ -29,59 +27,62 @@ namespace {
 #ifndef GPGP_NBO
 #define GPGP_NBO 384
 #endif
-constexpr int64_t NBO = GPGP_NBO;  // outer panel width of the mixed Cholesky (a build-time tuning knob)
+constexpr int64_t NBO = GPGP_NBO;  // outer panel width of the Cholesky (a build-time tuning knob)
+static_assert(NBO % NB == 0, "an outer panel is whole blocks wherever rows lie below it");
 // Lookahead: a trailing update of at least LOOK_MIN_ROWS rows leaves LOOK_PANEL_SMS
 // SMs to the next panel's factorisation, whose GEMMs are capped to them.
 constexpr int64_t LOOK_MIN_ROWS = 6144;
 constexpr int LOOK_PANEL_SMS = 32;
 
-// The 64-wide blocks of the outer panel [k0, k0 + kbo). Only the panel's own rows
-// lie on the chain from one diagonal block to the next, so they are kept apart:
-//  - chain (stream x): the FP64 factor and inverse W of the diagonal block, the
-//    block's rows inside the panel L_p = A_p W^T (FP64, by the inverse), and the
-//    FP64 update of the rest of the panel's lower triangle by them;
-//  - bulk (stream y, after the chain's block): the rows below the panel,
-//    L_b = A_b W^T, and their update of the panel's remaining columns
-//    A_b,rest -= L_b L_p^T, both sliced GEMMs.
-// x and y may be the same stream (the single-stream schedule; same products in
-// the same order, so the same factor). With two streams the bulk GEMMs take no
-// status word: the chain's diagonal kernels may set it while they run.
-void factor_panel(cudaStream_t x, cudaStream_t y, const SideStream *sd, double *A, int64_t n, int64_t lda,
-                  double *Winv, double *logdet_part, int *status, int *err, int64_t k0, int64_t kbo, SplitBuf &a,
-                  SplitBuf &w, SplitBuf &lp) {
+// The 64-wide blocks of the outer panel [k0, k0 + kbo). What the next diagonal block
+// waits for is kept apart from the rest:
+//  - chain (stream x): the factor and inverse W of the diagonal block, the panel's rows
+//    L_p = A_p W^T and the next diagonal block's update by its own rows, on the FP64 pipe;
+//  - the rest of the panel (stream z, after the panel's rows): the update of the panel's
+//    lower triangle beside that block. The chain waits for it after its next diagonal
+//    block;
+//  - bulk (stream y, after the panel's rows): the rows below the panel, L_b = A_b W^T,
+//    and their update of the panel's remaining columns (panel_block).
+// x, y and z may be the same stream (the single-stream schedule; same products in the
+// same order, so the same factor). With more streams the bulk takes no status word: the
+// chain's diagonal kernels may set it while they run.
+void factor_panel(cudaStream_t x, cudaStream_t y, cudaStream_t z, const SideStream *sd, double *A, int64_t n,
+                  int64_t lda, double *Winv, double *logdet_part, int *status, int *err, int64_t k0, int64_t kbo,
+                  int S) {
   const bool two = x != y;
   const int64_t pend = k0 + kbo;  // first row / column after the panel
   const int64_t mb = n - pend;    // rows below the panel
+  const int *sst = two ? nullptr : status;
+  bool rest = false;              // the block before left work on z
   for (int64_t j0 = k0; j0 < pend; j0 += NB) {
     const int jb = (int)std::min<int64_t>(NB, pend - j0);
     const int64_t blk = j0 / NB;
     double *Wb = Winv + blk * NB * NB;
-    potrf_diag(x, A + j0 + j0 * lda, jb, lda, Wb, logdet_part + blk, status, j0, 0, 0, 0, 1);
+    potrf_diag(x, A + j0 + j0 * lda, jb, lda, Wb, logdet_part + blk, status, j0, 0, 0, 0, 1, S != OZ_FP64);
     const int64_t mp = pend - (j0 + jb);  // panel rows below the block
-    double *Ap = A + (j0 + jb) + j0 * lda;
+    double *Ln = A + (j0 + NB) + j0 * lda;
     if (mp > 0) {
-      potrf_panel_inv_kernel<<<(unsigned)((mp + 3) / 4), 256, 0, x>>>(Ap, mp, jb, lda, Wb, status);
+      if (two && rest) GPGP_CUDA(cudaStreamWaitEvent(x, sd->e, 0));
+      potrf_panel_inv_kernel<<<(unsigned)((mp + 3) / 4), 256, 0, x>>>(Ln, mp, jb, lda, Wb, status);
       GPGP_CHECK_LAUNCH();
     }
+    rest = mp > NB;
     if (two) {
       GPGP_CUDA(cudaEventRecord(sd->c, x));
-      GPGP_CUDA(cudaStreamWaitEvent(y, sd->c, 0));
+      if (rest) GPGP_CUDA(cudaStreamWaitEvent(z, sd->c, 0));
+      if (mb > 0) GPGP_CUDA(cudaStreamWaitEvent(y, sd->c, 0));
     }
-    if (mp > 0)
-      gemm64(x, false, true, mp, mp, jb, -1.0, Ap, lda, Ap, lda, 1.0, A + (j0 + jb) + (j0 + jb) * lda, lda, true, 0);
-    if (mb <= 0) continue;
-    double *Ab = A + pend + j0 * lda;
-    const int *sst = two ? nullptr : status;
-    oz_split(y, Ab, lda, 0, mb, jb, &a.sp);
-    oz_split(y, Wb, NB, 0, jb, jb, &w.sp);
-    oz_gemm(y, a.sp, 0, w.sp, 0, mb, jb, 0, 1, 0, 1.0, 0.0, Ab, lda, false, err, sst);
-    if (mp > 0) {
-      oz_split(y, Ab, lda, 0, mb, jb, &a.sp);
-      oz_split(y, Ap, lda, 0, mp, jb, &lp.sp);
-      oz_gemm(y, a.sp, 0, lp.sp, 0, mb, mp, 0, 1, 0, -1.0, 1.0, A + pend + (j0 + jb) * lda, lda, false, err, sst);
+    if (mp > 0) syrk_block(x, Ln, lda, (int)std::min<int64_t>(NB, mp), A + (j0 + NB) * (lda + 1));
+    if (rest) {
+      const int64_t mr = mp - NB, i0 = j0 + 2 * NB;  // rows from i0 on
+      double *Lr = A + i0 + j0 * lda;
+      gemm64(z, false, true, mr, NB, jb, -1.0, Lr, lda, Ln, lda, 1.0, A + i0 + (j0 + NB) * lda, lda, false, 0);
+      gemm64(z, false, true, mr, mr, jb, -1.0, Lr, lda, Lr, lda, 1.0, A + i0 + i0 * lda, lda, true, 0);
+      if (two) GPGP_CUDA(cudaEventRecord(sd->e, z));
     }
+    if (mb > 0) panel_block(y, S, A, lda, pend, n, j0, Wb, (int)(mp / NB), err, sst);
   }
-  if (two) {  // the panel is complete on x once the bulk is
+  if (two) {  // the panel is complete on x once the bulk is (z's work precedes it or x's)
     GPGP_CUDA(cudaEventRecord(sd->b, y));
     GPGP_CUDA(cudaStreamWaitEvent(x, sd->b, 0));
   }
@@ -91,17 +92,15 @@ void factor_panel(cudaStream_t x, cudaStream_t y, const SideStream *sd, double *
 
 void potrf_mixed(cudaStream_t s, double *A, int64_t n, int64_t lda, double *Winv,
                  double *logdet_part, int *status, int *err, const SideStream *side, int S) {
-  SplitBuf a(s, n, NBO, S);    // panel operand (rows below the current block)
-  SplitBuf w(s, NB, NB, S);    // inverse of the diagonal block
-  SplitBuf lp(s, NBO, NB, S);  // the block's rows inside the panel
+  SplitBuf a(s, n, NBO, S);  // the panel as the trailing update's operand
   cudaStreamCaptureStatus cap_st = cudaStreamCaptureStatusNone;
   GPGP_CUDA(cudaStreamIsCapturing(s, &cap_st));
   // Per-kernel timers (tl_kt) time each launch alone, so a profiled call runs the
   // single-stream schedule.
-  if (!side || !side->s || n <= 2 * NBO || cap_st != cudaStreamCaptureStatusNone || tl_kt) {
+  if (!side || !side->s3 || n <= 2 * NBO || cap_st != cudaStreamCaptureStatusNone || tl_kt) {
     for (int64_t k0 = 0; k0 < n; k0 += NBO) {
       const int64_t kbo = std::min<int64_t>(NBO, n - k0);
-      factor_panel(s, s, nullptr, A, n, lda, Winv, logdet_part, status, err, k0, kbo, a, w, lp);
+      factor_panel(s, s, s, nullptr, A, n, lda, Winv, logdet_part, status, err, k0, kbo, S);
       const int64_t m2 = n - k0 - kbo;
       if (m2 > 0) {
         double *P = A + (k0 + kbo) + k0 * lda;
@@ -117,7 +116,6 @@ void potrf_mixed(cudaStream_t s, double *A, int64_t n, int64_t lda, double *Winv
   // (event a), and then applies p to the rest of the trailing matrix while panel
   // p + 1 is factored beside it (the two touch disjoint columns). Every product
   // is the one the plain schedule computes, so the factor is the same.
-  SplitBuf t(s, n, NBO, S);  // panel p as the trailing update's operand
   cudaStream_t x = side->s;
   GPGP_CUDA(cudaEventRecord(side->fork, s));
   GPGP_CUDA(cudaStreamWaitEvent(x, side->fork, 0));
@@ -127,8 +125,8 @@ void potrf_mixed(cudaStream_t s, double *A, int64_t n, int64_t lda, double *Winv
     const SideStream *sd;
     cudaStream_t main;
     ~Join() {
-      if (sd->s2) {  // the bulk stream first (an error may leave the panel loop early)
-        cudaEventRecord(sd->b, sd->s2);
+      for (cudaStream_t o : {sd->s2, sd->s3}) {  // (an error may leave the panel loop early)
+        cudaEventRecord(sd->b, o);
         cudaStreamWaitEvent(sd->s, sd->b, 0);
       }
       cudaEventRecord(sd->l, sd->s);
@@ -141,7 +139,7 @@ void potrf_mixed(cudaStream_t s, double *A, int64_t n, int64_t lda, double *Winv
     const int64_t kbo = std::min<int64_t>(NBO, n - k0);
     {
       OzGridCap cap(panel_cap);
-      factor_panel(x, side->s2 ? side->s2 : x, side, A, n, lda, Winv, logdet_part, status, err, k0, kbo, a, w, lp);
+      factor_panel(x, side->s2, side->s3, side, A, n, lda, Winv, logdet_part, status, err, k0, kbo, S);
     }
     GPGP_CUDA(cudaEventRecord(side->l, x));
     GPGP_CUDA(cudaStreamWaitEvent(s, side->l, 0));
@@ -149,9 +147,9 @@ void potrf_mixed(cudaStream_t s, double *A, int64_t n, int64_t lda, double *Winv
     if (m2 <= 0) break;
     double *P = A + (k0 + kbo) + k0 * lda;
     double *C = A + (k0 + kbo) + (k0 + kbo) * lda;
-    oz_split(s, P, lda, 0, m2, kbo, &t.sp);
+    oz_split(s, P, lda, 0, m2, kbo, &a.sp);
     const int64_t nb2 = std::min<int64_t>(NBO, m2);
-    oz_gemm(s, t.sp, 0, t.sp, 0, m2, nb2, 0, (kbo + 63) / 64, 0, -1.0, 1.0, C, lda, true, err, status);
+    oz_gemm(s, a.sp, 0, a.sp, 0, m2, nb2, 0, (kbo + 63) / 64, 0, -1.0, 1.0, C, lda, true, err, status);
     GPGP_CUDA(cudaEventRecord(side->a, s));
     GPGP_CUDA(cudaStreamWaitEvent(x, side->a, 0));
     const int64_t m3 = m2 - nb2;
@@ -162,7 +160,7 @@ void potrf_mixed(cudaStream_t s, double *A, int64_t n, int64_t lda, double *Winv
       OzGridCap cap(share ? sms - LOOK_PANEL_SMS : 0);
       // no status word: the side stream's diagonal kernels may set it while this
       // launch runs, and every role of a GEMM CTA must see the same value
-      oz_gemm(s, t.sp, nb2, t.sp, nb2, m3, m3, 0, (kbo + 63) / 64, 0, -1.0, 1.0, C + nb2 + nb2 * lda, lda,
+      oz_gemm(s, a.sp, nb2, a.sp, nb2, m3, m3, 0, (kbo + 63) / 64, 0, -1.0, 1.0, C + nb2 + nb2 * lda, lda,
               true, err, nullptr);
     }
   }
