@@ -309,7 +309,7 @@ constexpr int OZ_FP64 = 8;
 // against 2.38 / 2.54 / 18.6 (n <= 768 has one outer panel's lookahead too few: 2.76 /
 // 2.03 / 18.2 against 2.61 / 2.65 / 22.7 at 760).
 #ifndef GPGP_SLICED_MIN
-#define GPGP_SLICED_MIN 960
+#define GPGP_SLICED_MIN 896
 #endif
 constexpr int64_t SLICED_MIN = GPGP_SLICED_MIN;
 struct OzSplit {

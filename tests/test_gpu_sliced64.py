@@ -26,7 +26,7 @@ def test_sliced_product_is_as_accurate_as_fp64(M, N, K):
     assert 0.0 <= err.value <= 64.0 * K * (2.0 ** -58 + 2.0 ** -53) / 0.25
 
 
-@pytest.mark.parametrize("n", [959, 960, 961, 1024, 1153, 1600])
+@pytest.mark.parametrize("n", [895, 896, 897, 959, 960, 961, 1024, 1153, 1600])
 def test_fp64_fit_either_side_of_the_sliced_sizes(n):
     """Evidence, gradient and predictions around the size where the factorisation's
     products move to the tensor cores, at the FP64 path's tolerance."""
