@@ -489,8 +489,7 @@ void run_bucket(gpgp_batch *b, Bucket &k, cudaStream_t st) {
       for (int64_t j0 = k0; j0 < k0 + kbo; j0 += NB) {
         const int64_t blk = j0 / NB;
         double *Akk = k.Bm.p + j0 + j0 * nb;
-        potrf_diag(st, Akk, NB, nb, k.Winv.p + blk * NB * NB, k.ldp.p + blk, k.status.p, j0, nb * nb, nb * NB, nbl, P,
-                   true);
+        potrf_diag(st, Akk, NB, nb, k.Winv.p + blk * NB * NB, k.ldp.p + blk, k.status.p, j0, nb * nb, nb * NB, nbl, P);
         const int64_t m = nb - j0 - NB;
         if (m <= 0) continue;
         double *A21 = k.Bm.p + (j0 + NB) + j0 * nb;

@@ -219,15 +219,13 @@ void cov_matvec_df(cudaStream_t s, const DevKernel &dk, uint32_t gmask, const do
 // dense FP64 linear algebra (column-major)
 // ---------------------------------------------------------------------------
 constexpr int NB = 64;  // block size of the blocked factorisations
-constexpr int DIAG_THREADS = 512;  // threads of the diagonal-block kernel (potrf_diag_kernel)
 // D -= L L^T (lower triangle) for L = m x 64, m <= 64, both of leading dimension lda
 void syrk_block(cudaStream_t s, const double *Ln, int64_t lda, int m, double *D);
 // Factor and inverse of the kb x kb (kb <= 64) diagonal block of each of `batch` problems
 // (matrices sA, inverses sW, log-determinant parts sL apart, one status word each); a
-// pivot that is not positive sets the status to its number, k0 + 1 ... (rank1: the FP64
-// pipe's rounding that the mixed precision is kept at.)
+// pivot that is not positive sets the status to its number, k0 + 1 ...
 void potrf_diag(cudaStream_t s, double *A, int kb, int64_t lda, double *Winv, double *logdet_part, int *status,
-                int64_t k0, int64_t sA, int64_t sW, int64_t sL, int64_t batch, bool rank1 = false);
+                int64_t k0, int64_t sA, int64_t sW, int64_t sL, int64_t batch);
 
 // C = alpha * op(A) op(B) + beta * C. lower_only: only tiles on/below the
 // diagonal of C are computed (SYRK-style). tri_k: A and B are triangular so

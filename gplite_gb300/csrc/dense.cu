@@ -6,8 +6,8 @@
 // R/laplace.R:30, R/gp_pred.R:209).
 //
 // The factorisation is blocked right-looking with NB = 64: the diagonal block
-// is factored by one CTA in shared memory, which also inverts it (the inverses
-// serve the solves); the panel below is solved by row-parallel substitution,
+// is factored and inverted by one cluster of CTAs (diag.cu; the inverses serve the
+// solves); the panel below is solved by row-parallel substitution,
 // which stays backward stable when a diagonal block is ill-conditioned (FITC's
 // K_z); the trailing update is a lower-only GEMM on the FP64 pipe. The
 // triangular solves are single launches ordered by per-block flags.
@@ -244,564 +244,6 @@ void gemm64(cudaStream_t s, bool ta, bool tb, int64_t M, int64_t N, int64_t K, d
   }
   gemm64_batched(s, ta, tb, M, N, K, alpha, A, lda, 0, B, ldb, 0, beta, C, ldc, 0, 1, lower_only,
                  tri_mode);
-}
-
-// ---------------------------------------------------------------------------
-// diagonal block: factor + invert in shared memory (one CTA)
-// ---------------------------------------------------------------------------
-// On this part an FP64 warp instruction holds its SM sub-partition for 64 cycles (76
-// with all four busy, 1.7 multiply-adds a clock for the SM), so the block's factor and
-// inverse, 2 x 43.7 k multiply-adds, would be 52 k cycles of that pipe alone. Only the
-// chain of the 64 pivots stays on it. Everything else is products of 16 x 16 blocks, and
-// those run in 58-bit fixed point on the integer pipe (limb_dot): an operand's row gets
-// the power of two of its largest entry and each entry two signed 30-bit limbs, a
-// multiply-add is four 32 x 32 + 64-bit ones (10 a clock for the SM), and a term's error is
-// 2^-58 of the product of the rows' scales where the FP64 pipe's is 2^-53 of the sum.
-// 51 us per 64 x 64 block, against 65 us with a rank-1 update and a barrier per column on
-// the FP64 pipe. (The pivots in integers as well were no faster: 64-bit shifts, counts of
-// leading zeros and high products take 16 to 50 cycles each, and a pivot needs a dozen.)
-//  A(p)  four warps factor the 16 x 16 diagonal block of panel p in registers, as LDL^T:
-//        the update of entry (r, c) by pivot k is -(t_r t_c) y with y = 1 / d_k, so that
-//        between two pivots lie the reciprocal (three dependent FP64 instructions), one
-//        multiply-add and a trip through shared memory. The square roots come at the
-//        end, all at once. A fifth warp follows one step behind and builds the block's
-//        inverse W_pp; the other warps convert panel p's rows for B(p) and complete the
-//        inverse's block row p - 1.
-//  B(p)  the rows below: L_ip = A_ip W_pp^T;
-//  C(p)  their update of the trailing triangle.
-// The helpers are not inlined: unrolled into every place the kernel was 82 KB of code,
-// and its phases, which run once or a few times each, waited for instructions.
-
-// -x by flipping the sign bit (an integer instruction, not an FP64 one)
-__device__ __forceinline__ double neg_bits(double x) {
-  return __longlong_as_double(__double_as_longlong(x) ^ (long long)0x8000000000000000ull);
-}
-
-// 1/x for a positive normal x: the FP32 reciprocal of x's mantissa (relative error
-// |e| < 2^-22) refined by (1 - e)^-1 = 1 + e + e^2 + O(e^3), e = 1 - m y0, and the power
-// of two put back on the exponent. No branch, so that other work can be scheduled into
-// its latencies.
-__device__ __forceinline__ double rcp_fast(double x) {
-  const unsigned long long b = (unsigned long long)__double_as_longlong(x);
-  const int E = (int)((b >> 52) & 0x7FF);
-  const double m = __longlong_as_double((long long)((b & 0xFFFFFFFFFFFFFull) | (1023ull << 52)));
-  float yf;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(yf) : "f"(__uint_as_float((127u << 23) | (uint32_t)((b >> 29) & 0x7FFFFFu))));
-  const uint32_t yb = __float_as_uint(yf);
-  const double y0 = __longlong_as_double(
-      (long long)(((unsigned long long)((yb >> 23) + 896u) << 52) | ((unsigned long long)(yb & 0x7FFFFFu) << 29)));
-  const double e = fma(neg_bits(m), y0, 1.0);
-  const double y = fma(y0, fma(e, e, e), y0);
-  return __longlong_as_double(__double_as_longlong(y) + ((long long)(1023 - E) << 52));
-}
-
-constexpr int DP = 16;  // panel width inside the block
-constexpr int DK = 48;  // longest product inside the block (the inverse's last block row)
-constexpr int NSIDE = DIAG_THREADS - 160;  // threads beside the chain's four warps and the inverse's
-static_assert(DIAG_THREADS == 512, "the deal of work to warps");
-
-struct DiagShared {
-  double S[NB][NB + 1];  // the matrix, then its factor
-  double V[NB][NB + 1];  // the inverse's blocks (T_ij until W_ij replaces it)
-  double col[DP][DP + 1];  // col[k][r]: entry (r, k) of the panel's block after all updates
-  double y[DP];            // 1 / col[k][k]
-  double lg[NB];
-  // fixed-point operand rows, limbs (high, low), and their powers of two: the panel's rows
-  // before and after B, W_pp, and the operands of the inverse's block rows
-  int2 F[NB][DP + 1], FL[NB][DP + 1], G[DP][DP + 1], P[DP][DK + 1], Q[DK][DK + 1];
-  int fe[NB], fle[NB], ge[DP], pe[DP], qe[DK];
-  int failed;
-};
-
-constexpr int DFB = 60;  // fraction bits of the fixed point
-
-// x = high 2^30 + low, |low| <= 2^29
-__device__ __forceinline__ int2 limbs(long long x) {
-  const int lo = ((int)x << 2) >> 2;
-  return make_int2((int)((x - lo) >> 30), lo);
-}
-// the four limb sums of 16 products
-__device__ __forceinline__ void limb_sums(const int2 *a, const int2 *b, long long &hh, long long &c0, long long &c1,
-                                          long long &ll) {
-  hh = c0 = c1 = ll = 0;
-#pragma unroll 8
-  for (int k = 0; k < DP; ++k) {
-    const int2 x = a[k], y = b[k];
-    hh += (long long)x.x * y.x;
-    c0 += (long long)x.x * y.y;
-    c1 += (long long)x.y * y.x;
-    ll += (long long)x.y * y.y;
-  }
-}
-// round(v 2^(60 - e)), |v| < 2^e
-__device__ __forceinline__ long long fixed_entry(double v, int e) {
-  const unsigned long long b = (unsigned long long)__double_as_longlong(v);
-  const int E = (int)((b >> 52) & 0x7FF);
-  const int sh = E - 1075 + DFB - e;  // m 2^sh
-  const unsigned long long m = (b & 0xFFFFFFFFFFFFFull) | (1ull << 52);
-  unsigned long long X = 0ull;
-  if (E != 0) {
-    if (sh >= 0) X = m << sh;
-    else if (sh > -60) X = (m + (1ull << (-sh - 1))) >> -sh;
-  }
-  return (b >> 63) ? -(long long)X : (long long)X;
-}
-
-// A row of 16 nb entries v (nb <= 3 to a lane), 16 lanes to a row, as limbs of
-// round(v 2^(60 - e)), 2^e four times the power of two above the row's largest entry (so
-// that |high| <= 2^28 and sums of 16 products stay below 2^63); returns e
-__device__ __noinline__ int limb_row(double v0, double v1, double v2, int nb, int2 *out) {
-  const int lane = threadIdx.x & 15;
-  auto field = [](double v) { return (int)(((unsigned long long)__double_as_longlong(v) >> 52) & 0x7FF); };
-  int mx = field(v0);
-  if (nb > 1) mx = max(mx, field(v1));
-  if (nb > 2) mx = max(mx, field(v2));
-#pragma unroll
-  for (int o = 8; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-  const int e = mx - 1020;
-  out[lane] = limbs(fixed_entry(v0, e));
-  if (nb > 1) out[lane + 16] = limbs(fixed_entry(v1, e));
-  if (nb > 2) out[lane + 32] = limbs(fixed_entry(v2, e));
-  return e;
-}
-
-// sum of n products (16, 32 or 48) of limb rows with powers of two ea + eb = e
-__device__ __noinline__ double limb_dot(const int2 *a, const int2 *b, int n, int e) {
-  long long hi = 0, lo = 0;  // hi + lo 2^-30
-  for (int k = 0; k < n; k += DP) {
-    long long hh, c0, c1, ll;
-    limb_sums(a + k, b + k, hh, c0, c1, ll);
-    const long long t = c0 + c1 + (ll >> 30);
-    hi += hh + (t >> 30);
-    lo += t & 0x3FFFFFFF;
-  }
-  hi += lo >> 30;
-  bool slow = false;
-  const int l = (int)(lo & 0x3FFFFFFF) >> 6;
-  const double v = fixed_to_double(hi, l, e - DFB + 38, 0u, slow);
-  return slow ? fixed_to_double_slow(hi, l, e - DFB + 38, 0u) : v;
-}
-
-// A(p), warps 0..3, one to a sub-partition (t: 0..127), with the inverse's warp 4: they
-// meet at barrier 2 before every pivot. Entry e of the lower triangle in columns, last
-// column first, belongs to thread e % 128: the entries that pivot k updates (at most 120)
-// are a prefix of the list. Entries 128.. lie in column 0, which no pivot updates.
-constexpr int DCH = 128;
-__device__ __forceinline__ void chain_sync() { asm volatile("bar.sync 2, %0;" ::"n"(DCH + 32) : "memory"); }
-
-__device__ __forceinline__ void diag_entry(int e, int &r, int &c) {
-  int u = (int)((sqrtf(8.0f * (float)e + 1.0f) - 1.0f) * 0.5f);
-  if (u * (u + 1) / 2 > e) --u;
-  if ((u + 1) * (u + 2) / 2 <= e) ++u;
-  c = DP - 1 - u;
-  r = c + e - u * (u + 1) / 2;
-}
-
-__device__ __forceinline__ void diag_panel_factor(DiagShared &sh, int c0, int64_t k0, int *status, int t) {
-  constexpr int NE = DP * (DP + 1) / 2;
-  int er, ec;
-  diag_entry(t, er, ec);
-  double a = sh.S[c0 + er][c0 + ec];
-  if (ec == 0) sh.col[0][er] = a;
-  if (t >= DCH - 8) sh.col[0][t + 16 - DCH] = sh.S[c0 + t + 16 - DCH][c0];  // entries 128..135: rows 8..15
-#pragma unroll 1
-  for (int k = 0; k < DP - 1; ++k) {
-    chain_sync();
-    const double *ck = sh.col[k];
-    const double d = ck[k];
-    double q = ck[er] * ck[ec];
-    if (t >= (DP - 1 - k) * (DP - k) / 2) q = 0.0;  // not an entry that pivot k updates
-    const double y = rcp_fast(d);
-    a = fma(-q, y, a);
-    if (ec == k + 1) sh.col[k + 1][er] = a;
-    if (t == 0) sh.y[k] = y;
-  }
-  chain_sync();
-  // the last pivot updates nothing; the first pivot that is not positive (sign bit or
-  // zero) or not finite fails the block (the later ones are void then)
-  const double d = sh.col[t & (DP - 1)][t & (DP - 1)];
-  const long long db = __double_as_longlong(d);
-  const unsigned bad = __ballot_sync(0xffffffffu, db <= 0ll || (db >> 52) >= 0x7FFll) & 0xFFFFu;
-  if (t == 0 && bad) {
-    sh.failed = 1;
-    atomicCAS(status, 0, (int)(k0 + c0 + __ffs(bad)));
-  }
-  // the factor: column c scaled by 1 / sqrt(d_c)
-  const double rp = rsqrt_fast(bad ? 1.0 : d);
-  const double r = __shfl_sync(0xffffffffu, rp, ec), r0 = __shfl_sync(0xffffffffu, rp, 0);
-  sh.S[c0 + er][c0 + ec] = a * r;
-  if (t >= DCH - 8) sh.S[c0 + t + 16 - DCH][c0] = sh.col[0][t + 16 - DCH] * r0;
-  static_assert(NE == DCH + 8, "entries to threads");
-}
-
-// A(p), warp 4: V = M^-1 for the unit lower M(i, k) = col(i, k) y_k, right-looking, one
-// pivot behind: step k sets V(i, k) = -M(i, k) and adds V(i, k) V(k, c) to every V(i, c),
-// i > k > c; then W_pp = diag(1 / sqrt(d)) V.
-__device__ __forceinline__ void diag_panel_inverse(DiagShared &sh, int c0) {
-  const int lane = threadIdx.x & 31;
-  double(*V)[NB + 1] = &sh.V[c0];
-  if (lane < DP) V[lane][c0 + lane] = 1.0;
-  chain_sync();
-#pragma unroll 1
-  for (int k = 0; k < DP - 1; ++k) {
-    chain_sync();
-    if (lane > k && lane < DP) V[lane][c0 + k] = -(sh.col[k][lane] * sh.y[k]);
-    __syncwarp();
-    // entries (i, c), k < i < 16, c < k: (15 - k) k of them
-    const int cnt = (DP - 1 - k) * k;
-    const float rk = __fdividef(1.0f, (float)k);
-    for (int e = lane; e < cnt; e += 32) {
-      const int q = (int)(((float)e + 0.5f) * rk), i = k + 1 + q, c = e - q * k;
-      V[i][c0 + c] = fma(V[i][c0 + k], V[k][c0 + c], V[i][c0 + c]);
-    }
-    __syncwarp();
-  }
-  const double dv = sh.col[lane & (DP - 1)][lane & (DP - 1)];
-  const double rp = rsqrt_fast(dv > 0.0 ? dv : 1.0);
-#pragma unroll
-  for (int t = 0; t < DP * DP / 32; ++t) {
-    const int i = 2 * t + (lane >> 4), c = lane & (DP - 1);
-    const double r = __shfl_sync(0xffffffffu, rp, i);
-    if (c <= i) V[i][c0 + c] = r * V[i][c0 + c];
-  }
-}
-
-// The inverse's block row i >= 1, W_ij = -W_ii sum_{k=j..i-1} L_ik W_kj, by nt threads (a
-// multiple of 32, t of them) that meet at `bar`
-template <typename Bar>
-__device__ __forceinline__ void diag_inverse_row(DiagShared &sh, int i, int t, int nt, Bar bar) {
-  const int l = t & 15, K = DP * i;
-  // P row r: row r of [L_i0 .. L_i,i-1]; Q row c: column c of W above the block row (zero
-  // above its diagonal)
-  for (int row = t >> 4; row < DP + K; row += nt >> 4) {
-    const bool left = row < DP;
-    const int c = row - DP;
-    double v[3];
-#pragma unroll
-    for (int b = 0; b < 3; ++b)
-      v[b] = b < i ? (left ? sh.S[K + row][DP * b + l] : sh.V[DP * b + l][c]) : 0.0;
-    const int e = limb_row(v[0], v[1], v[2], i, left ? sh.P[row] : sh.Q[c]);
-    if (l == 0) (left ? sh.pe[row] : sh.qe[c]) = e;
-  }
-  bar();
-  for (int idx = t; idx < DP * K; idx += nt) {
-    const int r = idx & 15, c = idx >> 4, q0 = c & ~15;
-    sh.V[K + r][c] = limb_dot(sh.P[r] + q0, sh.Q[c] + q0, K - q0, sh.pe[r] + sh.qe[c]);
-  }
-  bar();
-  for (int row = t >> 4; row < DP + K; row += nt >> 4) {
-    const bool left = row < DP;
-    const int c = row - DP;
-    const int e = limb_row(left ? sh.V[K + row][K + l] : sh.V[K + l][c], 0.0, 0.0, 1, left ? sh.P[row] : sh.Q[c]);
-    if (l == 0) (left ? sh.pe[row] : sh.qe[c]) = e;
-  }
-  bar();
-  for (int idx = t; idx < DP * K; idx += nt) {
-    const int r = idx & 15, c = idx >> 4;
-    sh.V[K + r][c] = neg_bits(limb_dot(sh.P[r], sh.Q[c], DP, sh.pe[r] + sh.qe[c]));
-  }
-}
-
-__global__ void __launch_bounds__(DIAG_THREADS) potrf_diag_kernel(double *__restrict__ A, int kb, int64_t lda,
-                                                         double *__restrict__ Winv,
-                                                         double *__restrict__ logdet_part,
-                                                         int *__restrict__ status, int64_t k0,
-                                                         int64_t sA, int64_t sW, int64_t sL) {
-  // batched: problem blockIdx.x (strides sA, sW, sL; status has one word per problem)
-  A += blockIdx.x * sA;
-  Winv += blockIdx.x * sW;
-  logdet_part += blockIdx.x * sL;
-  status += blockIdx.x;
-  extern __shared__ double diag_smem[];
-  DiagShared &sh = *reinterpret_cast<DiagShared *>(diag_smem);
-  if (*(volatile int *)status != 0) return;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, r16 = tid & 15;
-  // a partial block is padded with the identity to a multiple of 16; nb16 panels
-  const int nb16 = (kb + DP - 1) / DP, rows = DP * nb16;
-  for (int idx = tid; idx < NB * NB; idx += DIAG_THREADS) {
-    const int r = idx % NB, c = idx / NB;
-    sh.S[r][c] = (r < kb && c < kb && r >= c) ? A[r + c * lda] : (r == c ? 1.0 : 0.0);
-    sh.V[r][c] = 0.0;
-  }
-  if (tid == 0) sh.failed = 0;
-  __syncthreads();
-  for (int p = 0; p < nb16; ++p) {
-    const int c0 = DP * p, c1 = c0 + DP;
-    if (warp < 4) {
-      diag_panel_factor(sh, c0, k0, status, tid);
-    } else if (warp == 4) {
-      diag_panel_inverse(sh, c0);
-    } else {
-      const int t = tid - (DIAG_THREADS - NSIDE);
-      for (int r = c1 + (t >> 4); r < rows; r += NSIDE / 16) {
-        const int e = limb_row(sh.S[r][c0 + r16], 0.0, 0.0, 1, sh.F[r]);
-        if (r16 == 0) {
-          sh.fe[r] = e;
-          if (e == 2047 - 1020) {  // the row's own pivot would be NaN
-            sh.failed = 1;
-            atomicCAS(status, 0, (int)(k0 + r + 1));
-          }
-        }
-      }
-      if (p > 1)
-        diag_inverse_row(sh, p - 1, t, NSIDE, [] { asm volatile("bar.sync 1, %0;" ::"n"(NSIDE) : "memory"); });
-    }
-    __syncthreads();
-    if (sh.failed) return;
-    if (p + 1 == nb16) break;
-    // B(p): L_ip = A_ip W_pp^T, and its rows in fixed point
-    if (warp < 8) {
-      const int e = limb_row(sh.V[c0 + (tid >> 4)][c0 + r16], 0.0, 0.0, 1, sh.G[tid >> 4]);
-      if (r16 == 0) sh.ge[tid >> 4] = e;
-    }
-    __syncthreads();
-    for (int r = c1 + (tid >> 4); r < rows; r += DIAG_THREADS / 16) {
-      const double v = limb_dot(sh.F[r], sh.G[r16], DP, sh.fe[r] + sh.ge[r16]);
-      sh.S[r][c0 + r16] = v;
-      const int e = limb_row(v, 0.0, 0.0, 1, sh.FL[r]);
-      if (r16 == 0) sh.fle[r] = e;
-    }
-    __syncthreads();
-    // C(p): the trailing triangle, entries (r, c) with c1 <= c <= r
-    const int m = rows - c1;
-    for (int idx = tid; idx < m * (m + 1) / 2; idx += DIAG_THREADS) {
-      int r = (int)((sqrtf(8.0f * (float)idx + 1.0f) - 1.0f) * 0.5f);
-      if (r * (r + 1) / 2 > idx) --r;
-      if ((r + 1) * (r + 2) / 2 <= idx) ++r;
-      const int c = c1 + idx - r * (r + 1) / 2;
-      r += c1;
-      sh.S[r][c] -= limb_dot(sh.FL[r], sh.FL[c], DP, sh.fle[r] + sh.fle[c]);
-    }
-    __syncthreads();
-  }
-  // the logarithms of the diagonal beside the inverse's last block row
-  if (warp < 2) {
-    const int r = 32 * warp + lane;
-    sh.lg[r] = r < kb ? log(sh.S[r][r]) : 0.0;
-  } else if (nb16 > 1) {
-    diag_inverse_row(sh, nb16 - 1, tid - 64, DIAG_THREADS - 64,
-                     [] { asm volatile("bar.sync 1, %0;" ::"n"(DIAG_THREADS - 64) : "memory"); });
-  }
-  __syncthreads();
-  for (int idx = tid; idx < NB * NB; idx += DIAG_THREADS) {
-    const int r = idx % NB, c = idx / NB;
-    if (r < kb && c <= r) A[r + c * lda] = sh.S[r][c];
-    Winv[r + c * NB] = (r < kb && c <= r) ? sh.V[r][c] : 0.0;
-  }
-  if (warp == 0) {  // log det in a fixed order
-    double l = sh.lg[lane] + sh.lg[lane + 32];
-    for (int o = 16; o > 0; o >>= 1) l += __shfl_down_sync(0xffffffffu, l, o);
-    if (lane == 0) *logdet_part = l;
-  }
-}
-
-// The same block on the FP64 pipe alone, column by column: the kernel of the mixed
-// precision. There the trailing updates cut their operands to 32 (batched: 40) bits, so
-// any other rounding of an entry here draws the whole truncation of the factor anew, and
-// predicted variances, whose error is 2e-8 of their scale, move by up to 2e-9 of it: with
-// this kernel mixed results stay the same to the bit. It costs 65 us a block where the
-// kernel above costs 51.
-// On this part the FP64 pipe retires about 2 lane operations per clock per SM,
-// and a warp instruction occupies it whether 1 or 32 lanes are active, so the
-// kernel issues as few FP64 warp instructions as it can, each with all lanes on
-// distinct entries, and runs the factor and the inverse in one loop with one
-// barrier per column:
-//  - factor, right-looking: warp 0 takes the pivots one column ahead (column
-//    j+1 gets its update from column j, then its inverse square root,
-//    rsqrt_fast) while the update warps apply the rank-1 update of column j to
-//    the trailing triangle c >= j+2. The trailing triangle's entries are
-//    numbered by column, last column first, so that step j's entries are the
-//    first (kb-2-j)(kb-1-j)/2 of one fixed list. The warps that share warp 0's
-//    sub-partition take no update work; the other twelve (three per
-//    sub-partition, enough to cover the FP64 latency) share it evenly.
-//  - inverse: W = L^-1 = D^-1 V with D = diag(L) and V the unit lower triangular
-//    inverse of the column-scaled factor L D^-1:
-//      V(i, c) = -sum_{k=c..i-1} (L(i, k) / L(k, k)) V(k, c),  V(c, c) = 1.
-//    The k = c term is written by the pivot of column c (V(i, c) starts as
-//    -L(i, c) / L(c, c)); the terms k > c are added right-looking, step k adding
-//    V(i, k) V(k, c) to every (i > k, c < k) while V(i, k) still holds only its
-//    first term. Step k needs column k of L and rows <= k of V final, so it runs
-//    beside the factor's step k + 1 in the same loop iteration. Every inverse
-//    entry costs one FMA; the row scaling by 1 / L(i, i) happens once, on the
-//    way out.
-//  - log L_jj summed in a fixed tree order.
-__device__ __forceinline__ int div_small(int e, int d, int magic) {
-  // e / d for e < 4096, 1 <= d <= 64, magic = ceil(2^20 / d): exact on that range
-  return (int)(((unsigned)e * (unsigned)magic) >> 20);
-}
-
-__global__ void __launch_bounds__(DIAG_THREADS) potrf_diag_rank1_kernel(double *__restrict__ A, int kb, int64_t lda,
-                                                         double *__restrict__ Winv,
-                                                         double *__restrict__ logdet_part,
-                                                         int *__restrict__ status, int64_t k0,
-                                                         int64_t sA, int64_t sW, int64_t sL) {
-  // batched: problem blockIdx.x (strides sA, sW, sL; status has one word per problem)
-  A += blockIdx.x * sA;
-  Winv += blockIdx.x * sW;
-  logdet_part += blockIdx.x * sL;
-  status += blockIdx.x;
-  __shared__ double S[NB][NB + 1];
-  __shared__ double V[NB][NB + 1];
-  __shared__ double rdiag[NB];
-  __shared__ double lg[NB];
-  __shared__ unsigned short pairs[NB * (NB + 1) / 2];  // (r | c << 8), column-major from the last column
-  __shared__ int failed;
-  if (*(volatile int *)status != 0) return;
-  const int tid = threadIdx.x;
-  const int lane = tid & 31, warp = tid >> 5;
-  for (int idx = tid; idx < NB * NB; idx += DIAG_THREADS) {
-    const int r = idx % NB, c = idx / NB;
-    // held negated until its column is pivoted (see the update loop)
-    S[r][c] = (r < kb && c < kb && r >= c) ? neg_bits(A[r + c * lda]) : 0.0;
-    V[r][c] = 0.0;
-  }
-  // entry e of the kb x kb triangle: u = kb - 1 - c is the largest u with
-  // u (u + 1) / 2 <= e; r = c + e - u (u + 1) / 2 (a partial block lists only its
-  // own entries)
-  for (int e = tid; e < kb * (kb + 1) / 2; e += DIAG_THREADS) {
-    int u = (int)((sqrtf(8.0f * (float)e + 1.0f) - 1.0f) * 0.5f);
-    while (u * (u + 1) / 2 > e) --u;
-    while ((u + 1) * (u + 2) / 2 <= e) ++u;
-    const int c = kb - 1 - u, r = c + (e - u * (u + 1) / 2);
-    pairs[e] = (unsigned short)(r | (c << 8));
-  }
-  if (tid == 0) failed = 0;
-  __syncthreads();
-  // Warp 0 keeps the current scaled column in registers: lane l owns rows l and
-  // l + 32, and lreg[u] holds L(l + 32 u, j) once column j is pivoted. Rows below
-  // 32 drop out after column 31, so their FP64 work is skipped from then on (a
-  // warp instruction costs the same with one lane or 32).
-  double lreg[2] = {0.0, 0.0};
-  // pivot of column j by warp 0 from t[u] = -S(l + 32 u, j) after all updates:
-  // L_jj, the scaled column below it (stored positive, and kept in lreg) and the
-  // first term of column j of V
-  auto pivot = [&](int j, const double (&t)[2]) {
-    const double dj = neg_bits(__shfl_sync(0xffffffffu, j < 32 ? t[0] : t[1], j & 31));
-    // not positive (sign bit or zero) or not finite, tested on the bits
-    const long long djb = __double_as_longlong(dj);
-    if (djb <= 0ll || (djb >> 52) >= 0x7FFll) {
-      if (lane == 0) {
-        failed = 1;
-        atomicCAS(status, 0, (int)(k0 + j + 1));
-      }
-      return;
-    }
-    const double rp = rsqrt_fast(dj);
-#pragma unroll
-    for (int u = 0; u < 2; ++u) {
-      if (u == 1 || j < 31) {
-        const int r = lane + 32 * u;
-        if (r > j && r < kb) {
-          const double l = -(t[u] * rp);
-          S[r][j] = l;
-          V[r][j] = -(l * rp);
-          lreg[u] = l;
-        }
-      }
-    }
-    if (lane == (j & 31)) {
-      S[j][j] = dj * rp;
-      rdiag[j] = rp;
-    }
-  };
-  if (warp == 0) {
-    double t0[2];
-#pragma unroll
-    for (int u = 0; u < 2; ++u) t0[u] = (lane + 32 * u < kb) ? S[lane + 32 * u][0] : 0.0;
-    pivot(0, t0);
-  }
-  __syncthreads();
-  if (failed) return;
-  // update workers: every warp off sub-partition 0 (warps 4, 8, 12 share warp 0's)
-  constexpr int NUPD = DIAG_THREADS / 32 - DIAG_THREADS / 128;  // 12 update warps
-  const int uw = warp - 1 - (warp >> 2);
-  const int ut = uw * 32 + lane;
-  for (int j = 0; j < kb; ++j) {
-    if (warp == 0) {
-      if (j + 1 < kb) {
-        // column j + 1 takes its last update, from column j, then its pivot
-        const double l = __shfl_sync(0xffffffffu, (j + 1) < 32 ? lreg[0] : lreg[1], (j + 1) & 31);
-        double t[2] = {0.0, 0.0};
-#pragma unroll
-        for (int u = 0; u < 2; ++u) {
-          if (u == 1 || j < 31) {
-            const int r = lane + 32 * u;
-            if (r > j && r < kb) t[u] = fma(lreg[u], l, S[r][j + 1]);
-          }
-        }
-        pivot(j + 1, t);
-      }
-    } else if ((warp & 3) != 0) {
-      // factor step j: entries (r, c), c >= j + 2, of the fixed list; inverse step
-      // k = j - 1: entries (i, c), k < i < kb, c < k, row-major by i. Both are
-      // dst += a b with a, b >= sign-free operands (the trailing matrix is held
-      // negated), so that each entry is exactly one FP64 instruction.
-      const int cf = j < kb - 2 ? (kb - 2 - j) * (kb - 1 - j) / 2 : 0;
-      const int k = j - 1;
-      const int ci = k >= 1 ? (kb - 1 - k) * k : 0;
-      const int magic = k >= 1 ? ((1 << 20) + k - 1) / k : 0;
-      for (int e = ut; e < cf + ci; e += NUPD * 32) {
-        const double *pa, *pb;
-        double *dst;
-        if (e < cf) {
-          const unsigned short pc = pairs[e];
-          const int r = pc & 0xFF, c = pc >> 8;
-          dst = &S[r][c];
-          pa = &S[r][j];
-          pb = &S[c][j];
-        } else {
-          const int e2 = e - cf;
-          const int q = div_small(e2, k, magic);
-          const int c = e2 - q * k, i = k + 1 + q;
-          dst = &V[i][c];
-          pa = &V[i][k];
-          pb = &V[k][c];
-        }
-        *dst = fma(*pa, *pb, *dst);
-      }
-    }
-    __syncthreads();
-    if (failed) return;
-  }
-  // write the factor back (lower part of the block)
-  for (int idx = tid; idx < kb * kb; idx += DIAG_THREADS) {
-    const int r = idx % kb, c = idx / kb;
-    if (r >= c) A[r + c * lda] = S[r][c];
-  }
-  if (tid < NB) lg[tid] = tid < kb ? log(S[tid][tid]) : 0.0;
-  __syncthreads();
-  // W = D^-1 V
-  for (int idx = tid; idx < NB * NB; idx += DIAG_THREADS) {
-    const int r = idx % NB, c = idx / NB;
-    double wv = 0.0;
-    if (r < kb && c <= r) wv = (r == c) ? rdiag[r] : rdiag[r] * V[r][c];
-    Winv[r + c * NB] = wv;
-  }
-  for (int st = NB / 2; st > 0; st >>= 1) {
-    if (tid < st) lg[tid] += lg[tid + st];
-    __syncthreads();
-  }
-  if (tid == 0) *logdet_part = lg[0];
-}
-
-void potrf_diag(cudaStream_t s, double *A, int kb, int64_t lda, double *Winv, double *logdet_part, int *status,
-                int64_t k0, int64_t sA, int64_t sW, int64_t sL, int64_t batch, bool rank1) {
-  KTScope kts(GPGP_KPROF_POTRF_DIAG, s, 2.0 * kb * kb * kb / 3 * (double)batch);
-  if (rank1) {
-    potrf_diag_rank1_kernel<<<(unsigned)batch, DIAG_THREADS, 0, s>>>(A, kb, lda, Winv, logdet_part, status, k0, sA,
-                                                                     sW, sL);
-    GPGP_CHECK_LAUNCH();
-    return;
-  }
-  static PerDevice attr;
-  per_device(attr, [] {
-    GPGP_CUDA(cudaFuncSetAttribute(potrf_diag_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)sizeof(DiagShared)));
-    return 1;
-  });
-  potrf_diag_kernel<<<(unsigned)batch, DIAG_THREADS, sizeof(DiagShared), s>>>(A, kb, lda, Winv, logdet_part, status,
-                                                                              k0, sA, sW, sL);
-  GPGP_CHECK_LAUNCH();
 }
 
 // ---------------------------------------------------------------------------

@@ -17,17 +17,27 @@ static __device__ __noinline__ double rsqrt_slow(double x) { return 1.0 / sqrt(x
 //   (1 - e)^(-1/2) = 1 + e/2 + 3e^2/8 + O(e^3),  e = 1 - x y0^2,
 // four dependent FP64 operations whose neglected terms are ~2^-66. Arguments
 // outside the float range take sqrt and division out of line.
-__device__ __forceinline__ double rsqrt_fast(double x) {
+__device__ __forceinline__ bool rsqrt_in_range(double x) {
+  const int E = (int)((unsigned long long)__double_as_longlong(x) >> 52);
+  return E >= 1023 - 125 && E <= 1023 + 125;
+}
+// rsqrt_fast in two steps, for an x in range: the FP32 seed and its refinement (so that
+// other FP64 instructions can run while the seed is on its way)
+__device__ __forceinline__ double rsqrt_seed(double x) {
   const unsigned long long b = (unsigned long long)__double_as_longlong(x);
   const int E = (int)(b >> 52);
-  if (E < 1023 - 125 || E > 1023 + 125) return rsqrt_slow(x);
   const float xf = __uint_as_float(((uint32_t)(E - 1023 + 127) << 23) | (uint32_t)((b >> 29) & 0x7FFFFFu));
   const uint32_t yb = __float_as_uint(rsqrtf(xf));
-  const double y0 = __longlong_as_double(
-      (long long)(((unsigned long long)(((yb >> 23) & 0xFFu) - 127u + 1023u) << 52) |
-                  ((unsigned long long)(yb & 0x7FFFFFu) << 29)));
+  return __longlong_as_double((long long)(((unsigned long long)(((yb >> 23) & 0xFFu) - 127u + 1023u) << 52) |
+                                          ((unsigned long long)(yb & 0x7FFFFFu) << 29)));
+}
+__device__ __forceinline__ double rsqrt_refine(double x, double y0) {
   const double e = fma(-(x * y0), y0, 1.0);
   return fma(y0 * e, fma(e, 0.375, 0.5), y0);
+}
+__device__ __forceinline__ double rsqrt_fast(double x) {
+  if (!rsqrt_in_range(x)) return rsqrt_slow(x);
+  return rsqrt_refine(x, rsqrt_seed(x));
 }
 
 static __device__ __noinline__ double sqrt_slow(double x) { return sqrt(x); }

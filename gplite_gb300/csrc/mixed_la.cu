@@ -58,7 +58,7 @@ void factor_panel(cudaStream_t x, cudaStream_t y, cudaStream_t z, const SideStre
     const int jb = (int)std::min<int64_t>(NB, pend - j0);
     const int64_t blk = j0 / NB;
     double *Wb = Winv + blk * NB * NB;
-    potrf_diag(x, A + j0 + j0 * lda, jb, lda, Wb, logdet_part + blk, status, j0, 0, 0, 0, 1, S != OZ_FP64);
+    potrf_diag(x, A + j0 + j0 * lda, jb, lda, Wb, logdet_part + blk, status, j0, 0, 0, 0, 1);
     const int64_t mp = pend - (j0 + jb);  // panel rows below the block
     double *Ln = A + (j0 + NB) + j0 * lda;
     if (mp > 0) {
