@@ -182,26 +182,63 @@ static void gemm64_dispatch(cudaStream_t s, bool ta, bool tb, dim3 grid, int64_t
 
 // Small products (few 64 x 64 tiles, short K): one thread per element of C, so
 // that the FP64 work spreads over many SMs instead of a few tile CTAs (an FP64
-// warp instruction holds its sub-partition for 64 cycles on this part).
-__global__ void gemm64_small_kernel(int64_t M, int64_t N, int64_t K, double alpha, const double *__restrict__ A,
-                                    int64_t lda, int ta, const double *__restrict__ B, int64_t ldb, int tb,
-                                    double beta, double *__restrict__ C, int64_t ldc, int lower) {
-  const int64_t i = (int64_t)blockIdx.x * 32 + (threadIdx.x & 31);
-  const int64_t j = (int64_t)blockIdx.y * 8 + (threadIdx.x >> 5);
-  if (i >= M || j >= N || (lower && j > i)) return;
+// warp instruction holds its sub-partition for 64 cycles on this part). A CTA is a warp
+// per sub-partition, 32 x 4 elements, whose operands come 64 K at a time through shared
+// memory: all of a chunk's loads are in flight at once (a load for each term from the L2
+// took 24 us for 256 x 64 x 64, this 7).
+constexpr int SG_N = 4, SG_K = 64;
+
+__global__ void __launch_bounds__(128) gemm64_small_kernel(int64_t M, int64_t N, int64_t K, double alpha,
+                                                           const double *__restrict__ A, int64_t lda, int ta,
+                                                           const double *__restrict__ B, int64_t ldb, int tb,
+                                                           double beta, double *__restrict__ C, int64_t ldc,
+                                                           int lower) {
+  __shared__ double As[SG_K][33], Bs[SG_K][SG_N + 1];
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  const int64_t i0 = (int64_t)blockIdx.x * 32, j0 = (int64_t)blockIdx.y * SG_N;
+  if (lower && j0 > i0 + 31) return;
+  const int64_t i = i0 + lane, j = j0 + w;
+  const bool mine = i < M && j < N && !(lower && j > i);
+  const double c = mine && beta != 0.0 ? C[i + j * ldc] : 0.0;
   double s0 = 0.0, s1 = 0.0;
-  int64_t k = 0;
-  for (; k + 1 < K; k += 2) {
-    const double a0 = ta ? A[k + i * lda] : A[i + k * lda];
-    const double a1 = ta ? A[k + 1 + i * lda] : A[i + (k + 1) * lda];
-    const double b0 = tb ? B[j + k * ldb] : B[k + j * ldb];
-    const double b1 = tb ? B[j + (k + 1) * ldb] : B[k + 1 + j * ldb];
-    s0 = fma(a0, b0, s0);
-    s1 = fma(a1, b1, s1);
+  for (int64_t k0 = 0; k0 < K; k0 += SG_K) {
+    const int kn = (int)(K - k0 < SG_K ? K - k0 : SG_K);
+    double ra[32 * SG_K / 128], rb[SG_N * SG_K / 128];
+#pragma unroll
+    for (int t = 0; t < 32 * SG_K / 128; ++t) {
+      const int idx = tid + 128 * t, r = ta ? idx / SG_K : idx & 31, k = ta ? idx % SG_K : idx >> 5;
+      ra[t] = k < kn && i0 + r < M ? A[ta ? k0 + k + (i0 + r) * lda : i0 + r + (k0 + k) * lda] : 0.0;
+    }
+#pragma unroll
+    for (int t = 0; t < SG_N * SG_K / 128; ++t) {
+      const int idx = tid + 128 * t, r = tb ? idx & (SG_N - 1) : idx / SG_K, k = tb ? idx / SG_N : idx % SG_K;
+      rb[t] = k < kn && j0 + r < N ? B[tb ? j0 + r + (k0 + k) * ldb : k0 + k + (j0 + r) * ldb] : 0.0;
+    }
+    if (k0 > 0) __syncthreads();
+#pragma unroll
+    for (int t = 0; t < 32 * SG_K / 128; ++t) {
+      const int idx = tid + 128 * t;
+      As[ta ? idx % SG_K : idx >> 5][ta ? idx / SG_K : idx & 31] = ra[t];
+    }
+#pragma unroll
+    for (int t = 0; t < SG_N * SG_K / 128; ++t) {
+      const int idx = tid + 128 * t;
+      Bs[tb ? idx / SG_N : idx % SG_K][tb ? idx & (SG_N - 1) : idx / SG_K] = rb[t];
+    }
+    __syncthreads();
+    if (mine) {
+      int k = 0;
+#pragma unroll 4
+      for (; k + 1 < kn; k += 2) {
+        s0 = fma(As[k][lane], Bs[k][w], s0);
+        s1 = fma(As[k + 1][lane], Bs[k + 1][w], s1);
+      }
+      if (k < kn) s0 = fma(As[k][lane], Bs[k][w], s0);
+    }
   }
-  if (k < K) s0 = fma(ta ? A[k + i * lda] : A[i + k * lda], tb ? B[j + k * ldb] : B[k + j * ldb], s0);
+  if (!mine) return;
   const double v = alpha * (s0 + s1);
-  C[i + j * ldc] = (beta == 0.0) ? v : v + beta * C[i + j * ldc];
+  C[i + j * ldc] = (beta == 0.0) ? v : v + beta * c;
 }
 
 void gemm64_batched(cudaStream_t s, bool ta, bool tb, int64_t M, int64_t N, int64_t K, double alpha,
@@ -236,8 +273,8 @@ void gemm64(cudaStream_t s, bool ta, bool tb, int64_t M, int64_t N, int64_t K, d
   // (the batched entry keeps the tile kernel for every batch size, so that a
   // problem's result does not depend on how many others share its launch)
   if (M > 0 && N > 0 && tri_mode == 0 && K <= 256 && ((M + GBM - 1) / GBM) * ((N + GBN - 1) / GBN) < 152) {
-    dim3 g((unsigned)((M + 31) / 32), (unsigned)((N + 7) / 8));
-    gemm64_small_kernel<<<g, 256, 0, s>>>(M, N, K, alpha, A, lda, ta ? 1 : 0, B, ldb, tb ? 1 : 0, beta, C, ldc,
+    dim3 g((unsigned)((M + 31) / 32), (unsigned)((N + SG_N - 1) / SG_N));
+    gemm64_small_kernel<<<g, 128, 0, s>>>(M, N, K, alpha, A, lda, ta ? 1 : 0, B, ldb, tb ? 1 : 0, beta, C, ldc,
                                           lower_only ? 1 : 0);
     GPGP_CHECK_LAUNCH();
     return;

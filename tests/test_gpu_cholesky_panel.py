@@ -29,3 +29,23 @@ def test_panel_edges(n, precision, rtol):
     p, q = G.gp_pred(g, xt, var=True), R.gp_pred(o, xt, var=True)
     assert np.abs(p["mean"] - q["mean"]).max() <= rtol
     assert np.abs(p["var"] - q["var"]).max() <= rtol
+
+
+@pytest.mark.parametrize("n,m", [(31, 1), (33, 5), (65, 64), (97, 3), (130, 63), (193, 65), (257, 129), (320, 7)])
+def test_small_product_edges(n, m):
+    """Products of few elements with K up to 256 (32 x 4 elements to a CTA, K in chunks of
+    64): the trailing updates of a fit, FITC's and the predictions' products at sizes around
+    those. Condition number below 1e4 as above: 1e-10."""
+    rng = np.random.default_rng(n + m)
+    x = rng.uniform(-1, 1, (n, 2))
+    y = np.sin(3 * x[:, 0]) + 0.2 * rng.standard_normal(n)
+    xt = rng.uniform(-1, 1, (m, 2))
+    z = x[rng.choice(n, min(n - 1, m + 8), replace=False)]
+    for gm, om in ((None, None), (G.method_fitc(inducing=z), R.method_fitc(z))):
+        g = G.gp_fit(G.gp_init(G.cf_matern32(lscale=0.3), G.lik_gaussian(sigma=0.2), *([gm] if gm else [])), x, y)
+        o = R.gp_fit(R.gp_init([R.cf("matern32", lscale=0.3, magn=1.0)], R.lik("gaussian", sigma=0.2),
+                               *([om] if om else [])), x, y)
+        assert abs(g.fit["log_evidence"] - o.fit["log_evidence"]) <= 1e-10 * n
+        p, q = G.gp_pred(g, xt, var=True), R.gp_pred(o, xt, var=True)
+        assert np.abs(p["mean"] - q["mean"]).max() <= 1e-10
+        assert np.abs(p["var"] - q["var"]).max() <= 1e-10
