@@ -74,10 +74,8 @@ __device__ __forceinline__ void send16(uint32_t dst, double2 v, uint32_t bar) {
                : "memory");
 }
 __device__ __forceinline__ void cluster_sync() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
-  asm volatile("mbarrier.arrive.release.cta.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+  cluster_arrive();
+  cluster_wait();
 }
 // Bounded wait for phase 0 of a barrier that another CTA completes (a second or so)
 __device__ __forceinline__ bool wait_peer(uint32_t bar) {
