@@ -260,7 +260,7 @@ void trsv_lower(cudaStream_t s, const double *L, int64_t n, int64_t lda, const d
                 double *b, double *x, const int *status);    // x = L^-1 b
 void trsv_lower_t(cudaStream_t s, const double *L, int64_t n, int64_t lda, const double *Winv,
                   double *b, double *x, const int *status);  // x = L^-T b
-// Single-launch versions (blocks ordered by device flags, bounded waits): sync
+// Single-launch versions (x's entries are their own flags, bounded waits): sync
 // holds n / 64 + 2 unsigned words of device scratch; err is set when a wait runs
 // out. b is not modified; x must not alias b.
 void trsv_flow(cudaStream_t s, const double *L, int64_t n, int64_t lda, const double *Winv,
