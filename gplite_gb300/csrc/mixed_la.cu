@@ -31,8 +31,13 @@ constexpr int64_t NBO = GPGP_NBO;  // outer panel width of the Cholesky (a build
 static_assert(NBO % NB == 0, "an outer panel is whole blocks wherever rows lie below it");
 // Lookahead: a trailing update of at least LOOK_MIN_ROWS rows leaves LOOK_PANEL_SMS
 // SMs to the next panel's factorisation, whose GEMMs are capped to them.
+// The panel's rows below (panel_block) take most of that share, and the chain's clusters
+// need four free SMs of one GPC: mixed step n = 16384 with 20 / 32 / 48 / 56 / 72 SMs left:
+// 92.9 / 82.6 / 78.6 / 77.9 / 80.6 ms, mixed Laplace n = 8192 86.9 / 81.5 / 80.6 / 78.6 /
+// 80.6, FP64 step n = 8192 33.2 / 31.8 / 31.7 / 30.8 / 31.7. From 3072 rows on: mixed
+// Laplace 85.1 (32 SMs).
 constexpr int64_t LOOK_MIN_ROWS = 6144;
-constexpr int LOOK_PANEL_SMS = 32;
+constexpr int LOOK_PANEL_SMS = 56;
 
 // The 64-wide blocks of the outer panel [k0, k0 + kbo). What the next diagonal block
 // waits for is kept apart from the rest:
