@@ -41,13 +41,13 @@ LSCALE, MAGN, CMAGN = 0.7, 1.0, 1.0
 NPRED = 8192
 
 # DRAM traffic of the sliced GEMM per launch of the n = 16384 mixed step: the mean of
-# dram__bytes_read.sum + dram__bytes_write.sum over the first 579 oz_gemm launches of
+# dram__bytes_read.sum + dram__bytes_write.sum over the 363 GEMM and panel launches of
 # one step, one-pass ncu capture (the profile summaries give the command and the
 # per-shape figures: the trailing updates move their FP64 C block in and out once,
 # e.g. 1.9 GB for a 16000 x 16000 lower triangle).
-OZ_TRAFFIC_PER_LAUNCH = {16384: 8.191e7}
+OZ_TRAFFIC_PER_LAUNCH = {16384: 9.448e7}
 OZ_TRAFFIC_SOURCE = ("ncu --metrics dram__bytes_read.sum,dram__bytes_write.sum,gpu__time_duration.sum "
-                     "-k regex:oz_gemm (1 pass), mean over the 579 launches of one n = 16384 step")
+                     "-k 'regex:oz_gemm_kernel|panel_block' (1 pass), mean over the 363 launches of one n = 16384 step")
 
 
 def theta_sequence(k):
@@ -493,18 +493,19 @@ def run_gpu(args):
             potrf_tf = (n ** 3 / 3) / (r["potrf_ms"] / max(r["potrf_calls"], 1) / 1e3) / 1e12
             if p == "fp64":
                 fp64 = fp64_peak_gflops(torch) / 1e3
-                k = r["kernels"]["gemm64"]
+                k = r["kernels"]["oz_gemm"]
                 ach = alg / (k["ms"] / 1e3) / 1e12 if k["ms"] > 0 else None
                 exe = k["flops"] / (k["ms"] / 1e3) / 1e12 if k["ms"] > 0 else None
-                return {"bound": "fp64", "kernel": "gemm64_kernel (FP64 trailing updates of potrf, "
-                                                   "trtri/lauum products)",
-                        "achieved": ach, "peak": fp64, "unit": "TFLOP/s", "frac": ach / fp64 if ach else None,
+                bf = peaks.get("bf16_tflops_sustained", 1700.0)
+                return {"bound": "tensor", "kernel": "oz_gemm_kernel<8> (63-bit fixed-point products of potrf, "
+                                                     "trtri, lauum on the tensor cores)",
+                        "achieved": ach, "peak": bf, "unit": "TFLOP/s", "frac": ach / bf if ach else None,
                         "algorithmic_flops_per_step": alg, "launches": k["launches"],
                         "avg_launch_ms": k["ms"] / max(k["launches"], 1),
-                        "peak_source": "cuBLAS DGEMM 8192^3 measured in this run (FP64 is not in "
-                                       "MEASURED_PEAKS.json)",
-                        "executed_tile_flops": {"achieved": exe, "frac": exe / fp64 if exe else None},
-                        "potrf_fp64_tflops": potrf_tf, "traffic": None}
+                        "peak_source": "of measured: MEASURED_PEAKS.json bf16_tflops_sustained",
+                        "executed_slice_products": {"achieved": exe, "frac": exe / bf if exe else None,
+                                                    "note": "BF16 MMA flops, 36 per FP64-equivalent product"},
+                        "dgemm_tflops": fp64, "potrf_fp64_tflops": potrf_tf, "traffic": None}
             k = r["kernels"]["oz_gemm"]
             bf = peaks.get("bf16_tflops_sustained", 1700.0)
             ach = alg / (k["ms"] / 1e3) / 1e12 if k["ms"] > 0 else None

@@ -1,4 +1,5 @@
-"""The diagonal-block kernel (factor and inverse of up to 64 x 64, in 16-wide panels)."""
+"""The diagonal-block kernel (factor and inverse of up to 64 x 64, in segments of 4
+columns, 16 to a CTA)."""
 import numpy as np
 import pytest
 
