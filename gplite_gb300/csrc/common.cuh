@@ -303,9 +303,9 @@ void getrs(cudaStream_t s, const double *LU, int64_t n, int64_t lda, const int *
 constexpr int OZ_FP64 = 8;
 // Size from which the FP64 path's factorisation, inverses and B^-1 take the tensor cores
 // with 8 slices. Optimiser step / fit and predict / EP fit in ms, FP64 pipe against slices:
-// n = 800: 2.92 / 2.16 / 19.1 against 2.28 / 2.28 / 19.9; n = 900: 3.58 / 2.72 / 21.0
-// against 2.38 / 2.54 / 18.6 (n <= 768 has one outer panel's lookahead too few: 2.76 /
-// 2.03 / 18.2 against 2.61 / 2.65 / 22.7 at 760).
+// n = 800: 2.69 / 1.96 / 17.3 against 2.14 / 2.15 / 18.8; 850: 3.11 / 2.22 / 19.3 against
+// 2.29 / 2.25 / 20.0; 900: 3.32 / 2.48 / 19.1 against 2.22 / 2.37 / 17.5; 1050: 4.08 / 3.08 /
+// 26.1 against 2.34 / 2.70 / 20.3.
 #ifndef GPGP_SLICED_MIN
 #define GPGP_SLICED_MIN 896
 #endif
