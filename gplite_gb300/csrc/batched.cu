@@ -7,10 +7,10 @@
 // part of B = I + K / sigma^2 is the identity, so it adds nothing to the factor,
 // the solves or the log-determinant, and every problem of a bucket can run the
 // blocked algorithms of dense.cu / mixed.cu in lockstep (problem index on a grid
-// axis). Each bucket's contractions run either on the FP64 pipe or through the
-// BF16-sliced tcgen05 GEMM; a small autotuner times both on the first run of a
-// mixed-precision plan and keeps the faster per bucket. The whole sequence is then
-// captured once into a CUDA graph and replayed.
+// axis). Each bucket's contractions run either on the FP64 pipe (FP64 plans) or
+// through the BF16-sliced tcgen05 GEMM (mixed-precision plans, with the outer panel
+// that plan_variant gives). The whole sequence is then captured once into a CUDA
+// graph and replayed.
 #include <math.h>
 
 #include <algorithm>
@@ -39,7 +39,7 @@ struct Bucket {
   void *sa = nullptr, *sb = nullptr;
   OzSplit SA, SB;
   int variant = 0;  // 0: FP64 pipe; sliced tensor cores with 1: 64-wide, 2: 256-wide outer panels
-  double best_ms = 0.0;  // the autotuner's time of the chosen variant
+  double run_ms = 0.0;  // measured time of one run (mixed-precision plans)
   ~Bucket() {
     if (sa) cudaFreeAsync(sa, X.s);
     if (sb) cudaFreeAsync(sb, X.s);
@@ -423,7 +423,7 @@ struct gpgp_batch {
   IBuf err;
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
-  double tune_ms[3] = {0, 0, 0};  // autotuning time per variant
+  double tune_ms[3] = {0, 0, 0};  // measured time of the buckets per variant
   int64_t graph_kernels = 0;  // kernel nodes of the captured graph
   // streams and events of the graph's concurrent bucket lanes (capture only)
   cudaStream_t lanes[4] = {nullptr, nullptr, nullptr, nullptr};
@@ -451,6 +451,24 @@ constexpr int kRefine = 2;
 
 size_t split_stride_bytes(int64_t rows, int64_t K) {
   return (oz_split_bytes(rows, K, kSlices) + 1023) / 1024 * 1024;
+}
+
+// The variant of a bucket of `count` problems of nb = 64 T rows. It follows from the
+// sizes alone, never from a timing: above T = 4 variants 1 and 2 round differently (K = 64
+// or 256 to a product), so the same plan must take the same one every time. Up to T = 4
+// they compute the same. The wider panel rewrites the trailing matrix less often but
+// splits its operand once more; time of variant 2 over variant 1, at the counts on either
+// side of the line, with the kernels the line was drawn for (in brackets with the current
+// ones, whose cheaper updates favour variant 1 a little longer):
+//   T = 5:  64 problems 1.010 (1.005), 128 0.997 (0.999), 256 0.993 (0.998)
+//   T = 8:  16 problems 0.999 (1.006), 32 0.992 (1.000), 128 0.972 (0.987)
+//   T = 12:  4 problems 1.000 (1.005), 8 0.998 (1.008), 64 0.958 (0.978)
+//   T = 16:  2 problems 1.003 (1.007), 4 0.996 (1.006), 16 0.970 (0.990), 256 0.909 (0.948)
+// The FP64 pipe is never ahead (1.02 to 4.4 times variant 1's time over T = 1 .. 16).
+int plan_variant(int32_t precision, int64_t nb, int64_t count) {
+  if (precision != GPGP_PREC_MIXED) return 0;
+  const int64_t T = nb / NB;
+  return T > 4 && count * (T - 3) * (T - 3) >= 506 ? 2 : 1;
 }
 
 // one bucket's pipeline, enqueued on stream st (no allocation, no sync)
@@ -567,9 +585,9 @@ void run_all(gpgp_batch *b) {
 // (set, never cleared, by the kernels), so they can run side by side: the graph
 // forks from the context stream into up to kLanes streams, each running its
 // buckets in turn, and joins back. Buckets go to lanes longest first by their
-// measured time (the autotuner's; FP64 plans: count x nb^3), each to the lane
-// with the least work so far. Small buckets whose launches fill few SMs then
-// overlap with the large ones.
+// measured time (FP64 plans: count x nb^3), each to the lane with the least work so
+// far (the lane does not enter a bucket's results). Small buckets whose launches fill
+// few SMs then overlap with the large ones.
 constexpr int kLanes = 4;
 
 void run_all_lanes(gpgp_batch *b) {
@@ -580,7 +598,7 @@ void run_all_lanes(gpgp_batch *b) {
   for (size_t i = 0; i < order.size(); ++i) order[i] = (int)i;
   auto cost = [&](int i) {
     const Bucket &k = *b->buckets[i];
-    return k.best_ms > 0 ? k.best_ms : (double)k.count * k.nb * k.nb * k.nb;
+    return k.run_ms > 0 ? k.run_ms : (double)k.count * k.nb * k.nb * k.nb;
   };
   std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return cost(x) > cost(y); });
   std::vector<double> load(nl, 0.0);
@@ -728,8 +746,8 @@ void build_plan(gpgp_batch *b, gpgp_ctx *ctx, const gpgp_batch_problem *probs, i
 }  // namespace
 
 // One-shot batched solve for the request server: plan, upload, run the pipeline
-// once without autotuning or graph capture (the tensor-core variant for mixed
-// precision, the FP64 pipe otherwise, so a problem's result does not depend on
+// once without graph capture (variant 1 for mixed precision, the FP64 pipe otherwise,
+// whatever the count, so a problem's result does not depend on
 // its batch-mates) and read the evidence, predictive means and variances back.
 gpgp_status gpgp::batch_solve_once(gpgp_ctx *ctx, const gpgp_batch_problem *probs, int32_t nprob,
                                    int32_t precision, double jitter, double *lml, double *mean,
@@ -767,32 +785,22 @@ gpgp_status gpgp_batch_create(gpgp_ctx *ctx, const gpgp_batch_problem *probs, in
     std::unique_ptr<gpgp_batch> b(new gpgp_batch());
     build_plan(b.get(), ctx, probs, nprob, precision, quad_order, jitter);
     cudaStream_t st = ctx->stream;
-    // autotune: the FP64 pipe or the sliced tensor-core GEMM, per bucket (mixed precision only)
+    // each bucket's time, for the lanes of the graph
     cudaEvent_t e0, e1;
     GPGP_CUDA(cudaEventCreate(&e0));
     GPGP_CUDA(cudaEventCreate(&e1));
     for (auto &kp : b->buckets) {
       Bucket &k = *kp;
-      const int nvar = precision == GPGP_PREC_MIXED ? 3 : 1;
-      float best = 1e30f;
-      int bestv = 0;
-      for (int v = 0; v < nvar; ++v) {
-        k.variant = v;
-        run_bucket(b.get(), k, st);  // warm
-        GPGP_CUDA(cudaEventRecord(e0, st));
-        run_bucket(b.get(), k, st);
-        GPGP_CUDA(cudaEventRecord(e1, st));
-        GPGP_CUDA(cudaEventSynchronize(e1));
-        float ms = 0.f;
-        GPGP_CUDA(cudaEventElapsedTime(&ms, e0, e1));
-        b->tune_ms[v] += ms;
-        if (ms < best) {
-          best = ms;
-          bestv = v;
-        }
-      }
-      k.variant = bestv;
-      k.best_ms = nvar > 1 ? best : 0.0;
+      k.variant = plan_variant(precision, k.nb, k.count);
+      run_bucket(b.get(), k, st);  // warm
+      GPGP_CUDA(cudaEventRecord(e0, st));
+      run_bucket(b.get(), k, st);
+      GPGP_CUDA(cudaEventRecord(e1, st));
+      GPGP_CUDA(cudaEventSynchronize(e1));
+      float ms = 0.f;
+      GPGP_CUDA(cudaEventElapsedTime(&ms, e0, e1));
+      b->tune_ms[k.variant] += ms;
+      k.run_ms = precision == GPGP_PREC_MIXED ? ms : 0.0;
     }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);

@@ -375,9 +375,8 @@ gpgp_status gpgp_loo_mc(gpgp_model *model, int64_t draws, const double *z, doubl
  * kind sexp / matern32 / matern52 over all d inputs), gp_loo (approx_laplace,
  * Gauss-Hermite of order quad_order) and gp_pred with var = TRUE at its m test
  * points. Host buffers, column-major; n <= 4096, d <= 8. A plan uploads the
- * inputs, autotunes each size bucket (mixed precision: FP64 pipe or sliced
- * tensor cores, whichever is faster) and captures the whole pipeline in one
- * CUDA graph; gpgp_batch_run replays it; gpgp_batch_upload replaces the inputs
+ * inputs, times each size bucket once (its variant follows from the precision,
+ * its size and its count) and captures the whole pipeline in one CUDA graph; gpgp_batch_run replays it; gpgp_batch_upload replaces the inputs
  * of a plan with new data of the same shapes. Results are packed in problem
  * order: log_evidence[nprob], mean/var[sum m_i], loos[sum n_i]. A problem whose
  * factor is not positive definite gets log_evidence = -Inf. */
@@ -395,6 +394,8 @@ gpgp_status gpgp_batch_upload(gpgp_batch *b, const gpgp_batch_problem *probs);
 gpgp_status gpgp_batch_run(gpgp_batch *b);
 gpgp_status gpgp_batch_results(gpgp_batch *b, double *log_evidence, double *mean, double *var,
                                double *loos);
+/* bucket_variant: 0 FP64 pipe, 1 and 2 sliced tensor cores with outer panels of 64
+ * and 256 columns; tune_ms[3]: the buckets' measured time, summed per variant. */
 gpgp_status gpgp_batch_info(gpgp_batch *b, int32_t *nbuckets, int32_t *bucket_n,
                             int32_t *bucket_count, int32_t *bucket_variant, double *tune_ms);
 gpgp_status gpgp_batch_destroy(gpgp_batch *b);

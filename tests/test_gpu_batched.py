@@ -110,3 +110,33 @@ def test_batched_rerun_and_upload_are_consistent():
     info = plan.info()
     assert sum(cnt for _, cnt, _ in info["buckets"]) == 20
     plan.close()
+
+
+def plan_variant(nb, count):
+    """The documented rule of a mixed plan's buckets (nb = 64 T rows)."""
+    T = nb // 64
+    return "tensor-256" if T > 4 and count * (T - 3) ** 2 >= 506 else "tensor-64"
+
+
+def test_variant_follows_from_the_sizes():
+    """The variants of a mixed plan round differently above 256 rows, so the choice is a
+    rule on bucket size and count: two plans of the same problems take the same variants and
+    give the same bits."""
+    rng = np.random.default_rng(12)
+    probs = []
+    for nb, count in [(64, 3), (128, 2), (192, 5), (256, 2), (320, 126), (384, 57), (448, 31), (512, 20), (576, 15)]:
+        for _ in range(count):
+            n = nb - int(rng.integers(0, 20))
+            x = rng.uniform(-2, 2, (n, 2))
+            probs.append(dict(x=x, y=np.sin(2 * x[:, 0]) + 0.1 * rng.standard_normal(n), xt=x[:3], kind="sexp",
+                              lscale=0.7, magn=1.0, sigma=0.1))
+    runs = []
+    for _ in range(2):
+        plan = BatchPlan(probs, precision="mixed")
+        plan.run()
+        runs.append(plan.results())
+        assert [v for _, _, v in plan.info()["buckets"]] == [plan_variant(n, c) for n, c, _ in plan.info()["buckets"]]
+        plan.close()
+    for a, b in zip(*runs):
+        for k in ("log_evidence", "mean", "var", "loos"):
+            np.testing.assert_array_equal(a[k], b[k])
