@@ -41,9 +41,10 @@ __device__ __forceinline__ void cluster_wait() {
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
-// Bounded wait: returns false after ~2^24 polls (about a second or more).
-__device__ __forceinline__ bool mbar_wait_bounded(uint32_t bar, uint32_t parity) {
-  for (uint32_t it = 0; it < (1u << 24); ++it)
+// Bounded wait: returns false after `polls` polls (the default: about a second or more).
+constexpr uint32_t WAIT_POLLS = 1u << 24;
+__device__ __forceinline__ bool mbar_wait_bounded(uint32_t bar, uint32_t parity, uint32_t polls = WAIT_POLLS) {
+  for (uint32_t it = 0; it < polls; ++it)
     if (mbar_try_wait(bar, parity)) return true;
   return false;
 }

@@ -28,6 +28,15 @@ struct CudaError {
     if (e__ != cudaSuccess) throw ::gpgp::CudaError{e__, #call, __LINE__}; \
   } while (0)
 
+// Bounds of the kernels' waits for launches from the calling thread: polls after which a
+// wait gives up, per kernel (gpgp_wait_kernel), and the K chunks after which a GEMM CTA's
+// producer falls silent. Only tests change them (gpgp_wait_bound).
+struct WaitBounds {
+  uint32_t polls[GPGP_NWAIT];
+  int gemm_chunks;
+};
+extern thread_local WaitBounds tl_wait;
+
 // Number of kernel launches issued through the library (all contexts and
 // threads). Launches recorded into a graph under capture are not counted; a
 // graph replay adds its kernel nodes.

@@ -40,6 +40,7 @@
 // and update C while the next group accumulates. Every wait is bounded: on
 // timeout the kernel records an error, drains what it issued, releases TMEM
 // and returns.
+#include <limits.h>
 #include <math.h>
 #include <stdint.h>
 
@@ -600,6 +601,8 @@ struct OzGemmArgs {
   int gx, gy;       // tiles per problem along M and N
   int order;        // OzOrder
   int per, ntiles;  // tiles per problem and in the launch
+  uint32_t polls;   // TEST only: bound of every wait ..
+  int chunks;       // .. and K chunks after which a CTA's producer falls silent
 };
 
 // The order in which a problem's tiles are dealt to the CTAs, longest K range first
@@ -678,15 +681,16 @@ __device__ __forceinline__ bool oz_tile_at(const OzGemmArgs &g, int L, OzTile &t
 }
 
 // Bounded wait that also gives up when another role has aborted.
-__device__ __forceinline__ bool oz_wait(uint32_t bar, uint32_t parity, volatile int *abort_flag) {
-  for (uint32_t it = 0; it < (1u << 24); ++it) {
+__device__ __forceinline__ bool oz_wait(uint32_t bar, uint32_t parity, volatile int *abort_flag, uint32_t polls) {
+  for (uint32_t it = 0; it < polls; ++it) {
     if (mbar_try_wait(bar, parity)) return true;
     if ((it & 255u) == 255u && *abort_flag) return false;
   }
   return false;
 }
 
-template <int S>
+// TEST: with the bounds of gpgp_wait_bound (as arguments of the one kernel they cost 7%)
+template <int S, bool TEST>
 // 576 threads: the register cap keeps the block inside one SM's register file
 __global__ void __maxnreg__(96) oz_gemm_kernel(const OzGemmArgs g) {
   using Cfg = OzCfg<S>;
@@ -697,6 +701,7 @@ __global__ void __maxnreg__(96) oz_gemm_kernel(const OzGemmArgs g) {
   __shared__ uint32_t tmem_base_sh;
   __shared__ int abort_sh;
   volatile int *abort_flag = &abort_sh;
+  const uint32_t polls = TEST ? g.polls : WAIT_POLLS;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // barriers: full[NST] (operands landed), empty[NST] (MMAs that read a stage done),
   // tfull[NSET] (an accumulator set is ready), tempty[NSET] (the epilogue drained it), drain
@@ -735,7 +740,7 @@ __global__ void __maxnreg__(96) oz_gemm_kernel(const OzGemmArgs g) {
   if (warp == 0) {
     // ---- producer: K chunks of this CTA's tiles into the stage ring ----
     if (lane == 0) {
-      int st = 0;
+      int st = 0, left = TEST ? g.chunks : 0;
       uint32_t ph = 0;
       for (int L = blockIdx.x; L < ntiles; L += gridDim.x) {
         OzTile t;
@@ -746,7 +751,8 @@ __global__ void __maxnreg__(96) oz_gemm_kernel(const OzGemmArgs g) {
                              ((int64_t)t.c0 * g.b_nrb + g.b_rb0 + t.col0 / OZ_TR) * Cfg::TILE;
         const int64_t asl = (int64_t)g.a_nkc * g.a_nrb * Cfg::TILE, bsl = (int64_t)g.b_nkc * g.b_nrb * Cfg::TILE;
         for (int c = 0; c < t.nch; ++c) {
-          if (!oz_wait(bar(EMPTY + st), ph ^ 1u, abort_flag)) {
+          if (TEST && --left < 0) goto producer_done;
+          if (!oz_wait(bar(EMPTY + st), ph ^ 1u, abort_flag, polls)) {
             if (!*abort_flag) atomicExch(g.err, 1);
             abort_sh = 1;
             goto producer_done;
@@ -780,7 +786,15 @@ __global__ void __maxnreg__(96) oz_gemm_kernel(const OzGemmArgs g) {
     // never carries).
     const uint64_t adesc = umma_desc(smem_u32(smem), 128u, 16u * Cfg::TK);
     const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0);
+    // Whether a wait gives up depends on a lane's own polls and on when it sees the abort
+    // flag, but the lanes must stay together (the barriers need all 32): a lane's outcome
+    // only keeps the leader from issuing, and the warp leaves the loop by a vote. The vote
+    // stands after the issue, off the way from the operands to their products: there the
+    // loop is also 3 to 5% faster than with a branch at each wait (4096^2 x 4096, S = 4 /
+    // 8: 1.20 / 2.96 ms; a branch 1.27 / 3.13, a vote at each wait 1.31 / 3.18, lane 0's
+    // outcome shuffled to the others 1.38 / 3.35).
     const bool leader = elect_one();
+    bool ok = true;
     int st = 0, b = 0;
     uint32_t ph = 0, tph = 0;  // tph bit b: parity of accumulator set b
     for (int L = blockIdx.x; L < ntiles; L += gridDim.x) {
@@ -790,30 +804,26 @@ __global__ void __maxnreg__(96) oz_gemm_kernel(const OzGemmArgs g) {
       for (int c = 0; c < t.nch; ++c) {
         const bool gend = ((c + 1) & (GROUP - 1)) == 0 || c == t.nch - 1;
         if ((c & (GROUP - 1)) == 0) {
-          if (!oz_wait(bar(TEMPTY + b), ((tph >> b) & 1u) ^ 1u, abort_flag)) {
-            if (!*abort_flag) atomicExch(g.err, 2);
-            abort_sh = 1;
-            goto mma_done;
-          }
+          ok &= oz_wait(bar(TEMPTY + b), ((tph >> b) & 1u) ^ 1u, abort_flag, polls);
           acc = 0;
         }
-        if (!oz_wait(bar(FULL + st), ph, abort_flag)) {
-          if (!*abort_flag) atomicExch(g.err, 2);
-          abort_sh = 1;
-          goto mma_done;
-        }
+        ok &= oz_wait(bar(FULL + st), ph, abort_flag, polls);
         tc_fence_after();
         const uint64_t ad0 = adesc + (uint64_t)((uint32_t)st * (uint32_t)(Cfg::STAGE >> 4));
         const uint64_t bd0 = ad0 + (uint64_t)((S * Cfg::A_SL) >> 4);
         const uint32_t d0 = tm + (uint32_t)(b * NACC * OZ_BN);
-        if (leader) {
+        if (leader && ok) {
           oz_issue<S, Cfg::TK / 16>(ad0, bd0, Cfg::A_SL, Cfg::B_SL, d0, acc);
           umma_commit(bar(EMPTY + st));
           if (gend) umma_commit(bar(TFULL + b));
         }
-        __syncwarp();
         acc = 1u;
         mma_issued = true;
+        if (!__all_sync(0xffffffffu, ok)) {
+          if (!*abort_flag) atomicExch(g.err, 2);
+          abort_sh = 1;
+          goto mma_done;
+        }
         if (++st == NST) {
           st = 0;
           ph ^= 1u;
@@ -887,7 +897,7 @@ __global__ void __maxnreg__(96) oz_gemm_kernel(const OzGemmArgs g) {
       }
       for (int gi = 0; gi < ngr; ++gi) {
         int ok = 1;
-        if (lane == 0) ok = oz_wait(bar(TFULL + b), tph[b], abort_flag) ? 1 : 0;
+        if (lane == 0) ok = oz_wait(bar(TFULL + b), tph[b], abort_flag, polls) ? 1 : 0;
         ok = __shfl_sync(0xffffffffu, ok, 0);
         if (!ok) {
           if (lane == 0) {
@@ -951,7 +961,7 @@ __global__ void __maxnreg__(96) oz_gemm_kernel(const OzGemmArgs g) {
   if (abort_sh) {
     // a wait ran out: let what was issued land (bounded) before the shared memory
     // and TMEM are released
-    if (warp == 1 && mma_issued && elect_one()) {
+    if (warp == 1 && mma_issued && elect_one()) {  // (the same lane as issued)
       umma_commit(bar(DRAIN));
       mbar_wait_bounded(bar(DRAIN), 0);
     }
@@ -969,6 +979,25 @@ __global__ void __maxnreg__(96) oz_gemm_kernel(const OzGemmArgs g) {
 
 thread_local int tl_oz_grid_cap = 0;
 
+static const WaitBounds kWaitDefault = {{WAIT_POLLS}, INT_MAX};
+thread_local WaitBounds tl_wait = kWaitDefault;
+
+template <int S>
+static void launch_oz_gemm(cudaStream_t s, int grid, const OzGemmArgs &g) {
+  static PerDevice attr;
+  per_device(attr, [] {
+    GPGP_CUDA(cudaFuncSetAttribute(oz_gemm_kernel<S, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   OzCfg<S>::SMEM));
+    GPGP_CUDA(cudaFuncSetAttribute(oz_gemm_kernel<S, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   OzCfg<S>::SMEM));
+    return 1;
+  });
+  if (g.polls == WAIT_POLLS && g.chunks == INT_MAX)
+    oz_gemm_kernel<S, false><<<(unsigned)grid, OZ_THREADS, OzCfg<S>::SMEM, s>>>(g);
+  else
+    oz_gemm_kernel<S, true><<<(unsigned)grid, OZ_THREADS, OzCfg<S>::SMEM, s>>>(g);
+}
+
 static int oz_sm_count() { return device_sms(); }
 
 void oz_gemm_batched(cudaStream_t s, const OzSplit &A, int64_t a_row0, const OzSplit &B, int64_t b_row0,
@@ -979,14 +1008,6 @@ void oz_gemm_batched(cudaStream_t s, const OzSplit &A, int64_t a_row0, const OzS
   if ((alpha != 1.0 && alpha != -1.0) || (beta != 0.0 && beta != 1.0))
     throw CudaError{cudaErrorInvalidValue, "oz_gemm: alpha must be 1 or -1, beta 0 or 1", __LINE__};
   if (A.S != B.S) throw CudaError{cudaErrorInvalidValue, "oz_gemm: operands split to different slice counts", __LINE__};
-  static PerDevice attr;
-  per_device(attr, [] {
-    GPGP_CUDA(cudaFuncSetAttribute(oz_gemm_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, OzCfg<4>::SMEM));
-    GPGP_CUDA(cudaFuncSetAttribute(oz_gemm_kernel<5>, cudaFuncAttributeMaxDynamicSharedMemorySize, OzCfg<5>::SMEM));
-    GPGP_CUDA(cudaFuncSetAttribute(oz_gemm_kernel<OZ_FP64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   OzCfg<OZ_FP64>::SMEM));
-    return 1;
-  });
   OzGemmArgs g;
   g.a_sl = A.sl;
   g.a_ex = A.ex;
@@ -1026,6 +1047,8 @@ void oz_gemm_batched(cudaStream_t s, const OzSplit &A, int64_t a_row0, const OzS
   g.order = lower_only ? OZ_LOWER : kmode == 3 ? OZ_ROWS_UP : OZ_COLS;
   g.per = lower_only ? oz_lower_tiles(g.gx, g.gy) : g.gx * g.gy;
   g.ntiles = (int)(g.per * batch);
+  g.polls = tl_wait.polls[GPGP_WAIT_GEMM];
+  g.chunks = tl_wait.gemm_chunks;
   const int cap = tl_oz_grid_cap > 0 ? std::min(tl_oz_grid_cap, oz_sm_count()) : oz_sm_count();
   const int grid = std::min(g.ntiles, cap);
   double fl = 0.0;
@@ -1043,12 +1066,9 @@ void oz_gemm_batched(cudaStream_t s, const OzSplit &A, int64_t a_row0, const OzS
   }
   {
     KTScope kts(GPGP_KPROF_OZ_GEMM, s, fl);
-    if (A.S == OZ_FP64)
-      oz_gemm_kernel<OZ_FP64><<<(unsigned)grid, OZ_THREADS, OzCfg<OZ_FP64>::SMEM, s>>>(g);
-    else if (A.S == 5)
-      oz_gemm_kernel<5><<<(unsigned)grid, OZ_THREADS, OzCfg<5>::SMEM, s>>>(g);
-    else
-      oz_gemm_kernel<4><<<(unsigned)grid, OZ_THREADS, OzCfg<4>::SMEM, s>>>(g);
+    if (A.S == OZ_FP64) launch_oz_gemm<OZ_FP64>(s, grid, g);
+    else if (A.S == 5) launch_oz_gemm<5>(s, grid, g);
+    else launch_oz_gemm<4>(s, grid, g);
   }
   GPGP_CHECK_LAUNCH();
 }
@@ -1336,6 +1356,14 @@ __global__ void wait_selftest_kernel(uint32_t polls, int *err) {
   __syncthreads();
 }
 }  // namespace gpgp
+
+extern "C" gpgp_status gpgp_wait_bound(int32_t kernel, int32_t polls, int32_t gemm_chunks) {
+  using namespace gpgp;
+  if (kernel < 0 || kernel >= GPGP_NWAIT) return GPGP_EINVAL;
+  tl_wait.polls[kernel] = polls < 0 ? kWaitDefault.polls[kernel] : (uint32_t)polls;
+  tl_wait.gemm_chunks = gemm_chunks < 0 ? kWaitDefault.gemm_chunks : gemm_chunks;
+  return GPGP_OK;
+}
 
 extern "C" gpgp_status gpgp_wait_selftest(gpgp_ctx *ctx, int32_t polls) {
   if (!ctx || polls < 1) return GPGP_EINVAL;

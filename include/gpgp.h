@@ -524,6 +524,17 @@ gpgp_status gpgp_cov_df_selftest(gpgp_ctx *ctx, const gpgp_kernel *k, const doub
  *      GPGP_ETIMEOUT and the context stays usable. ---- */
 gpgp_status gpgp_wait_selftest(gpgp_ctx *ctx, int32_t polls);
 
+/* ---- test hook: the bound of a kernel's waits, in polls, for launches made by the
+ *      calling thread from now on (negative: the default), and the number of K chunks
+ *      after which each CTA of a sliced GEMM stops loading operands (negative: never;
+ *      other kernels ignore it). A wait that runs out gives GPGP_ETIMEOUT from the call
+ *      that launched it, and the context stays usable. ---- */
+typedef enum gpgp_wait_kernel {
+  GPGP_WAIT_GEMM = 0, /* BF16-sliced tcgen05 GEMM */
+  GPGP_NWAIT = 1
+} gpgp_wait_kernel;
+gpgp_status gpgp_wait_bound(int32_t kernel, int32_t polls, int32_t gemm_chunks);
+
 #ifdef __cplusplus
 }
 #endif
