@@ -211,6 +211,14 @@ void refine_alpha(gpgp_model *m, Work &w, double *alpha, double *fnew, int iters
   }
 }
 
+// Reads the tensor-core error flag; a set flag means a bounded wait ran out.
+bool tc_error(gpgp_model *m) {
+  int h = 0;
+  GPGP_CUDA(cudaMemcpyAsync(&h, m->errflag.p, sizeof(int), cudaMemcpyDeviceToHost, m->ctx->stream));
+  GPGP_CUDA(cudaStreamSynchronize(m->ctx->stream));
+  return h != 0;
+}
+
 // refine < 0: the model's own refinement count (mixed precision only). hflags
 // (optional): w.flags[0] read back with the factorisation status in the same
 // synchronisation; a set site flag (NaN or V <= 0) makes the result void, and no
@@ -275,6 +283,7 @@ int64_t factor_and_solve(gpgp_model *m, Work &w, const double *zvec, double *alp
   GPGP_CUDA(cudaMemcpyAsync(&hstatus, w.status.p, sizeof(int), cudaMemcpyDeviceToHost, st));
   if (hflags) GPGP_CUDA(cudaMemcpyAsync(hflags, w.flags.p, sizeof(int), cudaMemcpyDeviceToHost, st));
   GPGP_CUDA(cudaStreamSynchronize(st));
+  check_wait(hstatus);
   m->have_binv_diag = false;
   m->have_Linv = use_w && hstatus == 0;
   if (hflags && (*hflags & 6)) return 0;
@@ -282,8 +291,9 @@ int64_t factor_and_solve(gpgp_model *m, Work &w, const double *zvec, double *alp
     // The sliced trailing updates carry an error of ~2^-33 of the largest entries
     // of B; when B's entries are large (big Laplace weights W) and a pivot is
     // small, that can break the factorisation of a matrix that is positive
-    // definite in FP64. Redo this factorisation on the FP64 pipe, whose
-    // verdict is the reference's.
+    // definite in FP64. Redo this factorisation at FP64 accuracy, whose
+    // verdict is the reference's. (A product that gave up on a wait is none.)
+    if (tc_error(m)) throw WaitTimeout{};
     ++m->fp64_fallbacks;
     return factor_and_solve(m, w, zvec, alpha, fnew, logdetL, true, refine, hflags);
   }
@@ -320,14 +330,6 @@ void compute_binv_diag(gpgp_model *m) {
   m->binv_diag.alloc(st, n);
   col_sumsq_lower(st, m->Linv.p, n, n, m->binv_diag.p);
   m->have_binv_diag = true;
-}
-
-// Reads the tensor-core error flag; a set flag means a bounded wait ran out.
-bool tc_error(gpgp_model *m) {
-  int h = 0;
-  GPGP_CUDA(cudaMemcpyAsync(&h, m->errflag.p, sizeof(int), cudaMemcpyDeviceToHost, m->ctx->stream));
-  GPGP_CUDA(cudaStreamSynchronize(m->ctx->stream));
-  return h != 0;
 }
 
 gpgp_status fit_full(gpgp_model *m, gpgp_fit_result *res) {
@@ -495,6 +497,7 @@ gpgp_status fit_full(gpgp_model *m, gpgp_fit_result *res) {
           res->log_evidence = NAN;
           return fail(ctx, GPGP_ENAN, "NaN in the Laplace pseudo-data");
         }
+        check_wait(hdef[0]);
         if (hdef[0] != 0) {
           res->status = GPGP_ENOT_PD;
           res->info = hdef[0];
@@ -746,6 +749,7 @@ gpgp_status fit_common(gpgp_ctx *ctx, const gpgp_kernel *k, const gpgp_lik *lik,
   if (st != GPGP_OK) {
     GPGP_CUDA(cudaStreamSynchronize(s));
     if (hflags[0]) return nan_inputs();
+    if (tc_error(m.get())) throw WaitTimeout{};  // (what it left behind may have failed the fit)
     return st;
   }
   hflags[1] = 0;

@@ -329,7 +329,7 @@ __global__ void __launch_bounds__(256) bat_finish_kernel(int64_t nb, int64_t mb,
                                                          const double *__restrict__ ghw, double jitter,
                                                          double *__restrict__ lml, double *__restrict__ mean,
                                                          double *__restrict__ var, double *__restrict__ loos,
-                                                         double *__restrict__ binv) {
+                                                         double *__restrict__ binv, int *__restrict__ err) {
   __shared__ double red[256];
   const int64_t z = blockIdx.x;
   const double *p = prm + z * PRM;
@@ -338,6 +338,7 @@ __global__ void __launch_bounds__(256) bat_finish_kernel(int64_t nb, int64_t mb,
   const int tid = threadIdx.x;
   if (status[z] != 0) {
     if (tid == 0) lml[z] = -INFINITY;
+    if (tid == 0 && status[z] < 0) atomicExch(err, 6);  // no verdict: a wait ran out
     return;
   }
   const double *Yz = Y + z * nb, *az = alpha + z * nb, *fz = fhat + z * nb;
@@ -573,7 +574,7 @@ void run_bucket(gpgp_batch *b, Bucket &k, cudaStream_t st) {
   }
   bat_finish_kernel<<<(unsigned)P, 256, 0, st>>>(nb, mb, k.prm.p, k.status.p, k.Y.p, k.alpha.p, k.fhat.p, k.W.p,
                                                  k.ldp.p, k.R.p, k.T.p, b->quad_order, b->ghx.p, b->ghw.p,
-                                                 b->jitter, k.lml.p, k.mean.p, k.var.p, k.loos.p, k.binv.p);
+                                                 b->jitter, k.lml.p, k.mean.p, k.var.p, k.loos.p, k.binv.p, b->err.p);
   GPGP_CHECK_LAUNCH();
 }
 

@@ -22,6 +22,14 @@ struct CudaError {
   int line;
 };
 
+// A bounded device wait ran out (GPGP_ETIMEOUT).
+struct WaitTimeout {};
+// A factorisation's status word, read back: thrown before the word is taken for a verdict on
+// the matrix.
+inline void check_wait(int64_t status) {
+  if (status < 0) throw WaitTimeout{};
+}
+
 #define GPGP_CUDA(call)                                                   \
   do {                                                                    \
     cudaError_t e__ = (call);                                             \
@@ -232,7 +240,9 @@ constexpr int NB = 64;  // block size of the blocked factorisations
 void syrk_block(cudaStream_t s, const double *Ln, int64_t lda, int m, double *D);
 // Factor and inverse of the kb x kb (kb <= 64) diagonal block of each of `batch` problems
 // (matrices sA, inverses sW, log-determinant parts sL apart, one status word each); a
-// pivot that is not positive sets the status to its number, k0 + 1 ...
+// pivot that is not positive sets the status to its number, k0 + 1 ..; a wait that ran out
+// sets it to STATUS_TIMEOUT, so that what follows skips the problem in either case.
+constexpr int STATUS_TIMEOUT = -1;
 void potrf_diag(cudaStream_t s, double *A, int kb, int64_t lda, double *Winv, double *logdet_part, int *status,
                 int64_t k0, int64_t sA, int64_t sW, int64_t sL, int64_t batch);
 

@@ -78,8 +78,8 @@ __device__ __forceinline__ void cluster_sync() {
   cluster_wait();
 }
 // Bounded wait for phase 0 of a barrier that another CTA completes (a second or so)
-__device__ __forceinline__ bool wait_peer(uint32_t bar) {
-  for (uint32_t it = 0; it < (1u << 24); ++it) {
+__device__ __forceinline__ bool wait_peer(uint32_t bar, uint32_t polls = WAIT_POLLS) {
+  for (uint32_t it = 0; it < polls; ++it) {
     uint32_t ok;
     asm volatile(
         "{\n.reg .pred p;\nmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], 0;\n"
@@ -97,10 +97,13 @@ __device__ __forceinline__ double held(double x, double after, uint32_t sel) {
   return __hiloint2double(__double2hiint(x), __byte_perm(__double2loint(x), __double2hiint(after), sel));
 }
 
+// TEST: waits of max_polls polls (gpgp_wait_bound)
+template <bool TEST>
 __global__ void __cluster_dims__(DIAG_C, 1, 1) __launch_bounds__(DCT)
     potrf_diag_kernel(double *__restrict__ A, int kb, int64_t lda, double *__restrict__ Winv,
                       double *__restrict__ logdet_part, int *__restrict__ status, int64_t k0, int64_t sA, int64_t sW,
-                      int64_t sL) {
+                      int64_t sL, uint32_t max_polls) {
+  const uint32_t polls = TEST ? max_polls : WAIT_POLLS;
   constexpr int C = DIAG_C, PW = DCW;
   static_assert(NB == 64 && PW == 4 * DSEG, "a segment to a sub-partition");
   __shared__ __align__(16) double col[NB][NB];  // column k < base: L(:, k); else V's first terms -L(:, k) / L(k, k)
@@ -152,9 +155,9 @@ __global__ void __cluster_dims__(DIAG_C, 1, 1) __launch_bounds__(DCT)
   bool ok = true;
   const int kown = min(base + PW, kb);  // own columns end
   auto wait = [&](int h, int k) {
-    if (ok && !(k >= base && k < kown ? mbar_wait_bounded(bar(h, k), 0) : wait_peer(bar(h, k)))) {
+    if (ok && !(k >= base && k < kown ? mbar_wait_bounded(bar(h, k), 0, polls) : wait_peer(bar(h, k), polls))) {
       ok = false;
-      atomicMin(&failc, 0);
+      atomicMin(&failc, -1);
     }
   };
   if (compute) {
@@ -284,9 +287,9 @@ __global__ void __cluster_dims__(DIAG_C, 1, 1) __launch_bounds__(DCT)
   if (warp < 8 && cw < kb) {
     auto wait_v = [&](int k) {
       if (k >= kown) wait(1, k);
-      else if (ok && !mbar_wait_bounded(smem_u32(&vown[k - base]), 0)) {
+      else if (ok && !mbar_wait_bounded(smem_u32(&vown[k - base]), 0, polls)) {
         ok = false;
-        atomicMin(&failc, 0);
+        atomicMin(&failc, -1);
       }
     };
     wait_v(cw);
@@ -328,7 +331,13 @@ __global__ void __cluster_dims__(DIAG_C, 1, 1) __launch_bounds__(DCT)
 #pragma unroll
   for (int r = 0; r < C; ++r) bad = min(bad, fails[r]);
   if (bad < NB) {
-    if (rank == 0 && tid == 0) atomicCAS(status, 0, (int)(k0 + bad + 1));
+    // A wait ran out: every CTA still sends all it would have, and a CTA stays until what
+    // is sent to it has landed (bounded).
+    if (bad < 0 && tid < kb && base < kb && (tid < base || tid >= base + PW)) {
+      if (tid < base && base < 32) wait_peer(bar(0, tid));
+      wait_peer(bar(1, tid));
+    }
+    if (rank == 0 && tid == 0) atomicCAS(status, 0, bad < 0 ? STATUS_TIMEOUT : (int)(k0 + bad + 1));
     return;
   }
   for (int idx = tid; idx < PW * NB; idx += DCT) {
@@ -543,9 +552,10 @@ __global__ void __launch_bounds__(DIAG_THREADS) potrf_diag_many_kernel(double *_
 void potrf_diag(cudaStream_t s, double *A, int kb, int64_t lda, double *Winv, double *logdet_part, int *status,
                 int64_t k0, int64_t sA, int64_t sW, int64_t sL, int64_t batch) {
   KTScope kts(GPGP_KPROF_POTRF_DIAG, s, 2.0 * kb * kb * kb / 3 * (double)batch);
+  const uint32_t polls = tl_wait.polls[GPGP_WAIT_DIAG];
   if (batch * DIAG_C <= device_sms())
-    potrf_diag_kernel<<<(unsigned)(batch * DIAG_C), DCT, 0, s>>>(A, kb, lda, Winv, logdet_part, status, k0, sA, sW,
-                                                                 sL);
+    (polls == WAIT_POLLS ? potrf_diag_kernel<false> : potrf_diag_kernel<true>)<<<(unsigned)(batch * DIAG_C), DCT, 0, s>>>(
+        A, kb, lda, Winv, logdet_part, status, k0, sA, sW, sL, polls);
   else
     potrf_diag_many_kernel<<<(unsigned)batch, DIAG_THREADS, 0, s>>>(A, kb, lda, Winv, logdet_part, status, k0, sA, sW,
                                                                     sL);

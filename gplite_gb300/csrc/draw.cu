@@ -120,6 +120,7 @@ gpgp_status gpgp_mvn_draw(gpgp_ctx *ctx, const double *mean, const double *cov, 
     int hs = 0;
     GPGP_CUDA(cudaMemcpyAsync(&hs, status.p, sizeof(int), cudaMemcpyDeviceToHost, s));
     GPGP_CUDA(cudaStreamSynchronize(s));
+    check_wait(hs);
     if (hs != 0) return fail(ctx, GPGP_ENOT_PD, "the predictive covariance is not positive definite");
     dim3 g((unsigned)std::min<int64_t>((d + 255) / 256, 64), (unsigned)std::min<int64_t>(d, 65535));
     zero_upper_cols_kernel<<<g, 256, 0, s>>>(C.p, d, d);

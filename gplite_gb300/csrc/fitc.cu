@@ -232,6 +232,7 @@ int64_t chol_small(gpgp_ctx *ctx, double *A, int64_t M, double *Wblk, double *lo
   int h = 0;
   GPGP_CUDA(cudaMemcpyAsync(&h, status.p, sizeof(int), cudaMemcpyDeviceToHost, st));
   *logdet_out = read_scalar(ctx, out.p);
+  check_wait(h);
   return h;
 }
 

@@ -790,8 +790,8 @@ __global__ void __maxnreg__(96) oz_gemm_kernel(const OzGemmArgs g) {
     // flag, but the lanes must stay together (the barriers need all 32): a lane's outcome
     // only keeps the leader from issuing, and the warp leaves the loop by a vote. The vote
     // stands after the issue, off the way from the operands to their products: there the
-    // loop is also 3 to 5% faster than with a branch at each wait (4096^2 x 4096, S = 4 /
-    // 8: 1.20 / 2.96 ms; a branch 1.27 / 3.13, a vote at each wait 1.31 / 3.18, lane 0's
+    // loop is also 2 to 5% faster than with a branch at each wait (4096^2 x 4096, S = 4 /
+    // 8: 1.24 / 2.96 ms; a branch 1.26 / 3.12, a vote at each wait 1.31 / 3.18, lane 0's
     // outcome shuffled to the others 1.38 / 3.35).
     const bool leader = elect_one();
     bool ok = true;
@@ -979,7 +979,7 @@ __global__ void __maxnreg__(96) oz_gemm_kernel(const OzGemmArgs g) {
 
 thread_local int tl_oz_grid_cap = 0;
 
-static const WaitBounds kWaitDefault = {{WAIT_POLLS}, INT_MAX};
+static const WaitBounds kWaitDefault = {{WAIT_POLLS, WAIT_POLLS}, INT_MAX};
 thread_local WaitBounds tl_wait = kWaitDefault;
 
 template <int S>

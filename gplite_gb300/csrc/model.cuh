@@ -235,6 +235,8 @@ gpgp_status guarded(gpgp_ctx *ctx, F &&fn) {
     return fail(ctx, GPGP_ECUDA, m);
   } catch (const std::bad_alloc &) {
     return fail(ctx, GPGP_EOOM, "device or host allocation failed");
+  } catch (const WaitTimeout &) {
+    return fail(ctx, GPGP_ETIMEOUT, "a bounded device wait ran out");
   }
 }
 

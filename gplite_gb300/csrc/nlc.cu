@@ -274,6 +274,7 @@ gpgp_status nlc_bad_terms(gpgp_model *m, int64_t nb, const int *bad, const doubl
   GPGP_CHECK_LAUNCH();
   GPGP_CUDA(cudaMemcpyAsync(&hs, status.p + 1, sizeof(int), cudaMemcpyDeviceToHost, s));
   GPGP_CUDA(cudaStreamSynchronize(s));
+  check_wait(hs);
   if (hs)
     return fail(ctx, GPGP_ENOT_PD,
                 "chol(pred_cov) of the bad sites failed: the posterior of the whole data is not proper");
@@ -298,6 +299,7 @@ gpgp_status nlc_bad_terms(gpgp_model *m, int64_t nb, const int *bad, const doubl
   potrf(s, A.p, nb, nb, Wa.p, lda_.p, status.p + 2);
   GPGP_CUDA(cudaMemcpyAsync(&hs, status.p + 2, sizeof(int), cudaMemcpyDeviceToHost, s));
   GPGP_CUDA(cudaStreamSynchronize(s));
+  check_wait(hs);
   if (hs) {
     *improper = true;
     return GPGP_OK;
@@ -427,6 +429,7 @@ gpgp_status nlc_fit_full(gpgp_model *m, const double *K, const double *logC, boo
   int hs = 0;
   GPGP_CUDA(cudaMemcpyAsync(&hs, status.p, sizeof(int), cudaMemcpyDeviceToHost, s));
   GPGP_CUDA(cudaStreamSynchronize(s));
+  check_wait(hs);
   if (hs) return fail(ctx, GPGP_ENOT_PD, "Cholesky factorisation of the good sites: not positive definite");
   // alpha1 = s L^-T L^-1 (s z)
   a1.alloc(s, ng);

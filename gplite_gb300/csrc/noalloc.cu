@@ -188,6 +188,7 @@ extern "C" gpgp_status gpgp_fit_gaussian_noalloc(gpgp_ctx *ctx, const gpgp_kerne
       *log_evidence = NAN;
       return fail(ctx, GPGP_ENAN, "x or y holds NaN or Inf");
     }
+    check_wait(hstatus[0]);
     if (hstatus[0] != 0) {
       *log_evidence = -INFINITY;
       return fail(ctx, GPGP_ENOT_PD, "Cholesky factorisation: matrix is not positive definite");

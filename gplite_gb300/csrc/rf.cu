@@ -323,6 +323,7 @@ gpgp_status fit_rf(gpgp_model *m, gpgp_fit_result *res) {
       res->log_evidence = NAN;
       return fail(ctx, GPGP_ENAN, "NaN in the Laplace pseudo-data");
     }
+    check_wait(hs[0]);
     if (hs[0] != 0) {
       res->status = GPGP_ENOT_PD;
       res->info = hs[0];
@@ -517,6 +518,7 @@ gpgp_status gpgp_rf_draw(gpgp_model *model, const double *xt, int64_t m, uint32_
     int hs = 0;
     GPGP_CUDA(cudaMemcpyAsync(&hs, status.p, sizeof(int), cudaMemcpyDeviceToHost, st));
     GPGP_CUDA(cudaStreamSynchronize(st));
+    check_wait(hs);
     if (hs != 0) return fail(ctx, GPGP_ENOT_PD, "chol(wcov) failed");
     // w = wmean + t(chol(wcov)) z (mvnrnd, R/gp_draw.R:182-188); sample = zt w
     copy_in(st, zd, z, (size_t)ks * draws, false);

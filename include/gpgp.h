@@ -531,7 +531,8 @@ gpgp_status gpgp_wait_selftest(gpgp_ctx *ctx, int32_t polls);
  *      that launched it, and the context stays usable. ---- */
 typedef enum gpgp_wait_kernel {
   GPGP_WAIT_GEMM = 0, /* BF16-sliced tcgen05 GEMM */
-  GPGP_NWAIT = 1
+  GPGP_WAIT_DIAG = 1, /* diagonal block of a Cholesky */
+  GPGP_NWAIT = 2
 } gpgp_wait_kernel;
 gpgp_status gpgp_wait_bound(int32_t kernel, int32_t polls, int32_t gemm_chunks);
 
