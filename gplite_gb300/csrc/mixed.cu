@@ -979,7 +979,7 @@ __global__ void __maxnreg__(96) oz_gemm_kernel(const OzGemmArgs g) {
 
 thread_local int tl_oz_grid_cap = 0;
 
-static const WaitBounds kWaitDefault = {{WAIT_POLLS, WAIT_POLLS}, INT_MAX};
+static const WaitBounds kWaitDefault = {{WAIT_POLLS, WAIT_POLLS, WAIT_POLLS}, INT_MAX};
 thread_local WaitBounds tl_wait = kWaitDefault;
 
 template <int S>
@@ -1138,7 +1138,8 @@ template <int S>
 __global__ void __launch_bounds__(PB_THREADS) panel_block_kernel(double *__restrict__ A, int64_t lda, int64_t r0,
                                                                  int64_t r1, int64_t j0,
                                                                  const double *__restrict__ W, int q1, int group,
-                                                                 int *err, const int *__restrict__ status) {
+                                                                 int *err, const int *__restrict__ status,
+                                                                 uint32_t polls) {
   using Cfg = PbCfg<S>;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t *As = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023), *Bs = As + S * Cfg::A_SL;
@@ -1180,7 +1181,7 @@ __global__ void __launch_bounds__(PB_THREADS) panel_block_kernel(double *__restr
       }
       __syncwarp();
     }
-    const bool done = mbar_wait_bounded(smem_u32(&bar), ph);
+    const bool done = mbar_wait_bounded(smem_u32(&bar), ph, polls);
     ph ^= 1u;
     tc_fence_after();
     return !__syncthreads_or(!done);
@@ -1285,7 +1286,12 @@ __global__ void __launch_bounds__(PB_THREADS) panel_block_kernel(double *__restr
       }
     }
   }
-  if (!ok && tid == 0) atomicExch(err, 5);
+  if (!ok && tid == 0) {
+    atomicExch(err, 5);
+    // the products that were waited for land (bounded) before their operands' shared memory
+    // and their TMEM are released
+    mbar_wait_bounded(smem_u32(&bar), ph ^ 1u);
+  }
   __syncthreads();
   if (warp == 0) {
     __syncwarp();
@@ -1322,7 +1328,8 @@ static void launch_panel_block(cudaStream_t s, double *A, int64_t lda, int64_t r
   cfg.stream = s;
   cfg.attrs = &at;
   cfg.numAttrs = 1;
-  GPGP_CUDA(cudaLaunchKernelEx(&cfg, panel_block_kernel<S>, A, lda, r0, r1, j0, W, q1, group, err, status));
+  GPGP_CUDA(cudaLaunchKernelEx(&cfg, panel_block_kernel<S>, A, lda, r0, r1, j0, W, q1, group, err, status,
+                               tl_wait.polls[GPGP_WAIT_PANEL]));
   GPGP_CHECK_LAUNCH();
 }
 

@@ -530,9 +530,10 @@ gpgp_status gpgp_wait_selftest(gpgp_ctx *ctx, int32_t polls);
  *      other kernels ignore it). A wait that runs out gives GPGP_ETIMEOUT from the call
  *      that launched it, and the context stays usable. ---- */
 typedef enum gpgp_wait_kernel {
-  GPGP_WAIT_GEMM = 0, /* BF16-sliced tcgen05 GEMM */
-  GPGP_WAIT_DIAG = 1, /* diagonal block of a Cholesky */
-  GPGP_NWAIT = 2
+  GPGP_WAIT_GEMM = 0,  /* BF16-sliced tcgen05 GEMM */
+  GPGP_WAIT_DIAG = 1,  /* diagonal block of a Cholesky */
+  GPGP_WAIT_PANEL = 2, /* rows below a block column of the sliced Cholesky */
+  GPGP_NWAIT = 3
 } gpgp_wait_kernel;
 gpgp_status gpgp_wait_bound(int32_t kernel, int32_t polls, int32_t gemm_chunks);
 

@@ -13,7 +13,7 @@ from gplite_gb300.batch import gp_fit_batched
 
 pytestmark = pytest.mark.gpu
 
-GEMM, DIAG = 0, 1
+GEMM, DIAG, PANEL = 0, 1, 2
 
 
 @contextlib.contextmanager
@@ -86,3 +86,10 @@ def test_batched_diagonal_block_gives_up_and_recovers(precision):
             gp_fit_batched(probs, precision=precision)
     assert e.value.status == L.ETIMEOUT
     assert all(np.isfinite(r["log_evidence"]) for r in gp_fit_batched(probs, precision=precision))
+
+
+@pytest.mark.parametrize("n,precision", [(500, "mixed"), (1000, "fp64"), (1700, "mixed"), (1700, "fp64")])
+def test_panel_gives_up_and_recovers(n, precision):
+    """The rows below a panel stop waiting for their products while these still run (one CTA
+    and a cluster of CTAs to a row tile): the products land before their memory is freed."""
+    gives_up_and_recovers(PANEL, n, precision)
