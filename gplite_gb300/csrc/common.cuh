@@ -44,6 +44,7 @@ struct WaitBounds {
   int gemm_chunks;
 };
 extern thread_local WaitBounds tl_wait;
+constexpr uint32_t FLOW_POLLS = 1u << 21;  // trsv_flow's (two loads from L2 each)
 
 // Number of kernel launches issued through the library (all contexts and
 // threads). Launches recorded into a graph under capture are not counted; a

@@ -725,7 +725,7 @@ __global__ void __launch_bounds__(256) trsv_flow_kernel(const double *__restrict
                                                         const double *__restrict__ Winv,
                                                         const double *__restrict__ b, double *x, int trans,
                                                         const int *__restrict__ status, unsigned *sync,
-                                                        int *err) {
+                                                        int *err, uint32_t polls) {
   __shared__ double Ws[NB][NB + 1];
   __shared__ double xs[FLOW_BATCH][NB];
   __shared__ double vs[NB];
@@ -794,7 +794,10 @@ __global__ void __launch_bounds__(256) trsv_flow_kernel(const double *__restrict
             asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(e[h]) : "l"(x + j0 + lane + 32 * h));
         }
         const bool all = __all_sync(0xffffffffu, e[0] != FLOW_EMPTY && e[1] != FLOW_EMPTY);
-        const bool last = warp > 0 || it >= (1u << 21) || ((it & 1023u) == 1023u && *(volatile const int *)err != 0);
+        // (one outcome for the warp, whose lanes may see the error word at different times:
+        // the vote above needs all of them)
+        const bool last =
+            warp > 0 || it >= polls || ((it & 1023u) == 1023u && __any_sync(0xffffffffu, *(volatile const int *)err != 0));
         if (all || last) {
           xs[warp][lane] = __longlong_as_double((long long)e[0]);
           xs[warp][lane + 32] = __longlong_as_double((long long)e[1]);
@@ -966,7 +969,8 @@ void trsv_flow(cudaStream_t s, const double *L, int64_t n, int64_t lda, const do
   GPGP_CHECK_LAUNCH();
   const unsigned grid = (unsigned)std::min<int64_t>(nblk, g_sms);
   KTScope kts(GPGP_KPROF_TRSV, s, (double)n * (double)n);
-  trsv_flow_kernel<<<grid, 256, 0, s>>>(L, n, lda, Winv, b, x, trans ? 1 : 0, status, sync, err);
+  trsv_flow_kernel<<<grid, 256, 0, s>>>(L, n, lda, Winv, b, x, trans ? 1 : 0, status, sync, err,
+                                        tl_wait.polls[GPGP_WAIT_FLOW]);
   GPGP_CHECK_LAUNCH();
 }
 

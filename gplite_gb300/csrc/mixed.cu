@@ -979,7 +979,7 @@ __global__ void __maxnreg__(96) oz_gemm_kernel(const OzGemmArgs g) {
 
 thread_local int tl_oz_grid_cap = 0;
 
-static const WaitBounds kWaitDefault = {{WAIT_POLLS, WAIT_POLLS, WAIT_POLLS}, INT_MAX};
+static const WaitBounds kWaitDefault = {{WAIT_POLLS, WAIT_POLLS, WAIT_POLLS, FLOW_POLLS}, INT_MAX};
 thread_local WaitBounds tl_wait = kWaitDefault;
 
 template <int S>

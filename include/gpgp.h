@@ -533,7 +533,8 @@ typedef enum gpgp_wait_kernel {
   GPGP_WAIT_GEMM = 0,  /* BF16-sliced tcgen05 GEMM */
   GPGP_WAIT_DIAG = 1,  /* diagonal block of a Cholesky */
   GPGP_WAIT_PANEL = 2, /* rows below a block column of the sliced Cholesky */
-  GPGP_NWAIT = 3
+  GPGP_WAIT_FLOW = 3,  /* triangular solve ordered by its solution's entries */
+  GPGP_NWAIT = 4
 } gpgp_wait_kernel;
 gpgp_status gpgp_wait_bound(int32_t kernel, int32_t polls, int32_t gemm_chunks);
 

@@ -13,7 +13,7 @@ from gplite_gb300.batch import gp_fit_batched
 
 pytestmark = pytest.mark.gpu
 
-GEMM, DIAG, PANEL = 0, 1, 2
+GEMM, DIAG, PANEL, FLOW = 0, 1, 2, 3
 
 
 @contextlib.contextmanager
@@ -93,3 +93,9 @@ def test_panel_gives_up_and_recovers(n, precision):
     """The rows below a panel stop waiting for their products while these still run (one CTA
     and a cluster of CTAs to a row tile): the products land before their memory is freed."""
     gives_up_and_recovers(PANEL, n, precision)
+
+
+@pytest.mark.parametrize("n", [577, 850, 3000])
+def test_triangular_solve_gives_up_and_recovers(n):
+    """Blocks of the solution that are not there at the first look (n > 512: many CTAs)."""
+    gives_up_and_recovers(FLOW, n, "fp64")
