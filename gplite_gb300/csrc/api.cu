@@ -1178,17 +1178,17 @@ static gpgp_status pred_impl(gpgp_model *m, const double *xt, int64_t mt, uint32
     } else if (var) {
       Phase ph(ctx, GPGP_PHASE_PRED_VAR);
       // var = diag(Ktt) - colSums((C_chol^-1 Kt^T)^2), C_chol^-1 = L^-1 diag(s)  (R/gp_pred.R:216-228)
-      const int64_t chunk = std::max<int64_t>(1, std::min<int64_t>(mt, (int64_t)(1ll << 28) / std::max<int64_t>(n, 1)));
+      const int64_t chunk = pred_chunk(n, mt);
       DBuf R, tmp, csum, kdiag;
       R.alloc(s, (size_t)n * chunk);
-      tmp.alloc(s, (size_t)NB * chunk);
       csum.alloc(s, mt);
       kdiag.alloc(s, mt);
       IBuf status;
       status.alloc(s, 1);
       GPGP_CUDA(cudaMemsetAsync(status.p, 0, sizeof(int), s));
-      const bool mixed = m->opts.precision == GPGP_PREC_MIXED;
+      const bool mixed = m->opts.precision == GPGP_PREC_MIXED, sliced = !mixed && n >= SLICED_MIN;
       if (mixed) compute_linv(m);
+      else if (!sliced) tmp.alloc(s, (size_t)NB * chunk);
       for (int64_t c0 = 0; c0 < mt; c0 += chunk) {
         const int64_t mc = std::min(chunk, mt - c0);
         if (df)
@@ -1199,7 +1199,7 @@ static gpgp_status pred_impl(gpgp_model *m, const double *xt, int64_t mt, uint32
         if (mixed) {
           trmv_sumsq_mixed(s, m->Linv.p, n, n, R.p, mc, n, csum.p + c0, m->errflag.p);
         } else {
-          if (n >= SLICED_MIN)
+          if (sliced)
             trsm_sliced(s, m->L.p, n, n, m->Winv.p, R.p, mc, n, m->errflag.p, OZ_FP64);
           else
             trsm_lower(s, m->L.p, n, n, m->Winv.p, R.p, mc, n, tmp.p, status.p);

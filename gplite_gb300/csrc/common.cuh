@@ -429,7 +429,8 @@ void trtri_mixed(cudaStream_t s, const double *L, int64_t n, int64_t lda, const 
 // Binv (lower) = W^T W for lower-triangular W
 void lauum_mixed(cudaStream_t s, const double *W, int64_t n, int64_t ldw, double *Binv,
                  int64_t ldb, int *err, int S = 4);
-// X = L^-1 R in place (n x m, leading dimension ldr)
+// X = L^-1 R in place (n x m, leading dimension ldr); its scratch in bytes
+size_t trsm_sliced_bytes(int64_t n, int64_t m, int S);
 void trsm_sliced(cudaStream_t s, const double *L, int64_t n, int64_t lda, const double *Winv, double *R, int64_t m,
                  int64_t ldr, int *err, int S);
 // T = W R (W lower n x n, R n x m), then out[j] = sum_i T_ij^2

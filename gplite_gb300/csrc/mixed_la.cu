@@ -189,12 +189,15 @@ __global__ void put_diag_inverses_kernel(const double *__restrict__ Winv, int64_
 constexpr int64_t TRTRI_BASE = 512;  // diagonal blocks inverted level by level, batched
 
 // Batched scratch for a level: `count` split operands of rows x K each.
+static size_t split_batch_bytes(int64_t rows, int64_t K, int S) {
+  return (oz_split_bytes(rows, K, S) + 1023) / 1024 * 1024;
+}
 struct SplitBatch {
   void *p = nullptr;
   cudaStream_t s = nullptr;
   OzSplit sp;
   SplitBatch(cudaStream_t st, int64_t rows, int64_t K, int64_t count, int S) : s(st) {
-    const size_t per = (oz_split_bytes(rows, K, S) + 1023) / 1024 * 1024;
+    const size_t per = split_batch_bytes(rows, K, S);
     if (cudaMallocAsync(&p, per * count, st) != cudaSuccess) {
       p = nullptr;
       (void)cudaGetLastError();
@@ -308,6 +311,11 @@ void lauum_mixed(cudaStream_t s, const double *W, int64_t n, int64_t ldw, double
 // need fewer launches, but 128-row ones made the predictive variance 1.6 times and
 // 512-row ones 4 times less accurate.
 constexpr int64_t TRSM_OUTER = 512;
+
+size_t trsm_sliced_bytes(int64_t n, int64_t m, int S) {
+  return (size_t)((n + NB - 1) / NB) * split_batch_bytes(NB, NB, S) + oz_split_bytes(n, TRSM_OUTER, S) +
+         oz_split_bytes(m, TRSM_OUTER, S);
+}
 
 void trsm_sliced(cudaStream_t s, const double *L, int64_t n, int64_t lda, const double *Winv, double *R, int64_t m,
                  int64_t ldr, int *err, int S) {

@@ -291,8 +291,13 @@ gpgp_status nlc_bad_terms(gpgp_model *m, int64_t nb, const int *bad, const doubl
 void gather_rows(cudaStream_t s, const double *F, int64_t ldf, int64_t nf, const int *idx, int64_t m, double *out);
 void split_sites(gpgp_model *m, std::vector<int> *hg, std::vector<int> *hb, IBuf *good, IBuf *bad);
 
+// Test points whose variance gp_pred computes at a time (n x chunk doubles: 2 GB).
+inline int64_t pred_chunk(int64_t n, int64_t mt) {
+  return std::max<int64_t>(1, std::min<int64_t>(mt, (int64_t)(1ll << 28) / std::max<int64_t>(n, 1)));
+}
+
 // Batched pipeline for the request server (batched.cu): one plan, one run, no
-// autotune or graph; lml[nprob], mean/var[sum m] packed in problem order.
+// graph; lml[nprob], mean/var[sum m] packed in problem order.
 gpgp_status batch_solve_once(gpgp_ctx *ctx, const gpgp_batch_problem *probs, int32_t nprob,
                              int32_t precision, double jitter, double *lml, double *mean, double *var);
 size_t batch_bytes_estimate(int64_t n, int64_t m, int32_t d, int32_t precision);

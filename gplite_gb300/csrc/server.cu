@@ -125,6 +125,15 @@ void estimate(const gpgp_server *s, Req *r) {
   if (r->kind == REQ_PREDICT) {
     const double nn = (double)r->target->n;
     r->bytes = (int64_t)(8.0 * (2.0 * nn * std::min(m, 4096.0) + 64.0 * m + 4.0 * nn) + (1 << 20));
+    const gpgp_model &t = *r->target;
+    if (t.fitc) {
+      // the substitution's operands (m x 64 and M x 64)
+      if (r->m >= SLICED_ROWS)
+        r->bytes += (int64_t)(oz_split_bytes(r->m, NB, OZ_FP64) + oz_split_bytes(t.fitc->M, NB, OZ_FP64));
+    } else if (r->var && !t.nlc && t.opts.precision == GPGP_PREC_FP64 && t.n >= SLICED_MIN) {
+      // the variance's solve: the diagonal blocks' inverses, n x 512 and m x 512, split
+      r->bytes += (int64_t)trsm_sliced_bytes(t.n, pred_chunk(t.n, r->m), OZ_FP64);
+    }
     r->work = 2.0 * nn * nn * m;
     return;
   }
@@ -149,7 +158,8 @@ void estimate(const gpgp_server *s, Req *r) {
   // the operands of the variance's solve (n x 512 and m x 512) or, for EP, L^-1 with the
   // operands of its products (2.5 n^2 doubles)
   const bool sliced = !mixed && r->n >= SLICED_MIN;
-  const double extra = mixed ? 900.0 * n : sliced ? 2700.0 * n + 1100.0 * std::min(m, 4096.0) : 64.0 * n;
+  const double extra =
+      mixed ? 900.0 * n : sliced ? 2700.0 * n + 1100.0 * (double)pred_chunk(r->n, r->m) : 64.0 * n;
   const double nn = mixed ? 5.0 : sliced && r->ap.kind == GPGP_APPROX_EP ? 5.5 : 3.0;
   r->bytes = (int64_t)(8.0 * (nn * n * n + 2.0 * n * std::min(m, 4096.0) + extra + 20.0 * n) + (4 << 20));
   r->resident = (int64_t)(8.0 * (2.0 * n * n + 64.0 * n + 12.0 * n));

@@ -149,3 +149,35 @@ def test_budget_admission():
         st = s.stats()
     assert st["bytes_peak"] <= budget
     assert st["failed"] == 1
+
+
+def split_bytes(rows, K):
+    """An operand in eight slices: 64-row tiles, one more than needed and an even count,
+    2 bytes an entry and slice, K in multiples of 64, and the rows' exponents."""
+    r = ((rows + 63) // 64 + 2) // 2 * 2 * 64
+    return 4 * r + 256 + 8 * ((K + 63) // 64) * r * 64 * 2
+
+
+def test_prediction_estimate_holds_the_variance_scratch():
+    """The variance of an FP64 model of 896 points or more is solved with split operands: n x
+    512, m x 512 and the inverses of the diagonal blocks. A budget that holds the model, the
+    cross covariance and half of them refuses the prediction; one that holds all admits it."""
+    rng = np.random.default_rng(9)
+    n, m = 1500, 4096
+    x = rng.uniform(-2, 2, (n, 2))
+    y = np.sin(3 * x[:, 0]) + 0.1 * rng.standard_normal(n)
+    xt = rng.uniform(-2, 2, (m, 2))
+    gp = G.gp_init(G.cf_matern52(lscale=0.6, magn=1.0), G.lik_gaussian(sigma=0.1))
+    inv = (split_bytes(64, 64) + 1023) // 1024 * 1024 * ((n + 63) // 64)
+    scratch = split_bytes(n, 512) + split_bytes(m, 512) + inv
+    assert scratch > 45e6
+    cross = 8 * (2 * n * m + 64 * m + 4 * n) + (1 << 20)
+    resident = 8 * (2 * n * n + 76 * n)
+    for budget, want in ((resident + cross + scratch // 2, L.EOOM), (resident + cross + scratch + 4096, 0)):
+        with GPServer(precision="fp64", workers=1, hbm_budget=budget) as s:
+            r = s.poll(s.submit(gp, x, y, x[:1], keep=True))
+            assert r["status"] == 0 and s.stats()["bytes_resident"] == resident
+            assert s.poll(s.submit_pred(r["model"], xt))["status"] == want
+            # the mean alone needs none of it
+            assert s.poll(s.submit_pred(r["model"], xt, want_var=False))["status"] == 0
+            assert s.stats()["bytes_peak"] <= budget
