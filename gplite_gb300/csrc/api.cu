@@ -309,9 +309,9 @@ void compute_linv(gpgp_model *m) {
   Phase ph(m->ctx, GPGP_PHASE_TRTRI);
   if (m->opts.precision == GPGP_PREC_MIXED) {
     trtri_mixed(st, m->L.p, n, n, m->Winv.p, m->Linv.p, n, m->errflag.p);
-  } else if (n >= SLICED_MIN) {
-    trtri_mixed(st, m->L.p, n, n, m->Winv.p, m->Linv.p, n, m->errflag.p, OZ_FP64);
-  } else {
+  } else if (n < SLICED_MIN || !with_scratch([&] {
+               trtri_mixed(st, m->L.p, n, n, m->Winv.p, m->Linv.p, n, m->errflag.p, OZ_FP64);
+             })) {
     DBuf tmp;
     tmp.alloc(st, (size_t)NB * n);
     IBuf status;
@@ -1186,9 +1186,8 @@ static gpgp_status pred_impl(gpgp_model *m, const double *xt, int64_t mt, uint32
       IBuf status;
       status.alloc(s, 1);
       GPGP_CUDA(cudaMemsetAsync(status.p, 0, sizeof(int), s));
-      const bool mixed = m->opts.precision == GPGP_PREC_MIXED, sliced = !mixed && n >= SLICED_MIN;
+      const bool mixed = m->opts.precision == GPGP_PREC_MIXED;
       if (mixed) compute_linv(m);
-      else if (!sliced) tmp.alloc(s, (size_t)NB * chunk);
       for (int64_t c0 = 0; c0 < mt; c0 += chunk) {
         const int64_t mc = std::min(chunk, mt - c0);
         if (df)
@@ -1199,10 +1198,12 @@ static gpgp_status pred_impl(gpgp_model *m, const double *xt, int64_t mt, uint32
         if (mixed) {
           trmv_sumsq_mixed(s, m->Linv.p, n, n, R.p, mc, n, csum.p + c0, m->errflag.p);
         } else {
-          if (sliced)
-            trsm_sliced(s, m->L.p, n, n, m->Winv.p, R.p, mc, n, m->errflag.p, OZ_FP64);
-          else
+          if (n < SLICED_MIN || !with_scratch([&] {
+                trsm_sliced(s, m->L.p, n, n, m->Winv.p, R.p, mc, n, m->errflag.p, OZ_FP64);
+              })) {
+            if (!tmp.p) tmp.alloc(s, (size_t)NB * chunk);
             trsm_lower(s, m->L.p, n, n, m->Winv.p, R.p, mc, n, tmp.p, status.p);
+          }
           col_sumsq(s, R.p, n, mc, n, csum.p + c0);
         }
       }
@@ -1346,9 +1347,8 @@ gpgp_status gpgp_model_grad(gpgp_model *m, double *grad_terms, double *grad_lik_
       Phase ph(ctx, GPGP_PHASE_LAUUM);
       if (m->opts.precision == GPGP_PREC_MIXED)
         lauum_mixed(s, m->Linv.p, n, n, Bi.p, n, m->errflag.p);
-      else if (n >= SLICED_MIN)
-        lauum_mixed(s, m->Linv.p, n, n, Bi.p, n, m->errflag.p, OZ_FP64);
-      else
+      else if (n < SLICED_MIN ||
+               !with_scratch([&] { lauum_mixed(s, m->Linv.p, n, n, Bi.p, n, m->errflag.p, OZ_FP64); }))
         gemm64(s, true, false, n, n, n, 1.0, m->Linv.p, n, m->Linv.p, n, 0.0, Bi.p, n, true, 1);
     }
     // tr(C^-1) = sum_i s_i^2 Binv_ii

@@ -5,6 +5,7 @@
 
 #include <atomic>
 #include <mutex>
+#include <new>
 #include <string>
 #include <vector>
 
@@ -362,6 +363,18 @@ struct SplitBuf {
     if (p) cudaFreeAsync(p, s);
   }
 };
+// Runs fn, whose inputs are as they were when its scratch cannot be had (false). The
+// sliced products need room for their operands (16 bytes an entry of FP64's: a gradient 16 n^2
+// bytes, L^-1 10 n^2), the FP64 pipe none: a size that leaves none takes that one.
+template <class F>
+bool with_scratch(F &&fn) {
+  try {
+    fn();
+    return true;
+  } catch (const std::bad_alloc &) {
+    return false;
+  }
+}
 // rows x K operand: element (r, k) = P[r + k*ld] (trans 0) or P[k + r*ld] (trans 1)
 void oz_split(cudaStream_t s, const double *P, int64_t ld, int trans, int64_t rows, int64_t K,
               OzSplit *out);
@@ -429,7 +442,8 @@ void trtri_mixed(cudaStream_t s, const double *L, int64_t n, int64_t lda, const 
 // Binv (lower) = W^T W for lower-triangular W
 void lauum_mixed(cudaStream_t s, const double *W, int64_t n, int64_t ldw, double *Binv,
                  int64_t ldb, int *err, int S = 4);
-// X = L^-1 R in place (n x m, leading dimension ldr); its scratch in bytes
+// X = L^-1 R in place (n x m, leading dimension ldr; R as it was when it throws
+// std::bad_alloc); its scratch in bytes
 size_t trsm_sliced_bytes(int64_t n, int64_t m, int S);
 void trsm_sliced(cudaStream_t s, const double *L, int64_t n, int64_t lda, const double *Winv, double *R, int64_t m,
                  int64_t ldr, int *err, int S);

@@ -347,11 +347,14 @@ __global__ void __launch_bounds__(128) tri_block_kernel(const double *__restrict
 // tensor cores at FP64 accuracy from SLICED_ROWS rows on.
 void rows_times_bt(cudaStream_t s, int64_t n, int64_t N, int64_t K, double alpha, const double *A, int64_t lda,
                    const double *B, int64_t ldb, double beta, double *C, int64_t ldc, int *err) {
-  if (n < SLICED_ROWS) {
+  SplitBuf a(s), b(s);
+  if (n < SLICED_ROWS || !with_scratch([&] {
+        a.bind(n, K, OZ_FP64);
+        b.bind(N, K, OZ_FP64);
+      })) {
     gemm64(s, false, true, n, N, K, alpha, A, lda, B, ldb, beta, C, ldc);
     return;
   }
-  SplitBuf a(s, n, K, OZ_FP64), b(s, N, K, OZ_FP64);
   oz_split(s, A, lda, 0, n, K, &a.sp);
   oz_split(s, B, ldb, 0, N, K, &b.sp);
   oz_gemm(s, a.sp, 0, b.sp, 0, n, N, 0, a.sp.nkb, 0, alpha, beta, C, ldc, false, err);
@@ -366,12 +369,11 @@ void tri_rows(cudaStream_t s, const double *L, int64_t M, int64_t ldl, const dou
     GPGP_CUDA(cudaMemcpy2DAsync(X, ldx * sizeof(double), B, ldb * sizeof(double), n * sizeof(double), M,
                                 cudaMemcpyDeviceToDevice, s));
   const unsigned grid = (unsigned)((n + 15) / 16);
-  const bool sliced = err && n >= SLICED_ROWS;
   SplitBuf xs(s), ls(s);
-  if (sliced && M > TB) {
-    xs.bind(n, TB, OZ_FP64);
-    ls.bind(M, TB, OZ_FP64);
-  }
+  const bool sliced = err && n >= SLICED_ROWS && M > TB && with_scratch([&] {
+                        xs.bind(n, TB, OZ_FP64);
+                        ls.bind(M, TB, OZ_FP64);
+                      });
   const int64_t nblk = (M + TB - 1) / TB;
   for (int64_t b = 0; b < nblk; ++b) {
     const int64_t k0 = (mode == 0 ? b : nblk - 1 - b) * TB;

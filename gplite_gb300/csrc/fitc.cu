@@ -249,8 +249,9 @@ void rows_times_cminv(gpgp_model *m, const double *B, double *X, int64_t n) {
 // log-determinant by ~1e-5 relative at n = 65536. Eight slices are as accurate as the
 // FP64 pipe, which small n keep (the split operands' launches cost more there).
 void gram_tn(gpgp_model *m, const double *A, const double *B, int64_t n, int64_t M, double *C) {
-  if (n >= GRAM_SLICED_MIN) gram_sliced(m->ctx->stream, A, n, B, n, n, M, M, C, M, m->errflag.p);
-  else gemm64(m->ctx->stream, true, false, M, M, n, 1.0, A, n, B, n, 0.0, C, M);
+  if (n < GRAM_SLICED_MIN ||
+      !with_scratch([&] { gram_sliced(m->ctx->stream, A, n, B, n, n, M, M, C, M, m->errflag.p); }))
+    gemm64(m->ctx->stream, true, false, M, M, n, 1.0, A, n, B, n, 0.0, C, M);
 }
 
 // The lemma for the current S (R/linear_algebra.R:3-43): iDU = Kxz / S, C_m and its

@@ -97,7 +97,15 @@ void factor_panel(cudaStream_t x, cudaStream_t y, cudaStream_t z, const SideStre
 
 void potrf_mixed(cudaStream_t s, double *A, int64_t n, int64_t lda, double *Winv,
                  double *logdet_part, int *status, int *err, const SideStream *side, int S) {
-  SplitBuf a(s, n, NBO, S);  // the panel as the trailing update's operand
+  SplitBuf a(s);  // the panel as the trailing update's operand
+  if (S == OZ_FP64) {
+    if (!with_scratch([&] { a.bind(n, NBO, S); })) {
+      potrf(s, A, n, lda, Winv, logdet_part, status, 1);
+      return;
+    }
+  } else {
+    a.bind(n, NBO, S);
+  }
   cudaStreamCaptureStatus cap_st = cudaStreamCaptureStatusNone;
   GPGP_CUDA(cudaStreamIsCapturing(s, &cap_st));
   // Per-kernel timers (tl_kt) time each launch alone, so a profiled call runs the

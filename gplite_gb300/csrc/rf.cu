@@ -304,8 +304,9 @@ gpgp_status fit_rf(gpgp_model *m, gpgp_fit_result *res) {
     rf_scale_kernel<<<gz, 256, 0, st>>>(n, D, R.Z.p, m->V.p, m->z.p, Zv.p, rhs.p, flags.p);
     GPGP_CHECK_LAUNCH();
     // H = t(Z) %*% (Z / V) + I, L = t(chol(H + I))
-    if (n >= GRAM_SLICED_MIN) gram_sliced(st, R.Z.p, n, Zv.p, n, n, D, D, R.L.p, D, m->errflag.p);
-    else gemm64(st, true, false, D, D, n, 1.0, R.Z.p, n, Zv.p, n, 0.0, R.L.p, D);
+    if (n < GRAM_SLICED_MIN ||
+        !with_scratch([&] { gram_sliced(st, R.Z.p, n, Zv.p, n, n, D, D, R.L.p, D, m->errflag.p); }))
+      gemm64(st, true, false, D, D, n, 1.0, R.Z.p, n, Zv.p, n, 0.0, R.L.p, D);
     rf_add_identity_kernel<<<g1(D), 256, 0, st>>>(R.L.p, D);
     GPGP_CHECK_LAUNCH();
     potrf(st, R.L.p, D, D, R.Wblk.p, lp.p, status.p);
