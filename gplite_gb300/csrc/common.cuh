@@ -366,8 +366,11 @@ struct SplitBuf {
 // Runs fn, whose inputs are as they were when its scratch cannot be had (false). The
 // sliced products need room for their operands (16 bytes an entry of FP64's: a gradient 16 n^2
 // bytes, L^-1 10 n^2), the FP64 pipe none: a size that leaves none takes that one.
+// tl_lean: as if it could not (a thread that was promised the smaller amount).
+extern thread_local bool tl_lean;
 template <class F>
 bool with_scratch(F &&fn) {
+  if (tl_lean) return false;
   try {
     fn();
     return true;

@@ -95,6 +95,8 @@ void factor_panel(cudaStream_t x, cudaStream_t y, cudaStream_t z, const SideStre
 
 }  // namespace
 
+thread_local bool tl_lean = false;
+
 void potrf_mixed(cudaStream_t s, double *A, int64_t n, int64_t lda, double *Winv,
                  double *logdet_part, int *status, int *err, const SideStream *side, int S) {
   SplitBuf a(s);  // the panel as the trailing update's operand

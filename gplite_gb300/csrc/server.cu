@@ -56,6 +56,8 @@ struct Req {
   gpgp_model *target = nullptr;  // predict / release: the resident model
   double *mean = nullptr, *var = nullptr;
   int64_t bytes = 0;     // in-flight device memory estimate
+  int64_t lean_bytes = 0;  // without the scratch of FP64's sliced products (with_scratch)
+  bool lean = false;       // admitted on lean_bytes: runs without that scratch
   int64_t resident = 0;  // bytes that stay while the model is kept
   double work = 0;       // flop estimate (worker load balance)
   bool batchable = false;
@@ -118,13 +120,15 @@ struct gpgp_server {
 
 namespace {
 
-// device bytes while the request runs, and while its model stays resident
+// Device bytes while the request runs, and while its model stays resident. FP64 requests
+// that the budget could not hold with the scratch of their sliced products run without it.
 void estimate(const gpgp_server *s, Req *r) {
   const double n = (double)r->n, m = (double)r->m;
   const bool mixed = s->o.precision == GPGP_PREC_MIXED;
   if (r->kind == REQ_PREDICT) {
     const double nn = (double)r->target->n;
     r->bytes = (int64_t)(8.0 * (2.0 * nn * std::min(m, 4096.0) + 64.0 * m + 4.0 * nn) + (1 << 20));
+    r->lean_bytes = r->bytes;
     const gpgp_model &t = *r->target;
     if (t.fitc) {
       // the substitution's operands (m x 64 and M x 64)
@@ -138,7 +142,7 @@ void estimate(const gpgp_server *s, Req *r) {
     return;
   }
   if (r->batchable) {
-    r->bytes = (int64_t)batch_bytes_estimate(r->n, r->m, r->d, s->o.precision);
+    r->bytes = r->lean_bytes = (int64_t)batch_bytes_estimate(r->n, r->m, r->d, s->o.precision);
     r->work = n * n * n / 3.0 + n * n * m;
     return;
   }
@@ -147,7 +151,8 @@ void estimate(const gpgp_server *s, Req *r) {
     // beside the fit, the Gram product's two split operands (16 bytes an entry with its
     // row padding, at most 128 MB each) or those of the substitution (n x 64)
     const double gram = std::max(std::min(32.0 * n * (M + 128.0), 2.7e8), 16.0 * n * 80.0);
-    r->bytes = (int64_t)(8.0 * (8.0 * n * M + 12.0 * M * M + 3.0 * m * M + 40.0 * n) + gram + (4 << 20));
+    r->lean_bytes = (int64_t)(8.0 * (8.0 * n * M + 12.0 * M * M + 3.0 * m * M + 40.0 * n) + (4 << 20));
+    r->bytes = r->lean_bytes + (int64_t)gram;
     r->resident = (int64_t)(8.0 * (5.0 * n * M + 8.0 * M * M + 20.0 * n));
     r->work = 4.0 * n * M * M;
     return;
@@ -162,6 +167,8 @@ void estimate(const gpgp_server *s, Req *r) {
       mixed ? 900.0 * n : sliced ? 2700.0 * n + 1100.0 * (double)pred_chunk(r->n, r->m) : 64.0 * n;
   const double nn = mixed ? 5.0 : sliced && r->ap.kind == GPGP_APPROX_EP ? 5.5 : 3.0;
   r->bytes = (int64_t)(8.0 * (nn * n * n + 2.0 * n * std::min(m, 4096.0) + extra + 20.0 * n) + (4 << 20));
+  r->lean_bytes = !sliced ? r->bytes
+                          : (int64_t)(8.0 * (3.0 * n * n + 2.0 * n * std::min(m, 4096.0) + 84.0 * n) + (4 << 20));
   r->resident = (int64_t)(8.0 * (2.0 * n * n + 64.0 * n + 12.0 * n));
   r->work = iters * n * n * n / 3.0 + n * n * m;
 }
@@ -205,7 +212,11 @@ void try_admit(gpgp_server *s) {  // with s->mu held
         continue;
       }
     }
-    const bool fits = s->bytes_inflight + s->bytes_resident + r->bytes <= s->budget;
+    bool fits = s->bytes_inflight + s->bytes_resident + r->bytes <= s->budget;
+    if (!fits && s->bytes_inflight == 0 && s->bytes_resident + r->lean_bytes <= s->budget) {
+      r->bytes = r->lean_bytes;
+      r->lean = fits = true;
+    }
     if (!fits) {
       if (s->bytes_inflight == 0) {  // only resident models stand in the way
         it = s->pending.erase(it);
@@ -247,6 +258,7 @@ void try_admit(gpgp_server *s) {  // with s->mu held
 
 void run_request(gpgp_server *s, Worker &w, Req *r) {
   gpgp_status st = GPGP_OK;
+  tl_lean = r->lean;  // (the worker's thread runs one request at a time)
   if (r->kind == REQ_RELEASE) {
     gpgp_model_free(r->target);
     return;
@@ -491,7 +503,7 @@ gpgp_status gpgp_server_submit(gpgp_server *s, const gpgp_request *q, int64_t *i
   ++s->unfinished;
   Req *rp = r.get();
   s->reqs[r->id] = std::move(r);
-  if (rp->bad_input || rp->bytes > s->budget) {
+  if (rp->bad_input || rp->lean_bytes > s->budget) {
     fail_now(s, rp, rp->bad_input ? GPGP_ENAN : GPGP_EOOM);
     s->cv_done.notify_all();
     return GPGP_OK;

@@ -160,8 +160,8 @@ def split_bytes(rows, K):
 
 def test_prediction_estimate_holds_the_variance_scratch():
     """The variance of an FP64 model of 896 points or more is solved with split operands: n x
-    512, m x 512 and the inverses of the diagonal blocks. A budget that holds the model, the
-    cross covariance and half of them refuses the prediction; one that holds all admits it."""
+    512, m x 512 and the inverses of the diagonal blocks. The prediction is charged for them
+    where the budget holds the model, the cross covariance and them."""
     rng = np.random.default_rng(9)
     n, m = 1500, 4096
     x = rng.uniform(-2, 2, (n, 2))
@@ -173,11 +173,38 @@ def test_prediction_estimate_holds_the_variance_scratch():
     assert scratch > 45e6
     cross = 8 * (2 * n * m + 64 * m + 4 * n) + (1 << 20)
     resident = 8 * (2 * n * n + 76 * n)
-    for budget, want in ((resident + cross + scratch // 2, L.EOOM), (resident + cross + scratch + 4096, 0)):
+    var = []
+    for room, charged in ((scratch + 4096, scratch), (scratch // 2, 0)):
+        budget = resident + cross + room
         with GPServer(precision="fp64", workers=1, hbm_budget=budget) as s:
             r = s.poll(s.submit(gp, x, y, x[:1], keep=True))
             assert r["status"] == 0 and s.stats()["bytes_resident"] == resident
-            assert s.poll(s.submit_pred(r["model"], xt))["status"] == want
             # the mean alone needs none of it
             assert s.poll(s.submit_pred(r["model"], xt, want_var=False))["status"] == 0
-            assert s.stats()["bytes_peak"] <= budget
+            assert s.stats()["bytes_peak"] == resident + cross
+            p = s.poll(s.submit_pred(r["model"], xt))
+            assert p["status"] == 0
+            assert s.stats()["bytes_peak"] == resident + cross + charged
+            var.append(p["var"])
+    # without room for it the solve takes the FP64 pipe
+    assert not np.array_equal(*var)
+    assert np.abs(var[0] - var[1]).max() <= 1e-11
+
+
+def test_budget_that_holds_a_fit_without_its_split_operands():
+    """A budget with room for the matrices of an FP64 EP fit (3 n^2 doubles) and not for the
+    operands of its sliced products (2.5 n^2 more): the fit runs on the FP64 pipe."""
+    rng = np.random.default_rng(10)
+    n = 1200
+    x = rng.uniform(-2, 2, (n, 2))
+    y = (np.sin(3 * x[:, 0]) + 0.3 * rng.standard_normal(n) > 0).astype(float)
+    gp = G.gp_init(G.cf_matern52(lscale=0.6, magn=1.0), G.lik_bernoulli(), approx=G.approx_ep())
+    lean = 8 * (3 * n * n + 2 * n * 5 + 84 * n) + (4 << 20)
+    out = []
+    for budget in (lean + 8 * n * n, 4 * lean):
+        with GPServer(precision="fp64", workers=1, hbm_budget=budget) as s:
+            r = s.poll(s.submit(gp, x, y, x[:5]))
+            assert r["status"] == 0 and s.stats()["bytes_peak"] <= budget
+            out.append(r)
+    assert out[0]["log_evidence"] != out[1]["log_evidence"]
+    assert abs(out[0]["log_evidence"] - out[1]["log_evidence"]) <= 1e-9 * abs(out[1]["log_evidence"])
