@@ -388,9 +388,11 @@ void rows_times_bt(cudaStream_t s, int64_t n, int64_t N, int64_t K, double alpha
 // SMs, 8-slice products, partials summed in a fixed order
 void gram_sliced(cudaStream_t s, const double *A, int64_t lda, const double *B, int64_t ldb, int64_t n, int64_t M,
                  int64_t N, double *C, int64_t ldc, int *err);
-// C = alpha sum_z P_z + beta C over nz M x N partials (fixed order)
+size_t gram_sliced_bytes(int64_t n, int64_t M, int64_t N, int sms);  // its scratch on a GPU of so many SMs
+// C = alpha sum_z P_z + beta C over nz M x N partials (fixed order); go_on (alpha 1, beta 0):
+// the sum goes on from the one in C
 void splitk_reduce(cudaStream_t s, int64_t M, int64_t N, int nz, const double *P, double alpha, double beta,
-                   double *C, int64_t ldc, bool lower_only);
+                   double *C, int64_t ldc, bool lower_only, bool go_on = false);
 // rows from which a product of many rows with a 64-wide K takes the tensor cores at FP64
 // accuracy (4096 x 192: 84 us on the FP64 pipe, ~20 with the two splits; 1000 rows: 20 us)
 constexpr int64_t SLICED_ROWS = 1024;

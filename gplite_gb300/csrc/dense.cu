@@ -122,26 +122,27 @@ __global__ void __launch_bounds__(256) gemm64_kernel(int64_t M, int64_t N, int64
   }
 }
 
-// C = alpha sum_z P_z + beta C over the split-K partials (fixed order)
+// C = alpha sum_z P_z + beta C over the split-K partials (fixed order); go_on: the sum goes
+// on from the one in C (alpha 1, beta 0), as if the partials had followed each other
 __global__ void splitk_reduce_kernel(int64_t M, int64_t N, int nz, const double *__restrict__ P,
                                      double alpha, double beta, double *__restrict__ C, int64_t ldc,
-                                     int lower_only) {
+                                     int lower_only, int go_on) {
   const int64_t MN = M * N;
   for (int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < MN;
        idx += (int64_t)gridDim.x * blockDim.x) {
     const int64_t r = idx % M, c = idx / M;
     if (lower_only && r < c) continue;
-    double s = 0.0;
-    for (int z = 0; z < nz; ++z) s += P[idx + z * MN];
     double *dst = C + r + c * ldc;
+    double s = go_on ? *dst : 0.0;
+    for (int z = 0; z < nz; ++z) s += P[idx + z * MN];
     *dst = (beta == 0.0) ? alpha * s : alpha * s + beta * *dst;
   }
 }
 
 void splitk_reduce(cudaStream_t s, int64_t M, int64_t N, int nz, const double *P, double alpha, double beta,
-                   double *C, int64_t ldc, bool lower_only) {
+                   double *C, int64_t ldc, bool lower_only, bool go_on) {
   splitk_reduce_kernel<<<(unsigned)std::min<int64_t>((M * N + 255) / 256, 4096), 256, 0, s>>>(
-      M, N, nz, P, alpha, beta, C, ldc, lower_only ? 1 : 0);
+      M, N, nz, P, alpha, beta, C, ldc, lower_only ? 1 : 0, go_on ? 1 : 0);
   GPGP_CHECK_LAUNCH();
 }
 

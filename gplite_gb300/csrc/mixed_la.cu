@@ -360,37 +360,71 @@ void trsm_sliced(cudaStream_t s, const double *L, int64_t n, int64_t lda, const 
 // cut into as many ranges as give every SM a tile (each with exponents of its own), the
 // ranges are one batched product, and the partials are added in order. 65536 x 256: the
 // FP64 pipe took 7.0 ms, this 0.45 ms, most of it the two splits.
+// The partials are kept in as many slots as 128 MB hold (at least one) and added whenever
+// the slots are full, so that they do not grow with n (M = 4096, n = 65536: 37 partials
+// of 134 MB each).
 constexpr int64_t GRAM_PASS_BYTES = (int64_t)1 << 27;
+
+struct GramPlan {
+  int64_t kc, full, rem, nz;  // K of a range, full ranges, rows after them, ranges
+  int64_t pass, slots;        // ranges to a product, partials kept
+};
+static GramPlan gram_plan(int64_t n, int64_t M, int64_t N, int sms) {
+  GramPlan g;
+  const int64_t tiles = ((M + 127) / 128) * ((N + 63) / 64);
+  const int64_t want = std::max<int64_t>(1, sms / tiles);
+  // a range: a multiple of the 256 K that are summed exactly, and small enough that the
+  // split operands of one pass over the SMs stay below 128 MB each
+  const int64_t krow = (int64_t)oz_split_bytes(std::max(M, N), 256, OZ_FP64) / 256;  // bytes per K
+  g.kc = ((n + want - 1) / want + 255) / 256 * 256;
+  g.kc = std::max<int64_t>(256, std::min<int64_t>(g.kc, GRAM_PASS_BYTES / (krow * want) / 256 * 256));
+  g.full = n / g.kc;
+  g.rem = n - g.full * g.kc;
+  g.nz = g.full + (g.rem > 0 ? 1 : 0);
+  g.pass = std::max<int64_t>(1, GRAM_PASS_BYTES / (krow * g.kc));
+  g.slots = std::min(g.nz, std::max<int64_t>(1, GRAM_PASS_BYTES / (int64_t)sizeof(double) / (M * N)));
+  return g;
+}
+
+size_t gram_sliced_bytes(int64_t n, int64_t M, int64_t N, int sms) {
+  const GramPlan g = gram_plan(n, M, N, sms);
+  const int64_t cnt = std::min(std::min(g.pass, g.slots), std::max<int64_t>(g.full, 1));
+  return (size_t)cnt * (split_batch_bytes(M, g.kc, OZ_FP64) + split_batch_bytes(N, g.kc, OZ_FP64)) +
+         (size_t)(g.slots * M * N) * sizeof(double);
+}
 
 void gram_sliced(cudaStream_t s, const double *A, int64_t lda, const double *B, int64_t ldb, int64_t n, int64_t M,
                  int64_t N, double *C, int64_t ldc, int *err) {
   if (M <= 0 || N <= 0) return;
-  const int64_t tiles = ((M + 127) / 128) * ((N + 63) / 64);
-  const int64_t want = std::max<int64_t>(1, oz_sms() / tiles);
-  // a range: a multiple of the 256 K that are summed exactly, and small enough that the
-  // split operands of one pass over the SMs stay below 128 MB each
-  const int64_t krow = (int64_t)oz_split_bytes(std::max(M, N), 256, OZ_FP64) / 256;  // bytes per K
-  int64_t kc = ((n + want - 1) / want + 255) / 256 * 256;
-  kc = std::max<int64_t>(256, std::min<int64_t>(kc, GRAM_PASS_BYTES / (krow * want) / 256 * 256));
-  const int64_t full = n / kc, rem = n - full * kc, nz = full + (rem > 0 ? 1 : 0);
+  const GramPlan g = gram_plan(n, M, N, oz_sms());
+  const int64_t kc = g.kc;
   DBuf P;
-  P.alloc(s, (size_t)nz * M * N);
-  const int64_t pass = std::max<int64_t>(1, GRAM_PASS_BYTES / (krow * kc));
-  for (int64_t z0 = 0; z0 < full; z0 += pass) {
-    const int64_t cnt = std::min<int64_t>(pass, full - z0);
+  P.alloc(s, (size_t)g.slots * M * N);
+  int64_t used = 0;
+  bool go_on = false;
+  auto flush = [&] {
+    splitk_reduce(s, M, N, (int)used, P.p, 1.0, 0.0, C, ldc, false, go_on);
+    used = 0;
+    go_on = true;
+  };
+  for (int64_t z0 = 0, cnt; z0 < g.full; z0 += cnt) {
+    cnt = std::min(std::min(g.pass, g.full - z0), g.slots - used);
     SplitBatch a(s, M, kc, cnt, OZ_FP64), b(s, N, kc, cnt, OZ_FP64);
     oz_split_batched(s, A + z0 * kc, lda, kc, 1, M, kc, &a.sp, cnt);
     oz_split_batched(s, B + z0 * kc, ldb, kc, 1, N, kc, &b.sp, cnt);
-    oz_gemm_batched(s, a.sp, 0, b.sp, 0, M, N, 0, kc / 64, 0, 1.0, 0.0, P.p + z0 * M * N, M, M * N, false, err,
+    oz_gemm_batched(s, a.sp, 0, b.sp, 0, M, N, 0, kc / 64, 0, 1.0, 0.0, P.p + used * M * N, M, M * N, false, err,
                     nullptr, 0, cnt);
+    used += cnt;
+    if (used == g.slots) flush();
   }
-  if (rem > 0) {
-    SplitBuf a(s, M, rem, OZ_FP64), b(s, N, rem, OZ_FP64);
-    oz_split(s, A + full * kc, lda, 1, M, rem, &a.sp);
-    oz_split(s, B + full * kc, ldb, 1, N, rem, &b.sp);
-    oz_gemm(s, a.sp, 0, b.sp, 0, M, N, 0, a.sp.nkb, 0, 1.0, 0.0, P.p + full * M * N, M, false, err);
+  if (g.rem > 0) {
+    SplitBuf a(s, M, g.rem, OZ_FP64), b(s, N, g.rem, OZ_FP64);
+    oz_split(s, A + g.full * kc, lda, 1, M, g.rem, &a.sp);
+    oz_split(s, B + g.full * kc, ldb, 1, N, g.rem, &b.sp);
+    oz_gemm(s, a.sp, 0, b.sp, 0, M, N, 0, a.sp.nkb, 0, 1.0, 0.0, P.p + used * M * N, M, false, err);
+    ++used;
   }
-  splitk_reduce(s, M, N, (int)nz, P.p, 1.0, 0.0, C, ldc, false);
+  if (used > 0) flush();
 }
 
 void trmv_sumsq_mixed(cudaStream_t s, const double *W, int64_t n, int64_t ldw, const double *R,

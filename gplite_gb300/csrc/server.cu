@@ -116,6 +116,7 @@ struct gpgp_server {
   int64_t submitted = 0, completed = 0, failed = 0, batches = 0, batched_requests = 0, unfinished = 0;
   std::vector<double> lat;
   bool stop = false;
+  int sms = 0;
 };
 
 namespace {
@@ -148,9 +149,12 @@ void estimate(const gpgp_server *s, Req *r) {
   }
   if (r->meth.kind == GPGP_METHOD_FITC) {
     const double M = (double)r->meth.num_inducing;
-    // beside the fit, the Gram product's two split operands (16 bytes an entry with its
-    // row padding, at most 128 MB each) or those of the substitution (n x 64)
-    const double gram = std::max(std::min(32.0 * n * (M + 128.0), 2.7e8), 16.0 * n * 80.0);
+    // beside the fit, the Gram product's scratch or the split operands of the substitution
+    // (n x 64) and of the row products (EP's, n x M)
+    const int64_t Mi = r->meth.num_inducing, K = r->ap.kind == GPGP_APPROX_EP ? std::max<int64_t>(Mi, NB) : NB;
+    size_t gram = 0;
+    if (r->n >= SLICED_ROWS) gram = oz_split_bytes(r->n, K, OZ_FP64) + oz_split_bytes(Mi, K, OZ_FP64);
+    if (r->n >= GRAM_SLICED_MIN) gram = std::max(gram, gram_sliced_bytes(r->n, Mi, Mi, s->sms));
     r->lean_bytes = (int64_t)(8.0 * (8.0 * n * M + 12.0 * M * M + 3.0 * m * M + 40.0 * n) + (4 << 20));
     r->bytes = r->lean_bytes + (int64_t)gram;
     r->resident = (int64_t)(8.0 * (5.0 * n * M + 8.0 * M * M + 20.0 * n));
@@ -403,6 +407,11 @@ gpgp_status gpgp_server_create(const gpgp_server_opts *opts, gpgp_server **out) 
   if (!(s->o.jitter > 0)) s->o.jitter = 1e-6;
   gpgp_status st = gpgp_create(&s->bctx, s->o.device);
   if (st != GPGP_OK) return st;
+  if (cudaDeviceGetAttribute(&s->sms, cudaDevAttrMultiProcessorCount, s->o.device) != cudaSuccess) {
+    (void)cudaGetLastError();
+    gpgp_destroy(s->bctx);
+    return GPGP_ECUDA;
+  }
   if (s->o.hbm_budget > 0) {
     s->budget = s->o.hbm_budget;
   } else {
