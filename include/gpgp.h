@@ -524,6 +524,11 @@ gpgp_status gpgp_cov_df_selftest(gpgp_ctx *ctx, const gpgp_kernel *k, const doub
  *      GPGP_ETIMEOUT and the context stays usable. ---- */
 gpgp_status gpgp_wait_selftest(gpgp_ctx *ctx, int32_t polls);
 
+/* ---- self-test of FITC's row scaling: out[i, m] = X[i, m] / v[i] (host arrays, n x M
+ *      column-major), as the fits compute it. ---- */
+gpgp_status gpgp_div_rows_selftest(gpgp_ctx *ctx, int64_t n, int64_t M, const double *X, const double *v,
+                                   double *out);
+
 /* ---- test hook: the bound of a kernel's waits, in polls, for launches made by the
  *      calling thread from now on (negative: the default), and the number of K chunks
  *      after which each CTA of a sliced GEMM stops loading operands (negative: never;
