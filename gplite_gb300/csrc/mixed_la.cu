@@ -548,3 +548,31 @@ extern "C" gpgp_status gpgp_mixed_selftest(gpgp_ctx *ctx, int64_t M, int64_t N, 
     return GPGP_EOOM;
   }
 }
+
+extern "C" gpgp_status gpgp_sliced_product_selftest(gpgp_ctx *ctx, int64_t M, int64_t N, int64_t K, int32_t slices,
+                                                    const double *A, const double *B, double *C) {
+  using namespace gpgp;
+  if (!ctx || M < 1 || N < 1 || K < 1 || !A || !B || !C || (slices != 4 && slices != 5 && slices != OZ_FP64))
+    return fail(ctx, GPGP_EINVAL, "invalid argument");
+  return guarded(ctx, [&]() -> gpgp_status {
+    GPGP_CUDA(cudaSetDevice(ctx->device));
+    cudaStream_t s = ctx->stream;
+    DBuf dA, dB, dC;
+    IBuf err;
+    copy_in(s, dA, A, (size_t)(M * K), false);
+    copy_in(s, dB, B, (size_t)(N * K), false);
+    dC.alloc(s, (size_t)(M * N));
+    err.alloc(s, 1);
+    GPGP_CUDA(cudaMemsetAsync(err.p, 0, sizeof(int), s));
+    SplitBuf a(s, M, K, slices), b(s, N, K, slices);
+    oz_split(s, dA.p, M, 0, M, K, &a.sp);
+    oz_split(s, dB.p, N, 0, N, K, &b.sp);
+    oz_gemm(s, a.sp, 0, b.sp, 0, M, N, 0, a.sp.nkb, 0, 1.0, 0.0, dC.p, M, false, err.p);
+    int herr = 0;
+    GPGP_CUDA(cudaMemcpyAsync(&herr, err.p, sizeof(int), cudaMemcpyDeviceToHost, s));
+    GPGP_CUDA(cudaMemcpyAsync(C, dC.p, (size_t)(M * N) * sizeof(double), cudaMemcpyDeviceToHost, s));
+    GPGP_CUDA(cudaStreamSynchronize(s));
+    if (herr) throw WaitTimeout{};
+    return GPGP_OK;
+  });
+}

@@ -524,6 +524,11 @@ gpgp_status gpgp_cov_df_selftest(gpgp_ctx *ctx, const gpgp_kernel *k, const doub
  *      GPGP_ETIMEOUT and the context stays usable. ---- */
 gpgp_status gpgp_wait_selftest(gpgp_ctx *ctx, int32_t polls);
 
+/* ---- the sliced product of given operands: C = A B^T (host arrays, column-major, M x K and
+ *      N x K; slices as above). ---- */
+gpgp_status gpgp_sliced_product_selftest(gpgp_ctx *ctx, int64_t M, int64_t N, int64_t K, int32_t slices,
+                                         const double *A, const double *B, double *C);
+
 /* ---- self-test of FITC's row scaling: out[i, m] = X[i, m] / v[i] (host arrays, n x M
  *      column-major), as the fits compute it. ---- */
 gpgp_status gpgp_div_rows_selftest(gpgp_ctx *ctx, int64_t n, int64_t M, const double *X, const double *v,
