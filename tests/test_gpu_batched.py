@@ -140,3 +140,25 @@ def test_variant_follows_from_the_sizes():
     for a, b in zip(*runs):
         for k in ("log_evidence", "mean", "var", "loos"):
             np.testing.assert_array_equal(a[k], b[k])
+
+
+@pytest.mark.parametrize("n", [1, 15, 16, 17, 31, 33, 48, 63, 64, 65, 127, 129, 200])
+def test_diagonal_kernels_give_the_same_bits(n):
+    """Up to 38 problems to a bucket the diagonal blocks are factored by a cluster of CTAs
+    each, from 39 on by one CTA each: same operations in the same order, so a problem's evidence
+    (log-determinant), mean (factor and inverse) and variance are the same bits alone and among 40. The
+    second problem is close to singular, the third is refused."""
+    rng = np.random.default_rng(n)
+    probs = []
+    for sigma, jitter in ((0.1, 0), (1e-6, 0), (1e-7, 1)):
+        x = rng.uniform(-1, 1, (n, 2))
+        if jitter:
+            x[:] = x[0]
+        probs.append(dict(x=x, y=np.sin(3 * x[:, 0]) + 0.1 * rng.standard_normal(n), xt=rng.uniform(-1, 1, (7, 2)),
+                          kind="sexp", lscale=0.8, magn=1.0, sigma=sigma))
+    for p in probs:
+        one = gp_fit_batched([p], precision="fp64", jitter=0.0)[0]
+        many = gp_fit_batched([p] * 40, precision="fp64", jitter=0.0)
+        for r in (many[0], many[39]):
+            for k in ("log_evidence", "mean", "var", "loos"):
+                np.testing.assert_array_equal(r[k], one[k])
