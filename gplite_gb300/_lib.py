@@ -161,6 +161,7 @@ SIGNATURES = {
     "gpgp_cov_df_selftest": (C.c_int, [_P, C.POINTER(Kernel), _P, C.c_int64, C.c_int32, C.c_double, _P]),
     "gpgp_wait_selftest": (C.c_int, [_P, C.c_int32]),
     "gpgp_sliced_product_selftest": (C.c_int, [_P, C.c_int64, C.c_int64, C.c_int64, C.c_int32, _P, _P, _P]),
+    "gpgp_tri_rows_selftest": (C.c_int, [_P, C.c_int64, C.c_int64, _P, _P, C.c_int32, _P]),
     "gpgp_div_rows_selftest": (C.c_int, [_P, C.c_int64, C.c_int64, _P, _P, _P]),
     "gpgp_wait_bound": (C.c_int, [C.c_int32, C.c_int32, C.c_int32]),
     "gpgp_fit_gaussian_noalloc": (C.c_int, [_P, C.POINTER(Kernel), C.c_double, C.c_double, _P, C.c_int64,

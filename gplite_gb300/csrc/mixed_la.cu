@@ -576,3 +576,27 @@ extern "C" gpgp_status gpgp_sliced_product_selftest(gpgp_ctx *ctx, int64_t M, in
     return GPGP_OK;
   });
 }
+
+extern "C" gpgp_status gpgp_tri_rows_selftest(gpgp_ctx *ctx, int64_t n, int64_t M, const double *L, const double *B,
+                                              int32_t mode, double *X) {
+  using namespace gpgp;
+  if (!ctx || n < 1 || M < 1 || !L || !B || !X || (mode != 0 && mode != 1))
+    return fail(ctx, GPGP_EINVAL, "invalid argument");
+  return guarded(ctx, [&]() -> gpgp_status {
+    GPGP_CUDA(cudaSetDevice(ctx->device));
+    cudaStream_t s = ctx->stream;
+    DBuf dL, dX;
+    IBuf err;
+    copy_in(s, dL, L, (size_t)(M * M), false);
+    copy_in(s, dX, B, (size_t)(n * M), false);
+    err.alloc(s, 1);
+    GPGP_CUDA(cudaMemsetAsync(err.p, 0, sizeof(int), s));
+    tri_rows(s, dL.p, M, M, dX.p, n, dX.p, n, n, mode, err.p);
+    int herr = 0;
+    GPGP_CUDA(cudaMemcpyAsync(&herr, err.p, sizeof(int), cudaMemcpyDeviceToHost, s));
+    GPGP_CUDA(cudaMemcpyAsync(X, dX.p, (size_t)(n * M) * sizeof(double), cudaMemcpyDeviceToHost, s));
+    GPGP_CUDA(cudaStreamSynchronize(s));
+    if (herr) throw WaitTimeout{};
+    return GPGP_OK;
+  });
+}

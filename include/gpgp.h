@@ -529,6 +529,11 @@ gpgp_status gpgp_wait_selftest(gpgp_ctx *ctx, int32_t polls);
 gpgp_status gpgp_sliced_product_selftest(gpgp_ctx *ctx, int64_t M, int64_t N, int64_t K, int32_t slices,
                                          const double *A, const double *B, double *C);
 
+/* ---- self-test of FITC's substitution: X = B L^-T (mode 0) or B L^-1 (mode 1) for the rows
+ *      of B (n x M) and a lower M x M factor (host arrays, column-major). ---- */
+gpgp_status gpgp_tri_rows_selftest(gpgp_ctx *ctx, int64_t n, int64_t M, const double *L, const double *B,
+                                   int32_t mode, double *X);
+
 /* ---- self-test of FITC's row scaling: out[i, m] = X[i, m] / v[i] (host arrays, n x M
  *      column-major), as the fits compute it. ---- */
 gpgp_status gpgp_div_rows_selftest(gpgp_ctx *ctx, int64_t n, int64_t M, const double *X, const double *v,
