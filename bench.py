@@ -40,14 +40,30 @@ SIGMA = 0.05
 LSCALE, MAGN, CMAGN = 0.7, 1.0, 1.0
 NPRED = 8192
 
-# DRAM traffic of the sliced GEMM per launch of the n = 16384 mixed step: the mean of
-# dram__bytes_read.sum + dram__bytes_write.sum over the 363 GEMM and panel launches of
-# one step, one-pass ncu capture (the profile summaries give the command and the
-# per-shape figures: the trailing updates move their FP64 C block in and out once,
-# e.g. 1.9 GB for a 16000 x 16000 lower triangle).
-OZ_TRAFFIC_PER_LAUNCH = {16384: 9.448e7}
-OZ_TRAFFIC_SOURCE = ("ncu --metrics dram__bytes_read.sum,dram__bytes_write.sum,gpu__time_duration.sum "
-                     "-k 'regex:oz_gemm_kernel|panel_block' (1 pass), mean over the 363 launches of one n = 16384 step")
+def oz_step_bytes(n, nbo=384, base=512):
+    """Operand and result bytes of the sliced products of one mixed step, from the sizes of its
+    schedule: four 2-byte slices an operand entry, FP64 results written once and read once where
+    they are updated (the rows of a panel in FP64 only). What L2 holds between two launches is
+    counted all the same, so DRAM moves less."""
+    def pair(n1, n2):  # L21 W11 and W22 (L21 W11) of a node of the inverse
+        return 8.0 * (n2 * n1 + n1 * n1 / 2 + n2 * n1) + 8.0 * (n2 * n2 / 2 + n1 * n2 + n2 * n1)
+
+    def inverse(size, off):
+        if size <= 64 or (size in (128, 256, base) and off % size == 0 and off + size <= n):
+            return 0.0
+        g = base if size > base else 64
+        n1 = -(-(size // 2) // g) * g
+        return inverse(n1, off) + inverse(size - n1, off + n1) + pair(n1, size - n1)
+
+    total = 0.0
+    for k0 in range(0, n - nbo, nbo):  # Cholesky: a panel's blocks, then the trailing update
+        m = n - k0 - nbo
+        total += sum(16.0 * m * 64 * (nbo // 64 - j) for j in range(nbo // 64)) + 8.0 * m * nbo + 8.0 * m * m
+    b = 128
+    while b <= base:
+        total += n // b * pair(b // 2, b // 2)
+        b *= 2
+    return total + inverse(n, 0) + 8.0 * n * n / 2 + 8.0 * n * n / 2  # and B^-1
 
 
 def theta_sequence(k):
@@ -525,8 +541,9 @@ def run_gpu(args):
                                 "FP64-equivalent product with 4 slices), incl. zero-padded tiles: a "
                                 "tensor-pipe utilisation, not algorithmic work"},
                     "potrf_fp64_equiv_tflops": potrf_tf,
-                    "traffic": OZ_TRAFFIC_PER_LAUNCH.get(n), "traffic_unit": "bytes per launch",
-                    "traffic_source": OZ_TRAFFIC_SOURCE if n in OZ_TRAFFIC_PER_LAUNCH else None}
+                    "traffic": oz_step_bytes(n) / nl, "traffic_unit": "bytes per launch",
+                    "traffic_source": "computed on the host from operand and result sizes of the step's "
+                                      "products (an upper bound for DRAM: L2 holds some in between)"}
 
         cpu = None
         if cpu1 is not None:
