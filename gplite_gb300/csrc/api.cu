@@ -1198,7 +1198,7 @@ static gpgp_status pred_impl(gpgp_model *m, const double *xt, int64_t mt, uint32
         if (mixed) {
           trmv_sumsq_mixed(s, m->Linv.p, n, n, R.p, mc, n, csum.p + c0, m->errflag.p);
         } else {
-          if (n < SLICED_MIN || !with_scratch([&] {
+          if (!trsm_takes_slices(n, chunk) || !with_scratch([&] {
                 trsm_sliced(s, m->L.p, n, n, m->Winv.p, R.p, mc, n, m->errflag.p, OZ_FP64);
               })) {
             if (!tmp.p) tmp.alloc(s, (size_t)NB * chunk);

@@ -450,6 +450,8 @@ void lauum_mixed(cudaStream_t s, const double *W, int64_t n, int64_t ldw, double
 // X = L^-1 R in place (n x m, leading dimension ldr; R as it was when it throws
 // std::bad_alloc); its scratch in bytes
 size_t trsm_sliced_bytes(int64_t n, int64_t m, int S);
+// FP64: whether a solve of n x m takes the slices (trsm_lower's products below that)
+bool trsm_takes_slices(int64_t n, int64_t m);
 void trsm_sliced(cudaStream_t s, const double *L, int64_t n, int64_t lda, const double *Winv, double *R, int64_t m,
                  int64_t ldr, int *err, int S);
 // T = W R (W lower n x n, R n x m), then out[j] = sum_i T_ij^2

@@ -322,6 +322,19 @@ void lauum_mixed(cudaStream_t s, const double *W, int64_t n, int64_t ldw, double
 // 512-row ones 4 times less accurate.
 constexpr int64_t TRSM_OUTER = 512;
 
+// For few right-hand sides the FP64 pipe's products are small ones (gemm64_small_kernel, up to
+// 151 tiles of 64 x 64), and the sliced solve's five launches to a block cost more: gp_pred
+// with variance, FP64 pipe against slices, at the last m on the one side of 180 tiles and the
+// first measured on the other:
+//   n = 900   m = 555 (135 tiles) 0.83 / 0.99 ms   777 (195) 1.32 / 1.07
+//   n = 2000  m = 300 (160)       1.94 / 2.04      350 (192) 2.43 / 2.06
+//   n = 4500  m = 111 (142)       3.97 / 4.30      133 (213) 5.87 / 4.35
+//   n = 10000 m = 1 (157)         6.31 / 8.63, n = 12000 m = 16 (188) 11.83 / 11.32
+constexpr int64_t TRSM_TILES = 180;
+bool trsm_takes_slices(int64_t n, int64_t m) {
+  return n >= SLICED_MIN && ((n + 63) / 64) * ((m + 63) / 64) >= TRSM_TILES;
+}
+
 size_t trsm_sliced_bytes(int64_t n, int64_t m, int S) {
   return (size_t)((n + NB - 1) / NB) * split_batch_bytes(NB, NB, S) + oz_split_bytes(n, TRSM_OUTER, S) +
          oz_split_bytes(m, TRSM_OUTER, S);

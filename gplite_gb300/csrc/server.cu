@@ -135,7 +135,8 @@ void estimate(const gpgp_server *s, Req *r) {
       // the substitution's operands (m x 64 and M x 64)
       if (r->m >= SLICED_ROWS)
         r->bytes += (int64_t)(oz_split_bytes(r->m, NB, OZ_FP64) + oz_split_bytes(t.fitc->M, NB, OZ_FP64));
-    } else if (r->var && !t.nlc && t.opts.precision == GPGP_PREC_FP64 && t.n >= SLICED_MIN) {
+    } else if (r->var && !t.nlc && t.opts.precision == GPGP_PREC_FP64 &&
+               trsm_takes_slices(t.n, pred_chunk(t.n, r->m))) {
       // the variance's solve: the diagonal blocks' inverses, n x 512 and m x 512, split
       r->bytes += (int64_t)trsm_sliced_bytes(t.n, pred_chunk(t.n, r->m), OZ_FP64);
     }

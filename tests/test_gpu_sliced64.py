@@ -76,3 +76,30 @@ def test_fitc_either_side_of_the_sliced_sizes(n, M):
     assert np.allclose(p["var"], q["var"], rtol=1e-8, atol=1e-9)
     if n < 5000:
         assert np.allclose(G.gp_loo(g, x, y)["loos"], R.gp_loo(o, x, y)["loos"], rtol=1e-8, atol=1e-8)
+
+
+@pytest.mark.parametrize("n,m", [(900, 704), (900, 769), (1500, 448), (1500, 449), (4600, 129)])
+def test_variance_either_side_of_the_sliced_solve(n, m):
+    """The variance's solve moves to the tensor cores at 180 tiles of 64 x 64 (condition number of
+    B below 1e4: 1e-10)."""
+    rng = np.random.default_rng(n + m)
+    x = rng.uniform(-1, 1, (n, 3))
+    y = np.sin(3 * x[:, 0]) + 0.2 * rng.standard_normal(n)
+    xt = rng.uniform(-1, 1, (m, 3))
+    g = G.gp_fit(G.gp_init(G.cf_matern32(lscale=0.5), G.lik_gaussian(sigma=0.2)), x, y)
+    o = R.gp_fit(R.gp_init([R.cf("matern32", lscale=0.5, magn=1.0)], R.lik("gaussian", sigma=0.2)), x, y)
+    p, q = G.gp_pred(g, xt, var=True), R.gp_pred(o, xt, var=True)
+    assert np.abs(p["mean"] - q["mean"]).max() <= 1e-10
+    assert np.abs(p["var"] - q["var"]).max() <= 1e-10
+
+
+def test_few_predictions_take_few_launches():
+    """The sliced solve takes at least five launches for each 64 rows, which few right-hand sides
+    do not repay; the FP64 pipe's two."""
+    rng = np.random.default_rng(2)
+    x = rng.uniform(-1, 1, (1500, 2))
+    g = G.gp_fit(G.gp_init(G.cf_sexp(lscale=0.5), G.lik_gaussian(sigma=0.2)), x, np.sin(3 * x[:, 0]))
+    for m in (1, 300):
+        before = L.launch_count()
+        G.gp_pred(g, x[:m], var=True)
+        assert L.launch_count() - before <= 3 * 24
