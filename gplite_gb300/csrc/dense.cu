@@ -295,35 +295,39 @@ void gemm64(cudaStream_t s, bool ta, bool tb, int64_t M, int64_t N, int64_t K, d
 // FP64 instructions: 1.6 ms for 256 rows of M = 256, and 65536 rows took 8.1 ms.)
 constexpr int TB = 64;
 
-// One block: rows of X (n x kb, in place) against the kb x kb lower block L. The lanes
+// One block: rows of B (n x kb) against the kb x kb lower block L, into X (which may be B).
+// The lanes
 // of a warp share few rows: lane q of a group of eight owns columns q, q + 8, .. of its
 // row, so that an FP64 instruction (64 cycles of its sub-partition, whatever the number
-// of active lanes) works on four rows and eight columns.
-template <int MODE>
+// of active lanes) works on four rows and eight columns. CG: groups of eight columns, as
+// many as kb needs (a chain step to each: all 64 took a FITC prediction through one inducing
+// input from 124 to 159 us).
+template <int MODE, int CG>
 __global__ void __launch_bounds__(128) tri_block_kernel(const double *__restrict__ L, int64_t ldl, int kb,
-                                                        double *__restrict__ X, int64_t ldx, int64_t n,
-                                                        const int *__restrict__ status) {
+                                                        const double *B, int64_t ldb, double *X, int64_t ldx,
+                                                        int64_t n, const int *__restrict__ status) {
   if (status && *(volatile const int *)status != 0) return;
-  __shared__ double Ls[TB][TB + 1];  // [c][r] = L(r, c): a step reads one column (mode 0) or row (mode 1)
-  __shared__ double rd[TB];
-  for (int idx = threadIdx.x; idx < TB * TB; idx += 128) {
-    const int r = idx % TB, c = idx / TB;
+  constexpr int W = 8 * CG;
+  __shared__ double Ls[W][W + 1];  // [c][r] = L(r, c): a step reads one column (mode 0) or row (mode 1)
+  __shared__ double rd[W];
+  for (int idx = threadIdx.x; idx < W * W; idx += 128) {
+    const int r = idx % W, c = idx / W;
     Ls[c][r] = (r < kb && c < kb && r >= c) ? L[r + c * ldl] : 0.0;
   }
   __syncthreads();
-  if (threadIdx.x < TB) rd[threadIdx.x] = threadIdx.x < kb ? 1.0 / Ls[threadIdx.x][threadIdx.x] : 0.0;
+  if (threadIdx.x < W) rd[threadIdx.x] = threadIdx.x < kb ? 1.0 / Ls[threadIdx.x][threadIdx.x] : 0.0;
   __syncthreads();
   const int lane = threadIdx.x & 31, q = lane & 7;
   const int64_t i = ((int64_t)blockIdx.x * 4 + (threadIdx.x >> 5)) * 4 + (lane >> 3);
-  double x[TB / 8];
+  double x[CG];
 #pragma unroll
-  for (int t = 0; t < TB / 8; ++t) {
+  for (int t = 0; t < CG; ++t) {
     const int c = 8 * t + q;
-    x[t] = (i < n && c < kb) ? X[i + c * ldx] : 0.0;
+    x[t] = (i < n && c < kb) ? B[i + c * ldb] : 0.0;
   }
 #pragma unroll
-  for (int s0 = 0; s0 < TB / 8; ++s0) {
-    const int t0 = MODE == 0 ? s0 : TB / 8 - 1 - s0;  // the eight columns 8 t0 ..
+  for (int s0 = 0; s0 < CG; ++s0) {
+    const int t0 = MODE == 0 ? s0 : CG - 1 - s0;  // the eight columns 8 t0 ..
 #pragma unroll
     for (int s1 = 0; s1 < 8; ++s1) {
       const int cq = MODE == 0 ? s1 : 7 - s1, c = 8 * t0 + cq;
@@ -332,16 +336,26 @@ __global__ void __launch_bounds__(128) tri_block_kernel(const double *__restrict
       if (q == cq) x[t0] = xc;
       else if (MODE == 0 ? q > cq : q < cq) x[t0] = fma(-xc, MODE == 0 ? Ls[c][8 * t0 + q] : Ls[8 * t0 + q][c], x[t0]);
 #pragma unroll
-      for (int t = MODE == 0 ? t0 + 1 : 0; t < (MODE == 0 ? TB / 8 : t0); ++t)
+      for (int t = MODE == 0 ? t0 + 1 : 0; t < (MODE == 0 ? CG : t0); ++t)
         x[t] = fma(-xc, MODE == 0 ? Ls[c][8 * t + q] : Ls[8 * t + q][c], x[t]);
     }
   }
   if (i < n)
 #pragma unroll
-    for (int t = 0; t < TB / 8; ++t) {
+    for (int t = 0; t < CG; ++t) {
       const int c = 8 * t + q;
       if (c < kb) X[i + c * ldx] = x[t];
     }
+}
+
+template <int MODE>
+static void tri_block(cudaStream_t s, const double *L, int64_t ldl, int kb, const double *B, int64_t ldb, double *X,
+                      int64_t ldx, int64_t n, const int *status) {
+  const unsigned grid = (unsigned)((n + 15) / 16);
+  auto kern = kb > 32 ? tri_block_kernel<MODE, 8> : kb > 16 ? tri_block_kernel<MODE, 4>
+              : kb > 8 ? tri_block_kernel<MODE, 2> : tri_block_kernel<MODE, 1>;
+  kern<<<grid, 128, 0, s>>>(L, ldl, kb, B, ldb, X, ldx, n, status);
+  GPGP_CHECK_LAUNCH();
 }
 
 // C = alpha A B^T + beta C (n x N, alpha 1 or -1, beta 0 or 1) for many rows n: on the
@@ -366,12 +380,16 @@ void rows_times_bt(cudaStream_t s, int64_t n, int64_t N, int64_t K, double alpha
 void tri_rows(cudaStream_t s, const double *L, int64_t M, int64_t ldl, const double *B, int64_t ldb,
               double *X, int64_t ldx, int64_t n, int mode, int *err) {
   if (n <= 0 || M <= 0) return;
+  if (M <= TB) {
+    if (mode == 0) tri_block<0>(s, L, ldl, (int)M, B, ldb, X, ldx, n, nullptr);
+    else tri_block<1>(s, L, ldl, (int)M, B, ldb, X, ldx, n, nullptr);
+    return;
+  }
   if (X != B)
     GPGP_CUDA(cudaMemcpy2DAsync(X, ldx * sizeof(double), B, ldb * sizeof(double), n * sizeof(double), M,
                                 cudaMemcpyDeviceToDevice, s));
-  const unsigned grid = (unsigned)((n + 15) / 16);
   SplitBuf xs(s), ls(s);
-  const bool sliced = err && n >= SLICED_ROWS && M > TB && with_scratch([&] {
+  const bool sliced = err && n >= SLICED_ROWS && with_scratch([&] {
                         xs.bind(n, TB, OZ_FP64);
                         ls.bind(M, TB, OZ_FP64);
                       });
@@ -380,9 +398,8 @@ void tri_rows(cudaStream_t s, const double *L, int64_t M, int64_t ldl, const dou
     const int64_t k0 = (mode == 0 ? b : nblk - 1 - b) * TB;
     const int kb = (int)std::min<int64_t>(TB, M - k0);
     double *Xk = X + k0 * ldx;
-    if (mode == 0) tri_block_kernel<0><<<grid, 128, 0, s>>>(L + k0 * (ldl + 1), ldl, kb, Xk, ldx, n, nullptr);
-    else tri_block_kernel<1><<<grid, 128, 0, s>>>(L + k0 * (ldl + 1), ldl, kb, Xk, ldx, n, nullptr);
-    GPGP_CHECK_LAUNCH();
+    if (mode == 0) tri_block<0>(s, L + k0 * (ldl + 1), ldl, kb, Xk, ldx, Xk, ldx, n, nullptr);
+    else tri_block<1>(s, L + k0 * (ldl + 1), ldl, kb, Xk, ldx, Xk, ldx, n, nullptr);
     // the columns after the block (mode 0: X_rest -= X_k L_rest,k^T) or before it
     // (mode 1: X_rest -= X_k L_k,rest)
     const int64_t rest = mode == 0 ? M - k0 - kb : k0;
@@ -589,11 +606,12 @@ void potrf(cudaStream_t s, double *A, int64_t n, int64_t lda, double *Winv, doub
     const int64_t m = n - k0 - kb;
     if (m > 0) {
       double *A21 = A + (k0 + kb) + k0 * lda;
-      if (panel_mode == 1)
+      if (panel_mode == 1) {
         potrf_panel_inv_kernel<<<(unsigned)((m + 3) / 4), 256, 0, s>>>(A21, m, kb, lda, W, status);
-      else
-        tri_block_kernel<0><<<(unsigned)((m + 15) / 16), 128, 0, s>>>(Akk, lda, kb, A21, lda, m, status);
-      GPGP_CHECK_LAUNCH();
+        GPGP_CHECK_LAUNCH();
+      } else {
+        tri_block<0>(s, Akk, lda, kb, A21, lda, A21, lda, m, status);
+      }
       double *A22 = A + (k0 + kb) + (k0 + kb) * lda;
       gemm64(s, false, true, m, m, kb, -1.0, A21, lda, A21, lda, 1.0, A22, lda, true, 0);
     }
