@@ -393,9 +393,14 @@ size_t gram_sliced_bytes(int64_t n, int64_t M, int64_t N, int sms);  // its scra
 // the sum goes on from the one in C
 void splitk_reduce(cudaStream_t s, int64_t M, int64_t N, int nz, const double *P, double alpha, double beta,
                    double *C, int64_t ldc, bool lower_only, bool go_on = false);
-// rows from which a product of many rows with a 64-wide K takes the tensor cores at FP64
-// accuracy (4096 x 192: 84 us on the FP64 pipe, ~20 with the two splits; 1000 rows: 20 us)
-constexpr int64_t SLICED_ROWS = 1024;
+// Whether a product of many rows (n x N, K terms) takes the tensor cores at FP64 accuracy:
+// 4096 x 192 x 64 takes 84 us on the FP64 pipe and ~20 with the two splits, 1000 x 192 x 64
+// 20 us. Below 16 M multiply-adds (28 us of the pipe) the two splits and their scratch cost
+// more than they save (gp_loo of a FITC fit, n = 1100, M = 70 and 100: 2.00 -> 1.96 ms).
+constexpr int64_t SLICED_ROWS = 1024, SLICED_ROW_WORK = (int64_t)1 << 24;
+inline bool rows_take_slices(int64_t n, int64_t N, int64_t K) {
+  return n >= SLICED_ROWS && n * N * K >= SLICED_ROW_WORK;
+}
 // rows from which a Gram product takes gram_sliced
 constexpr int64_t GRAM_SLICED_MIN = 4096;
 // C = alpha A B^T + beta C on K chunks [kc0, kc1) (64 wide); a_row0/b_row0 multiples of 64.

@@ -359,11 +359,11 @@ static void tri_block(cudaStream_t s, const double *L, int64_t ldl, int kb, cons
 }
 
 // C = alpha A B^T + beta C (n x N, alpha 1 or -1, beta 0 or 1) for many rows n: on the
-// tensor cores at FP64 accuracy from SLICED_ROWS rows on.
+// tensor cores at FP64 accuracy where rows_take_slices.
 void rows_times_bt(cudaStream_t s, int64_t n, int64_t N, int64_t K, double alpha, const double *A, int64_t lda,
                    const double *B, int64_t ldb, double beta, double *C, int64_t ldc, int *err) {
   SplitBuf a(s), b(s);
-  if (n < SLICED_ROWS || !with_scratch([&] {
+  if (!rows_take_slices(n, N, K) || !with_scratch([&] {
         a.bind(n, K, OZ_FP64);
         b.bind(N, K, OZ_FP64);
       })) {
@@ -389,7 +389,8 @@ void tri_rows(cudaStream_t s, const double *L, int64_t M, int64_t ldl, const dou
     GPGP_CUDA(cudaMemcpy2DAsync(X, ldx * sizeof(double), B, ldb * sizeof(double), n * sizeof(double), M,
                                 cudaMemcpyDeviceToDevice, s));
   SplitBuf xs(s), ls(s);
-  const bool sliced = err && n >= SLICED_ROWS && with_scratch([&] {
+  // (the first block has the most columns after it)
+  const bool sliced = err && rows_take_slices(n, M - TB, TB) && with_scratch([&] {
                         xs.bind(n, TB, OZ_FP64);
                         ls.bind(M, TB, OZ_FP64);
                       });
@@ -406,7 +407,7 @@ void tri_rows(cudaStream_t s, const double *L, int64_t M, int64_t ldl, const dou
     if (rest <= 0) continue;
     double *Xr = mode == 0 ? X + (k0 + kb) * ldx : X;
     const double *Lr = mode == 0 ? L + (k0 + kb) + k0 * ldl : L + k0;
-    if (sliced) {
+    if (sliced && rows_take_slices(n, rest, TB)) {
       oz_split(s, Xk, ldx, 0, n, kb, &xs.sp);
       oz_split(s, Lr, ldl, mode == 0 ? 0 : 1, rest, kb, &ls.sp);
       oz_gemm(s, xs.sp, 0, ls.sp, 0, n, rest, 0, 1, 0, -1.0, 1.0, Xr, ldx, false, err);

@@ -1,5 +1,6 @@
 """FITC's substitution with the rows of a matrix, whose products run on the tensor cores from 1024
-rows on: its residual, which no condition number enters, for the factor of a smooth kernel."""
+rows and 16 M multiply-adds on: its residual, which no condition number enters, for the factor
+of a smooth kernel."""
 import numpy as np
 import pytest
 
@@ -14,7 +15,8 @@ def sexp(a, b, lscale):
 
 @pytest.mark.parametrize("mode", [0, 1])
 @pytest.mark.parametrize("n,M", [(3, 1), (40, 8), (17, 9), (40, 16), (33, 17), (50, 32), (1100, 33), (70, 63), (40, 200),
-                                 (1023, 65), (1024, 64), (1024, 65), (1500, 100), (2049, 257), (4500, 200)])
+                                 (1023, 65), (1024, 64), (1024, 65), (1500, 100), (2047, 192), (2048, 192), (2049, 257),
+                                 (4500, 200)])
 def test_residual_of_a_smooth_kernels_factor(n, M, mode):
     """X L^T = B (mode 1: X L = B) for the factor L of a squared exponential's K_z, singular up
     to its jitter of 1e-6, where inverses of diagonal blocks would lose digits. Substitution is
