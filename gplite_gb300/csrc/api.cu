@@ -300,7 +300,8 @@ int64_t factor_and_solve(gpgp_model *m, Work &w, const double *zvec, double *alp
   return hstatus;
 }
 
-// W = L^-1, kept on the model (FP64 blocked solve or the sliced recursive inverse).
+// W = L^-1, kept on the model (the sliced recursive inverse, or the FP64 pipe's blocked
+// solve for small n and where the slices do not fit).
 void compute_linv(gpgp_model *m) {
   if (m->have_Linv) return;
   cudaStream_t st = m->ctx->stream;

@@ -9,8 +9,9 @@
 // is factored and inverted by one cluster of CTAs (diag.cu; the inverses serve the
 // solves); the panel below is solved by row-parallel substitution,
 // which stays backward stable when a diagonal block is ill-conditioned (FITC's
-// K_z); the trailing update is a lower-only GEMM on the FP64 pipe. The
-// triangular solves are single launches ordered by per-block flags.
+// K_z); the trailing update is a lower-only GEMM on the FP64 pipe. (FP64 fits of
+// SLICED_MIN points and more factor on the tensor cores, mixed_la.cu.) The triangular solves
+// are single launches ordered by the solution's entries, which are their own flags.
 #include <math.h>
 
 #include <algorithm>

@@ -26,7 +26,7 @@
 // N = 256 128), so a K step of S = 4 is 476 cycles at least. What bounds the kernel:
 // at long K the MMAs (1.37 to 1.5 PFLOP/s at 4096^2 x 4096, S = 4; 1.15 with the issue
 // loop inside one lane's branch), at K <= 384 the epilogue's integer work and C
-// traffic (8192^2, lower-only off: K = 384 0.55 ms, K = 256 0.43, K = 64 0.41; 0.70,
+// traffic (8192^2, lower-only off: K = 384 0.52 ms, K = 256 0.41, K = 64 0.41; 0.70,
 // 0.60 and 0.63 with 64-bit tile arithmetic in every warp and a branch per converted
 // output).
 //
@@ -66,7 +66,9 @@ constexpr int OZ_THREADS = 32 * (2 + OZ_EPI_WARPS);  // producer, MMA, epilogue
 // S = 8 (OZ_FP64; 63-bit fixed point, digits of at most 128): the products of levels
 // 0..7 (36), each level in an accumulator of its own, all 512 columns of TMEM. An
 // operand entry keeps its 53 bits down to 2^-10 of its row's largest, the sums are
-// exact to 2^-62 of the product of both rows' scales, and the outputs of fits of 1000
+// exact to 2^-62 of the product of both rows' scales (unless the digits of 256 products
+// line up: a level's sum beyond 2^24, possible from the fifth on, rounds to units of 2^-46
+// and finer), and the outputs of fits of 1000
 // to 3000 points are as far from 64-bit references as with the FP64 pipe's products
 // (prediction mean 4.1e-14 against 4.4e-14, variance 9.8e-14 / 9.8e-14, gradient
 // 1.53e-12 / 1.54e-12: geometric means over 36 and 24 fits). With 7 slices, which are

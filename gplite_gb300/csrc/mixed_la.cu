@@ -1,8 +1,9 @@
-// Mixed-precision blocked algorithms built on the sliced tensor-core GEMM
-// (mixed.cu): Cholesky, triangular inverse, B^-1 = L^-T L^-1 and the
-// predictive-variance product. Outputs have the same meaning and layout as the
-// FP64 routines of dense.cu; only the contractions change precision (products
-// of 32-bit fixed-point row slices, accumulated exactly, summed in FP64).
+// Blocked algorithms built on the sliced tensor-core GEMM (mixed.cu): Cholesky,
+// triangular inverse, B^-1 = L^-T L^-1, the predictive variance's solve or product, and Gram
+// products. Outputs have the same meaning and layout as the FP64 routines of dense.cu; only
+// the contractions differ: products of fixed-point row slices, accumulated exactly and
+// summed in FP64, of 32 bits (S = 4, the mixed precision) or 63 (S = OZ_FP64, the FP64 path
+// of large n).
 //
 // Cholesky is two-level right-looking: outer panels of NBO columns (384: faster
 // at n = 16384 than 256 or 512), each factored in 64-wide blocks (factor_panel); one
